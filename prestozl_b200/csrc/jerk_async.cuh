@@ -1,0 +1,86 @@
+// Bulk (TMA engine) row copies into shared memory and the bounded wait for
+// them, and the status bits the kernels report through.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+namespace jerk {
+
+__device__ __forceinline__ unsigned smem_u32(const void *p)
+{
+    return static_cast<unsigned>(__cvta_generic_to_shared(p));
+}
+
+__device__ __forceinline__ void bulk_row_load(void *dst, const void *src, unsigned bytes,
+                                              uint64_t *bar)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                 :: "r"(smem_u32(bar)), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
+// Waits for phase `parity` of the mbarrier; gives up after a bounded number
+// of polls (each try_wait itself suspends for a bounded time) and returns
+// false.
+__device__ __forceinline__ bool bar_wait(uint64_t *bar, unsigned parity)
+{
+    for (int it = 0; it < (1 << 16); it++) {
+        unsigned done;
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (done)
+            return true;
+    }
+    return false;
+}
+
+// Status bits written by the kernels (read back after each pass).
+constexpr unsigned kStatusRind = 1u;     // harmsum: a subharmonic r index left its row
+constexpr unsigned kStatusCopy = 2u;     // a copy into shared memory did not complete
+
+// SMs of the current device (queried once; every B200 has 148)
+inline int sm_count()
+{
+    static int n = 0;
+    if (n <= 0) {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess &&
+            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0)
+            n = v;
+        else
+            return 148;
+    }
+    return n;
+}
+
+// Lets a kernel take all of the shared memory a CTA may have (carveout: and
+// asks for the largest shared-memory share of the SM).
+template <class K>
+inline cudaError_t smem_attrs(K kernel, bool carveout)
+{
+    cudaFuncAttributes a;
+    cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 227 * 1024 - (int)a.sharedSizeBytes);
+    if (e == cudaSuccess && carveout)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 (int)cudaSharedmemCarveoutMaxShared);
+    return e;
+}
+
+// this CTA's rsteps: all of the batch, or a share of them when a small
+// group's rows alone would leave SMs idle (ny > 1 chunks)
+__device__ __forceinline__ void rstep_chunk(int nb, int ny, int y, int *b0, int *b1)
+{
+    const int bchunk = (nb + ny - 1) / ny;
+    *b0 = min(nb, y * bchunk);
+    *b1 = min(nb, *b0 + bchunk);
+}
+
+}  // namespace jerk

@@ -162,6 +162,87 @@ template <int SIGN> struct Dft<5, SIGN> {
     }
 };
 
+template <int SIGN> struct Dft<7, SIGN> {
+    __device__ __forceinline__ static void run(float2 *v)
+    {
+        const float c[3] = {0.62348980185873353053f, -0.22252093395631440429f,
+                            -0.90096886790241912624f};  // cos(2 pi m/7)
+        const float s[3] = {0.78183148246802980871f, 0.97492791218182360702f,
+                            0.43388373911755812048f};   // sin(2 pi m/7)
+        const float2 x0 = v[0];
+        float2 a[3], b[3];
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            a[m] = cadd(v[m + 1], v[6 - m]);
+            b[m] = csub(v[m + 1], v[6 - m]);
+        }
+        v[0] = cadd(cadd(x0, a[0]), cadd(a[1], a[2]));
+#pragma unroll
+        for (int k = 1; k <= 3; k++) {
+            float2 p = x0, q = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int m = 1; m <= 3; m++) {
+                // cos and sin of 2 pi k m / 7 from the first half period
+                const int e = (k * m) % 7, f = e <= 3 ? e : 7 - e;
+                const float cc = c[f - 1], ss = e <= 3 ? s[f - 1] : -s[f - 1];
+                p = make_float2(p.x + cc * a[m - 1].x, p.y + cc * a[m - 1].y);
+                q = make_float2(q.x + ss * b[m - 1].x, q.y + ss * b[m - 1].y);
+            }
+            const float2 iq = mul_si<SIGN>(q);
+            v[k] = cadd(p, iq);
+            v[7 - k] = csub(p, iq);
+        }
+    }
+};
+
+// Index maps of the prime-factor transform of A B points, A and B coprime:
+// input (B n1 + A n2) mod A B, output (B B' k1 + A A' k2) mod A B with
+// B B' = 1 mod A and A A' = 1 mod B; the A x B transform between them needs
+// no twiddles.
+template <int A, int B>
+struct Pfa {
+    static constexpr int N = A * B;
+    static constexpr int unit(int m, int mod)  // m m' with m m' = 1 mod `mod`
+    {
+        for (int i = 1; i < mod; i++)
+            if (m * i % mod == 1)
+                return m * i;
+        return m;
+    }
+    static constexpr int in(int n1, int n2) { return (B * n1 + A * n2) % N; }
+    static constexpr int out(int k1, int k2) { return (unit(B, A) * k1 + unit(A, B) * k2) % N; }
+};
+
+template <int A, int B, int SIGN>
+struct DftPfa {
+    __device__ __forceinline__ static void run(float2 *v)
+    {
+        float2 t[A][B];
+#pragma unroll
+        for (int n1 = 0; n1 < A; n1++) {
+#pragma unroll
+            for (int n2 = 0; n2 < B; n2++)
+                t[n1][n2] = v[Pfa<A, B>::in(n1, n2)];
+            Dft<B, SIGN>::run(t[n1]);
+        }
+#pragma unroll
+        for (int k2 = 0; k2 < B; k2++) {
+            float2 u[A];
+#pragma unroll
+            for (int n1 = 0; n1 < A; n1++)
+                u[n1] = t[n1][k2];
+            Dft<A, SIGN>::run(u);
+#pragma unroll
+            for (int k1 = 0; k1 < A; k1++)
+                v[Pfa<A, B>::out(k1, k2)] = u[k1];
+        }
+    }
+};
+template <int SIGN> struct Dft<6, SIGN> : DftPfa<2, 3, SIGN> {};
+template <int SIGN> struct Dft<10, SIGN> : DftPfa<2, 5, SIGN> {};
+template <int SIGN> struct Dft<12, SIGN> : DftPfa<3, 4, SIGN> {};
+template <int SIGN> struct Dft<14, SIGN> : DftPfa<2, 7, SIGN> {};
+
 // Radix plans: the first radix fixes the thread count T = N / R0.
 //
 // Twiddles live in per-stage tables: stage s >= 1 (Ns = product of the
@@ -191,9 +272,12 @@ JERK_FFT_PLAN(192, 4, 16, 3)
 JERK_FFT_PLAN(256, 8, 8, 4)
 JERK_FFT_PLAN(384, 8, 16, 3)
 JERK_FFT_PLAN(512, 8, 16, 4)
+JERK_FFT_PLAN(640, 8, 16, 5)
 JERK_FFT_PLAN(768, 16, 16, 3)
 JERK_FFT_PLAN(1024, 16, 16, 4)
 JERK_FFT_PLAN(1280, 16, 16, 5)
+JERK_FFT_PLAN(1536, 16, 16, 6)
+JERK_FFT_PLAN(1792, 16, 16, 7)
 JERK_FFT_PLAN(2048, 16, 16, 8)
 JERK_FFT_PLAN(4096, 16, 16, 16)
 JERK_FFT_PLAN(5120, 16, 16, 4, 5)
@@ -481,8 +565,8 @@ __device__ __forceinline__ Cp pmul(Cp a, float c, float s)
     return {fma2(a.re, bc(c), mul2(a.im, bc(-s))), fma2(a.im, bc(c), mul2(a.re, bc(s)))};
 }
 
-// Inverse (exponent sign +1) DFTs of radix 4, 8 and 5 on lane pairs; the
-// output order is that of Dft<R, +1>.
+// Inverse (exponent sign +1) DFTs of radix 2 to 6 and 8 on lane pairs; the output
+// order is that of Dft<R, +1>.
 __device__ __forceinline__ void pdft4(Cp &v0, Cp &v1, Cp &v2, Cp &v3)
 {
     const Cp a = padd(v0, v2), b = psub(v0, v2), c = padd(v1, v3), e = psub(v1, v3);
@@ -540,6 +624,56 @@ __device__ __forceinline__ void pdft5(Cp *v)
     v[4] = psub_i(p1, t1);
     v[2] = padd_i(p2, t2);
     v[3] = psub_i(p2, t2);
+}
+
+__device__ __forceinline__ void pdft2(Cp &v0, Cp &v1)
+{
+    const Cp a = v0;
+    v0 = padd(a, v1);
+    v1 = psub(a, v1);
+}
+
+__device__ __forceinline__ void pdft3(Cp &v0, Cp &v1, Cp &v2)
+{
+    const float s3 = 0.86602540378443864676f;  // sin(2 pi / 3)
+    const Cp t = padd(v1, v2), d = psub(v1, v2);
+    const Cp m = {fma2(bc(-0.5f), t.re, v0.re), fma2(bc(-0.5f), t.im, v0.im)};
+    v0 = padd(v0, t);
+    v1 = {fma2(bc(-s3), d.im, m.re), fma2(bc(s3), d.re, m.im)};
+    v2 = {fma2(bc(s3), d.im, m.re), fma2(bc(-s3), d.re, m.im)};
+}
+
+template <int R>
+__device__ __forceinline__ void pdft(Cp *v)
+{
+    static_assert(R >= 2 && R <= 8 && R != 7, "packed radices");
+    if constexpr (R == 2) {
+        pdft2(v[0], v[1]);
+    } else if constexpr (R == 3) {
+        pdft3(v[0], v[1], v[2]);
+    } else if constexpr (R == 4) {
+        pdft4(v[0], v[1], v[2], v[3]);
+    } else if constexpr (R == 5) {
+        pdft5(v);
+    } else if constexpr (R == 6) {  // prime factors 2 x 3, as DftPfa<2, 3>
+        using X = Pfa<2, 3>;
+        Cp t[2][3];
+#pragma unroll
+        for (int n1 = 0; n1 < 2; n1++) {
+#pragma unroll
+            for (int n2 = 0; n2 < 3; n2++)
+                t[n1][n2] = v[X::in(n1, n2)];
+            pdft3(t[n1][0], t[n1][1], t[n1][2]);
+        }
+#pragma unroll
+        for (int k2 = 0; k2 < 3; k2++) {
+            pdft2(t[0][k2], t[1][k2]);
+            v[X::out(0, k2)] = t[0][k2];
+            v[X::out(1, k2)] = t[1][k2];
+        }
+    } else {
+        pdft8(v);
+    }
 }
 
 // Host: the per-stage twiddle tables of FftPlan<N>, forward sign, computed

@@ -29,6 +29,8 @@
 #include <cmath>
 #include <cstdint>
 
+#include "jerk_async.cuh"
+#include "jerk_corr.cuh"
 #include "jerk_fft.cuh"
 #include "jerk_kernels.cuh"
 
@@ -61,8 +63,7 @@ constexpr double kLn2 = 0.69314718055994530942;  // log(2.0), correctly rounded
 constexpr int kLocAvg = 20;   // NUMLOCPOWAVG (include/presto.h:100)
 constexpr int kLocDelta = 5;  // DELTAAVGBINS (include/presto.h:104)
 
-template <int M>
-__device__ __forceinline__ float local_power(const float *pw, int i)
+__device__ __forceinline__ float local_power(const float *pw, int M, int i)
 {
     constexpr int khw = kLocAvg / 2 + kLocDelta;
     const double w = (double)((M / 2) / kLocAvg) * 2.0 / (double)M;
@@ -160,10 +161,73 @@ __host__ __device__ constexpr int prep_buf_len()
     return fft_buf_len<N>() * 2 > kSelInts ? fft_buf_len<N>() : kSelInts / 2;
 }
 
+// The chunk of (rstep b, subharmonic s): gather its M bins into data (the
+// powers into keys), normalise.  hist: kSelInts words of shared memory that
+// nothing else uses until the next barrier after this.
+__device__ __forceinline__ void prep_chunk(const SearchDev &P, const SubDev &sd, const StepDev &st,
+                                           int M, float2 *data, float *keys, unsigned *hist)
+{
+    const int tid = threadIdx.x, nt = blockDim.x;
+    // get_fourier_amplitudes: M bins from lobin, zero outside the file
+    const long long lobin = st.rlo - sd.halfwidth;
+    for (int i = tid; i < M; i += nt) {
+        const long long bi = lobin - P.lobin + i;
+        float2 v = make_float2(0.f, 0.f);
+        if (bi >= 0 && bi < P.numbins)
+            v = P.spec[bi];
+        data[i] = v;
+        keys[i] = __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y));
+    }
+    __syncthreads();
+
+    if (!(P.nph > 0.0f) && P.norm_type == 1) {
+        // -locpow: a float norm per bin (src/accel_utils.c:1186-1203)
+        for (int i = tid; i < M; i += nt) {
+            const float nrm = invsqrtf_ref(local_power(keys, M, i));
+            float2 v = data[i];
+            v.x = __fmul_rn(v.x, nrm);
+            v.y = __fmul_rn(v.y, nrm);
+            data[i] = v;
+        }
+    } else {
+        double norm;
+        if (P.nph > 0.0f) {
+            norm = __ddiv_rn(1.0, __dsqrt_rn((double)P.nph));
+        } else {
+            // median(): the order statistic of rank (M-1)/2 (src/median.c)
+            const double med = (double)select_rank(keys, M, (M - 1) / 2, hist);
+            norm = __ddiv_rn(1.0, __dsqrt_rn(__ddiv_rn(med, kLn2)));
+        }
+        for (int i = tid; i < M; i += nt) {
+            float2 v = data[i];
+            v.x = __double2float_rn(__dmul_rn((double)v.x, norm));
+            v.y = __double2float_rn(__dmul_rn((double)v.y, norm));
+            data[i] = v;
+        }
+    }
+    __syncthreads();
+}
+
+// rinds: fundamental r -> subharmonic r index (src/accel_utils.c:1114-1123)
+__device__ __forceinline__ void prep_rinds(const SearchDev &P, const SubDev &sd, const StepDev &st,
+                                           int b, int s)
+{
+    if (sd.numharm <= 1)
+        return;
+    uint16_t *rinds = P.rinds + ((long long)b * P.nsubs + s) * P.corr_uselen;
+    const double rlo = (double)st.rlo;
+    for (int ii = threadIdx.x; ii < P.corr_uselen; ii += blockDim.x) {
+        const double rr = __dadd_rn(st.fullrlo, __dmul_rn((double)ii, 0.5));
+        const double subr = calc_required_r_d(sd.harm_fract, rr);
+        rinds[ii] = (uint16_t)index_from_r_d(subr, rlo);
+    }
+}
+
 template <int N>
 __device__ void prep_impl(const SearchDev &P, int b, int s, float *smem)
 {
     constexpr int M = N / 2;  // numdata = fftlen / ACCEL_NUMBETWEEN
+    static_assert(M >= 2 * (kLocAvg / 2 + kLocDelta), "chunk too short for -locpow");
     constexpr int R0 = FftPlan<N>::R0;
     const SubDev sd = P.subs[s];
     const StepDev st = P.steps[(P.first_rstep + b) * P.nsubs + s];
@@ -182,47 +246,7 @@ __device__ void prep_impl(const SearchDev &P, int b, int s, float *smem)
         for (int i = tid; i < TWN; i += nt)
             tws[i] = P.twiddles[sd.twoff + i];
     }
-
-    // get_fourier_amplitudes: M bins from lobin, zero outside the file
-    const long long lobin = st.rlo - sd.halfwidth;
-    for (int i = tid; i < M; i += nt) {
-        const long long bi = lobin - P.lobin + i;
-        float2 v = make_float2(0.f, 0.f);
-        if (bi >= 0 && bi < P.numbins)
-            v = P.spec[bi];
-        data[i] = v;
-        keys[i] = __fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y));
-    }
-    __syncthreads();
-
-    double norm = 1.0;
-    if (P.nph > 0.0f) {
-        norm = __ddiv_rn(1.0, __dsqrt_rn((double)P.nph));
-    } else if (P.norm_type == 1) {
-        // -locpow: a float norm per bin (src/accel_utils.c:1186-1203)
-        static_assert(M >= 2 * (kLocAvg / 2 + kLocDelta), "chunk too short for -locpow");
-        for (int i = tid; i < M; i += nt) {
-            const float nrm = invsqrtf_ref(local_power<M>(keys, i));
-            float2 v = data[i];
-            v.x = __fmul_rn(v.x, nrm);
-            v.y = __fmul_rn(v.y, nrm);
-            data[i] = v;
-        }
-    } else {
-        // median(): the order statistic of rank (M-1)/2 (src/median.c)
-        const double med =
-            (double)select_rank(keys, M, (M - 1) / 2, reinterpret_cast<unsigned *>(buf));
-        norm = __ddiv_rn(1.0, __dsqrt_rn(__ddiv_rn(med, kLn2)));
-    }
-    if (!(P.nph <= 0.0f && P.norm_type == 1)) {
-        for (int i = tid; i < M; i += nt) {
-            float2 v = data[i];
-            v.x = __double2float_rn(__dmul_rn((double)v.x, norm));
-            v.y = __double2float_rn(__dmul_rn((double)v.y, norm));
-            data[i] = v;
-        }
-    }
-    __syncthreads();
+    prep_chunk(P, sd, st, M, data, keys, reinterpret_cast<unsigned *>(buf));
 
     // spread_no_pad (data at even interbins) + forward FFT (sign -1).  For a
     // power-of-two fftlen the chunk is scaled by 1/fftlen here, exactly (a
@@ -245,22 +269,63 @@ __device__ void prep_impl(const SearchDev &P, int b, int s, float *smem)
             outp[m] = y;
     };
     fft_block<N, -1>(buf, tw, tid, in, out);
-
-    // rinds: fundamental r -> subharmonic r index (src/accel_utils.c:1114-1123)
-    if (sd.numharm > 1) {
-        uint16_t *rinds = P.rinds + ((long long)b * P.nsubs + s) * P.corr_uselen;
-        const double rlo = (double)st.rlo;
-        for (int ii = tid; ii < P.corr_uselen; ii += nt) {
-            const double rr = __dadd_rn(st.fullrlo, __dmul_rn((double)ii, 0.5));
-            const double subr = calc_required_r_d(sd.harm_fract, rr);
-            rinds[ii] = (uint16_t)index_from_r_d(subr, rlo);
-        }
-    }
+    prep_rinds(P, sd, st, b, s);
 }
 
+// Forward transform of one window of the normalised chunk (FoldClass).
+template <int L>
+__device__ __forceinline__ void prep_window(float2 *buf, const float2 *tw, const float2 *data,
+                                            float2 *outp)
+{
+    const int tid = threadIdx.x;
+    auto in = [&](int r) -> float2 { return data[tid + r * (L / FftPlan<L>::R0)]; };
+    auto out = [&](int m, float2 y) { outp[m] = y; };
+    fft_block<L, -1>(buf, tw, tid, in, out);
+    __syncthreads();  // buf is the next window's too
+}
+
+// Shared float2 of prep_folded's FFT buffer for an M-bin chunk.
+__host__ __device__ inline int prep_folded_buf(int M)
+{
+    return fft_buf_len_rt(M) * 2 > kSelInts ? fft_buf_len_rt(M) : kSelInts / 2;
+}
+
+// A folded subharmonic (jerk_fold.cu): the same chunk, then the transform of
+// each of its windows.  The spread to interbins drops out (the folded rows
+// hold both output parities), so a window of L bins takes an L-point
+// transform.
+__device__ void prep_folded(const SearchDev &P, const SubDev &sd, int b, int s, float *smem)
+{
+    const StepDev st = P.steps[(P.first_rstep + b) * P.nsubs + s];
+    const int M = sd.fftlen / 2;
+    float2 *buf = reinterpret_cast<float2 *>(smem);
+    float2 *data = buf + prep_folded_buf(M);
+    float *keys = reinterpret_cast<float *>(data + M);
+    prep_chunk(P, sd, st, M, data, keys, reinterpret_cast<unsigned *>(buf));
+    for (int c = sd.cls0; c < sd.cls0 + sd.ncls; c++) {
+        const FoldClass fc = P.classes[c];
+        float2 *outp = P.prepped + fc.data_off + (long long)b * fc.len;
+        const float2 *tw = P.twiddles + fc.twoff;
+        switch (fc.len) {
+#define JERK_WIN(LL) case LL: prep_window<LL>(buf, tw, data + fc.wstart, outp); break;
+        JERK_WIN(256) JERK_WIN(384) JERK_WIN(512) JERK_WIN(640) JERK_WIN(768)
+        JERK_WIN(1024) JERK_WIN(1280) JERK_WIN(1536) JERK_WIN(1792) JERK_WIN(2048)
+#undef JERK_WIN
+        default: break;
+        }
+    }
+    prep_rinds(P, sd, st, b, s);
+}
+
+// LONG: the lengths whose FFT plans need more than 256 threads too.
+template <bool LONG>
 __device__ __forceinline__ void prep_dispatch(const SearchDev &P, int b, int s)
 {
     extern __shared__ float smem[];
+    if (P.subs[s].ncls > 0) {
+        prep_folded(P, P.subs[s], b, s, smem);
+        return;
+    }
     switch (P.subs[s].fftlen) {
 #define JERK_PREP_CASE(NN)                   \
     case NN:                                 \
@@ -276,19 +341,31 @@ __device__ __forceinline__ void prep_dispatch(const SearchDev &P, int b, int s)
         JERK_PREP_CASE(1280)
         JERK_PREP_CASE(2048)
         JERK_PREP_CASE(4096)
-        JERK_PREP_CASE(5120)
-        JERK_PREP_CASE(7680)
-        JERK_PREP_CASE(10240)
-        JERK_PREP_CASE(15360)
-#undef JERK_PREP_CASE
     default:
+        if constexpr (LONG) {
+            switch (P.subs[s].fftlen) {
+                JERK_PREP_CASE(5120)
+                JERK_PREP_CASE(7680)
+                JERK_PREP_CASE(10240)
+                JERK_PREP_CASE(15360)
+#undef JERK_PREP_CASE
+            default:
+                break;
+            }
+        }
         break;
     }
 }
 
-__global__ void __launch_bounds__(1024) prep_kernel(const __grid_constant__ SearchDev P)
+// Threads of a prep CTA: 256 serve every length up to 4096 (and leave the
+// compiler 128 registers); the longer ones take their FFT plan's count.
+constexpr int kPrepLong = 4096;
+
+template <bool LONG>
+__global__ void __launch_bounds__(LONG ? 1024 : 256, LONG ? 1 : 2)
+    prep_kernel(const __grid_constant__ SearchDev P)
 {
-    prep_dispatch(P, blockIdx.x, blockIdx.y);
+    prep_dispatch<LONG>(P, blockIdx.x, blockIdx.y);
 }
 
 // plan i of the wave: index of the plan that owns flat CTA x
@@ -300,83 +377,18 @@ __device__ __forceinline__ int group_plan(const GroupLaunch &M, int x)
     return i;
 }
 
-__global__ void __launch_bounds__(1024) prep_group_kernel(const __grid_constant__ GroupLaunch M)
+template <bool LONG>
+__global__ void __launch_bounds__(LONG ? 1024 : 256, LONG ? 1 : 2)
+    prep_group_kernel(const __grid_constant__ GroupLaunch M)
 {
     const int i = group_plan(M, blockIdx.x);
     const int local = blockIdx.x - M.cta0[i];
     const int nsubs = M.P[i].nsubs;
-    prep_dispatch(M.P[i], local / nsubs, local % nsubs);
+    prep_dispatch<LONG>(M.P[i], local / nsubs, local % nsubs);
 }
 
 // ---------------------------------------------------------------------------
 // 2. Correlation: one CTA per kernel row, all rsteps of the batch.
-
-// Occupancy target for corr_kernel: enough CTAs per SM that 128-thread CTAs
-// give 16 resident warps (registers are capped to fit); CTAs of 384 threads
-// or more run one per SM (two would cap them at 64 registers and spill).
-template <int N>
-struct CorrOcc {
-    static constexpr int T = FftPlan<N>::T;
-    static constexpr int value = T >= 384 ? 1 : (T >= 256 ? 2 : (T >= 128 ? 4 : 8));
-};
-
-// Shared memory of corr_kernel<N>, in float2: the FFT buffer, the twiddle
-// tables and (when that still leaves CorrOcc CTAs per SM) a staging row for
-// the next rstep's prepared data.
-// Lengths whose twiddle tables do not fit beside the buffer (15360: 158 KB of
-// tables) read twiddles and kernel rows from global memory (L1/L2) instead of
-// shared memory and registers; 960 threads leave 68 registers a thread.
-template <int N>
-struct CorrBig {
-    static constexpr bool value =
-        (size_t)(fft_buf_len<N>() + FftPlan<N>::twsize()) * 8 > 200 * 1024;
-};
-
-template <int N>
-struct CorrSmem {
-    static constexpr int kBase =
-        (fft_buf_len<N>() + (CorrBig<N>::value ? 0 : FftPlan<N>::twsize()) + 1) & ~1;
-    // the staged row is the prepared chunk's first half (see corr_body)
-    static constexpr bool kStage = (size_t)(kBase + N / 2) * 8 * CorrOcc<N>::value <= 220 * 1024;
-    static constexpr int value = kBase + (kStage ? N / 2 : 0);
-};
-
-// Bulk (TMA engine) copy of one data row into shared memory, completed on an
-// mbarrier, and the bounded wait for it.
-__device__ __forceinline__ unsigned smem_u32(const void *p)
-{
-    return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void bulk_row_load(void *dst, const void *src, unsigned bytes,
-                                              uint64_t *bar)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                 :: "r"(smem_u32(bar)), "r"(bytes) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-
-// Waits for phase `parity` of the mbarrier; gives up after a bounded number
-// of polls (each try_wait itself suspends for a bounded time) and returns
-// false.
-__device__ __forceinline__ bool bar_wait(uint64_t *bar, unsigned parity)
-{
-    for (int it = 0; it < (1 << 16); it++) {
-        unsigned done;
-        asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-        if (done)
-            return true;
-    }
-    return false;
-}
-
-// Status bits written by the kernels (read back after each pass).
-constexpr unsigned kStatusRind = 1u;     // harmsum: a subharmonic r index left its row
-constexpr unsigned kStatusCopy = 2u;     // corr: a data-row copy did not complete
 
 // A wait that must run out: the correlation's bounded wait (bar_wait) on an
 // mbarrier whose phase 0 nothing completes (no copy is involved, so nothing
@@ -396,124 +408,6 @@ cudaError_t launch_wait_probe(unsigned int *status, cudaStream_t st)
 {
     wait_probe_kernel<<<1, 1, 0, st>>>(status);
     return cudaGetLastError();
-}
-
-// One CTA of a wave: kernel row `row` of the fftlen-N group G, rsteps
-// [b0, b1) of the batch.  (A plan's own launch, corr_kernel below, is the
-// same code reading its arguments straight from the kernel parameters: the
-// body, which reaches them through references, measured 6 % slower at
-// fftlen 2048 and spills at 1280, where CTAs of 80 threads run 8 per SM.)
-template <int N>
-__device__ __forceinline__ void corr_body(const SearchDev &P, const RowGroup &G, const int row,
-                                          const int b0, const int b1)
-{
-    constexpr int R0 = FftPlan<N>::R0;
-    constexpr int T = FftPlan<N>::T;
-    constexpr int TWN = FftPlan<N>::twsize();
-    constexpr bool kStage = CorrSmem<N>::kStage;
-    constexpr bool kBig = CorrBig<N>::value;
-    extern __shared__ __align__(16) float2 sm2[];
-    __shared__ uint64_t s_bar;
-    float2 *buf = sm2;
-    float2 *tws = sm2 + fft_buf_len<N>();
-    float2 *dsm = sm2 + CorrSmem<N>::kBase;  // staged data row (kStage)
-    const int tid = threadIdx.x;
-    int gi = 0;
-    while (gi + 1 < G.n && row >= G.rowstart[gi + 1])
-        gi++;
-    const int s = G.sub[gi];
-    const int lrow = row - G.rowstart[gi];
-    const SubDev sd = P.subs[s];
-    const float2 *D0 = P.prepped + sd.data_off;
-
-    // The prepared chunk is the FFT of data spread to even interbins, which
-    // repeats with period N/2 (X[k + N/2] = X[k]); prep_kernel stores its
-    // first half only, and element m of the product reads X[m mod N/2].  In
-    // the first-stage butterfly of thread tid, input r is element
-    // tid + r N/R0, so inputs r and r + R0/2 read the same value.
-    static_assert(R0 % 2 == 0 && (N / R0) * (R0 / 2) == N / 2, "half-row reads");
-    constexpr unsigned kRowBytes = N / 2 * sizeof(float2);
-    if constexpr (kStage) {
-        if (tid == 0) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_bar)) : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-        __syncthreads();
-        if (tid == 0 && b0 < b1)
-            bulk_row_load(dsm, D0 + (long long)b0 * N, kRowBytes, &s_bar);
-    }
-
-    const float2 *tw = kBig ? P.twiddles + sd.twoff : tws;
-    if constexpr (!kBig) {
-        for (int i = tid; i < TWN; i += T)
-            tws[i] = P.twiddles[sd.twoff + i];
-    }
-
-
-    // the kernel row, in the order this thread's first-stage butterfly reads it
-    // (kBig: read from global memory at every rstep instead)
-    float2 kreg[R0];
-    const float2 *K = P.bank + sd.kern_off + (long long)lrow * N;
-    if constexpr (!kBig) {
-#pragma unroll
-        for (int r = 0; r < R0; r++)
-            kreg[r] = K[tid + r * (N / R0)];
-    }
-    __syncthreads();
-
-    const int offset = sd.halfwidth * 2;  // binoffset * ACCEL_NUMBETWEEN
-    const float norm = sd.pownorm;
-    for (int b = b0; b < b1; b++) {
-        const int numrs = P.steps[(P.first_rstep + b) * P.nsubs + s].numrs;
-        float *outp = P.planes + sd.plane_off + (long long)b * sd.plane_size +
-                      (long long)lrow * sd.stride;
-        // the power is formed for every output and the store predicated on
-        // the good-bin range (one unsigned compare): measured faster than a
-        // branch around both.  Power-of-two fftlen: 1/fftlen^2 is already in
-        // the chunk.
-        auto out = [&](int m, float2 y) {
-            const int kk = m - offset;
-            const float pw = fmaf(y.x, y.x, y.y * y.y);
-            const float o = IsPow2<N>::value ? pw : pw * norm;
-            if ((unsigned)kk < (unsigned)numrs)
-                outp[kk] = o;
-        };
-        if constexpr (kStage) {
-            // rstep b's row is (or will shortly be) in dsm; once every thread
-            // has read it, thread 0 starts the copy of rstep b + 1's row
-            if (!bar_wait(&s_bar, (b - b0) & 1) && P.status)
-                atomicOr(P.status, kStatusCopy);
-            auto in = [&](int r) -> float2 {
-                // kBig: the kernel row is read from global memory here too
-                return cmulconj(dsm[tid + (r % (R0 / 2)) * (N / R0)],
-                                kBig ? K[tid + r * (N / R0)] : kreg[r]);
-            };
-            auto mid = [&] {
-                if (tid == 0 && b + 1 < b1) {
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    bulk_row_load(dsm, D0 + (long long)(b + 1) * N, kRowBytes, &s_bar);
-                }
-            };
-            fft_block<N, +1>(buf, tw, tid, in, out, mid);
-        } else {
-            const float2 *D = D0 + (long long)b * N;
-            auto in = [&](int r) -> float2 {
-                const int m = tid + r * (N / R0);
-                return cmulconj(D[tid + (r % (R0 / 2)) * (N / R0)], kBig ? K[m] : kreg[r]);
-            };
-            fft_block<N, +1>(buf, tw, tid, in, out);
-        }
-        __syncthreads();
-    }
-}
-
-// this CTA's rsteps: all of the batch, or a share of them when a small
-// group's rows alone would leave SMs idle (ny > 1 chunks)
-__device__ __forceinline__ void rstep_chunk(int nb, int ny, int y, int *b0, int *b1)
-{
-    const int bchunk = (nb + ny - 1) / ny;
-    *b0 = min(nb, y * bchunk);
-    *b1 = min(nb, *b0 + bchunk);
 }
 
 // A plan's own launch: one CTA per kernel row (blockIdx.x) of the group,
@@ -625,429 +519,6 @@ __global__ void __launch_bounds__(FftPlan<N>::T, CorrOcc<N>::value)
         }
         __syncthreads();
     }
-}
-
-// A wave's CTAs reach their plan's arguments by index, which costs registers:
-// at fftlen 1280 (80-thread CTAs, 8 per SM, 80 registers) the body spills,
-// so those run 5 per SM.
-template <int N>
-struct CorrGroupOcc {
-    static constexpr int value = N == 1280 ? 5 : CorrOcc<N>::value;
-};
-
-template <int N>
-__global__ void __launch_bounds__(FftPlan<N>::T, CorrGroupOcc<N>::value)
-    corr_group_kernel(const __grid_constant__ GroupLaunch M)
-{
-    const int i = group_plan(M, blockIdx.x);
-    const int local = blockIdx.x - M.cta0[i];
-    const int ny = M.ny[i];
-    int b0, b1;
-    rstep_chunk(M.P[i].nb, ny, local % ny, &b0, &b1);
-    corr_body<N>(M.P[i], M.G[i], local / ny, b0, b1);
-}
-
-// ---------------------------------------------------------------------------
-// 2b. Correlation at fftlen 2048 and 1280 on folded kernel rows.
-//
-// The prepared chunk D repeats with period N/2 (it is the transform of data
-// spread to even interbins), so the inverse transform of D conj(K) splits
-// into two half-length transforms, one per output parity:
-//   y[2m]     = IFFT_{N/2}(D A)[m],  A[k] = conj K[k] + conj K[k + N/2]
-//   y[2m + 1] = IFFT_{N/2}(D B)[m],  B[k] = (conj K[k] - conj K[k + N/2]) e^{+2 pi i k/N}
-// for k < N/2.  A and B depend only on the kernel row, so a plan folds its
-// rows of a folded length once (fold_rows_kernel, in double, each value
-// rounded once) and the correlation runs two half-length transforms that read
-// each data value once for both: the first radix-2 layer of the full
-// transform (its butterflies and twiddles) is gone, and the two transforms
-// share every twiddle and every data value.
-//
-// The half-length plan is [8, 16, R2] for T = N/16 threads (H = N/2 = 128
-// R2: 1024 = [8, 16, 8] on 128 threads, 640 = [8, 16, 5] on 80).  Stages 0
-// and 2 run the two transforms in the two lanes of packed FP32 instructions
-// (Cp, pdft8, pdft5): every butterfly of the even transform has its twin in
-// the odd one at the same position with the same twiddle and data value, so
-// each instruction does both.  Stage 0 (radix 8, T butterflies): thread j
-// does butterfly j of both from the same 8 data values, and applies stage 1's
-// input twiddles.  Stage 1 (radix 16, T/2 butterflies per transform): one
-// transform per thread in scalar FP32, the first half of the threads the even
-// one and the second half the odd one, so every warp works (a scalar
-// instruction holds the FP32 pipe for one cycle, a packed one for two: the
-// pipe time is the same either way).  Stage 2 (radix R2, 128 butterflies,
-// Ns = 128): butterfly j of both, and the lane pair of powers (outputs 2 m,
-// 2 m + 1) is one 8-byte store.
-
-static int sm_count();
-
-template <int N>
-struct FoldPlan;
-// CTAs per SM: 5 at 2048 (93 registers, 44 KB of shared memory); 6 at 1280
-template <>
-struct FoldPlan<2048> {
-    static constexpr int R2 = 8, Occ = 5;
-};
-template <>
-struct FoldPlan<1280> {
-    static constexpr int R2 = 5, Occ = 6;
-};
-template <int N>
-struct Fold : FoldPlan<N> {
-    static constexpr int H = N / 2;
-    static constexpr int T = H / 8;                   // threads, stage-0 butterflies
-    static constexpr int Plane = fft_buf_len<H>();     // float2 per transform buffer
-    static constexpr int Tw2 = 128 * FoldPlan<N>::R2;  // stage 2: W_H^(r k) at [r 128 + k]
-    // shared memory: four transform buffers, stage 0's table, the data row
-    static constexpr int Smem = (4 * Plane + 128 + H) * 8;
-    static_assert(H == 128 * FoldPlan<N>::R2 && T % 16 == 0, "[8, 16, R2] on N/16 threads");
-    static_assert((4 * Plane + 128) % 2 == 0, "16-byte aligned staging row");
-};
-constexpr int kFoldTw1 = 8 * 16;  // stage 1's roots W_128^(r k) at [r 8 + k] (both lengths)
-
-bool fold_length(int N) { return N == 2048 || N == 1280; }
-int fold_occ(int N) { return N == 2048 ? Fold<2048>::Occ : N == 1280 ? Fold<1280>::Occ : 0; }
-
-int fold_twiddle_size(int N)
-{
-    return N == 2048 ? kFoldTw1 + Fold<2048>::Tw2 : N == 1280 ? kFoldTw1 + Fold<1280>::Tw2 : 0;
-}
-
-// Host: the two tables of a folded length, forward sign, in double rounded
-// to float.
-void fold_twiddle_table(int N, float2 *out)
-{
-    const double tau = 2.0 * 3.14159265358979323846264338327950288;
-    const int H = N / 2, R2 = H / 128;
-    for (int r = 0; r < 16; r++)
-        for (int k = 0; k < 8; k++) {
-            const double a = -tau * (double)(r * k) / 128.0;
-            out[r * 8 + k] = make_float2((float)cos(a), (float)sin(a));
-        }
-    for (int r = 0; r < R2; r++)
-        for (int k = 0; k < 128; k++) {
-            const double a = -tau * (double)(r * k) / (double)H;
-            out[kFoldTw1 + r * 128 + k] = make_float2((float)cos(a), (float)sin(a));
-        }
-}
-
-// Folded rows: row i of the launch's groups (consecutive over its
-// subharmonics) from bank row src[i]; out[i] = A (first half), B (second).
-template <int N>
-__global__ void fold_rows_kernel(const float2 *__restrict__ bank, const long long *src,
-                                 float2 *__restrict__ out, int nrows)
-{
-    constexpr int H = N / 2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long row = t / H;
-    const int k = (int)(t % H);
-    if (row >= nrows)
-        return;
-    const float2 *K = bank + src[row];
-    const float2 k0 = K[k], k1 = K[k + H];
-    // conj K[k] +/- conj K[k + N/2], in double
-    const double ar = (double)k0.x + (double)k1.x, ai = -(double)k0.y - (double)k1.y;
-    const double dr = (double)k0.x - (double)k1.x, di = -(double)k0.y + (double)k1.y;
-    double sn, cs;
-    sincospi((double)k / (double)H, &sn, &cs);  // e^{+2 pi i k / N}
-    float2 *o = out + row * N;
-    o[k] = make_float2((float)ar, (float)ai);
-    o[k + H] = make_float2((float)(dr * cs - di * sn), (float)(dr * sn + di * cs));
-}
-
-cudaError_t launch_fold_rows(int N, const float2 *bank, const long long *src, float2 *out,
-                             int nrows, cudaStream_t st)
-{
-    const long long n = (long long)nrows * (N / 2);
-    const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (N == 2048)
-        fold_rows_kernel<2048><<<blocks, 256, 0, st>>>(bank, src, out, nrows);
-    else if (N == 1280)
-        fold_rows_kernel<1280><<<blocks, 256, 0, st>>>(bank, src, out, nrows);
-    else
-        return cudaErrorInvalidValue;
-    return cudaGetLastError();
-}
-
-// v (c + i s) with (c, s) the conjugate of a forward table root w: the
-// inverse transform's twiddle
-__device__ __forceinline__ Cp pmul_conj(const Cp &v, float2 w) { return pmul(v, w.x, -w.y); }
-
-// The rstep loop of one CTA of the folded correlation (both launch forms).
-// Shared memory holds four transform buffers (stage 0 writes even / odd,
-// stage 1 reads them and writes the other two, stage 2 reads those), each a
-// padded float2 plane (pad(), conflict-free for all three stages' access
-// patterns), stage 0's table and the staged half data row; stage 2's roots
-// are read through L1 (shared by the CTAs of an SM).
-// kr[r], ki[r]: the lane pairs (re A, re B), (im A, im B) of the row's
-// folded values at k = tid + T r.  steps: the row's subharmonic at b = 0
-// (stride nsubs per rstep); out: its volume row at b = 0; norm: the
-// subharmonic's 1/fftlen^2, applied to the powers where N is not a power
-// of two (prep_kernel scales power-of-two chunks by 1/fftlen instead).
-template <int N>
-__device__ __forceinline__ void fold_rsteps(float2 *bufE, float2 *bufO, float2 *outE,
-                                            float2 *outO, const float2 *tw1,
-                                            const float2 *tw2, const float2 *dsm, uint64_t *bar,
-                                            const float2 (&kr)[8], const float2 (&ki)[8],
-                                            const float2 *D0, const StepDev *steps, int nsubs,
-                                            float *out, long long plane_size, int offset,
-                                            float norm, int b0, int b1, unsigned *status)
-{
-    using F = Fold<N>;
-    constexpr int T = F::T, H = F::H, R2 = F::R2;
-    constexpr int NB1 = T / 2;  // stage-1 butterflies per transform
-    constexpr unsigned kRowBytes = H * sizeof(float2);
-    const int tid = threadIdx.x;
-    for (int b = b0; b < b1; b++) {
-        const int numrs = steps[(long long)b * nsubs].numrs;
-        float *outp = out + (long long)b * plane_size;
-        if (!bar_wait(bar, (b - b0) & 1) && status)
-            atomicOr(status, kStatusCopy);
-        // stage 0: radix 8 of both transforms from the same data values
-        {
-            Cp v[8];
-#pragma unroll
-            for (int r = 0; r < 8; r++) {
-                const float2 d = dsm[tid + T * r];
-                // d A and d B: (dr ar - di ai, dr ai + di ar) per lane
-                v[r].re = fma2(bc(d.x), kr[r], mul2(bc(-d.y), ki[r]));
-                v[r].im = fma2(bc(d.x), ki[r], mul2(bc(d.y), kr[r]));
-            }
-            pdft8(v);
-            // stage 1's input twiddles, applied here: element 8 t + r of
-            // this stage is input t / (T/16) of stage-1 butterfly
-            // (8 t + r) mod (T/2), whose twiddle is W_128^((t / (T/16)) r)
-            const float2 *w1 = tw1 + (tid / (T / 16)) * 8;
-#pragma unroll
-            for (int r = 1; r < 8; r++)
-                v[r] = pmul_conj(v[r], w1[r]);
-            const int pd = pad(tid * 8);
-#pragma unroll
-            for (int r = 0; r < 8; r++) {
-                bufE[pad_add(pd, r)] = make_float2(v[r].re.x, v[r].im.x);
-                bufO[pad_add(pd, r)] = make_float2(v[r].re.y, v[r].im.y);
-            }
-        }
-        __syncthreads();
-        // every thread has read the staged row: start the next rstep's copy
-        if (tid == 0 && b + 1 < b1) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            bulk_row_load(const_cast<float2 *>(dsm), D0 + (long long)(b + 1) * N, kRowBytes, bar);
-        }
-        // stage 1: radix 16 (Ns = 8), one transform per thread (scalar): the
-        // first T/2 threads butterfly j = tid of the even transform, the rest
-        // of the odd one; its input twiddles were applied by stage 0
-        {
-            const bool odd = tid >= NB1;
-            const int j = odd ? tid - NB1 : tid;
-            const float2 *src = odd ? bufO : bufE;
-            float2 *dst = odd ? outO : outE;
-            float2 x[16];
-            if constexpr (IsPow2<NB1>::value) {
-                const int pj = pad(j);
-#pragma unroll
-                for (int r = 0; r < 16; r++)
-                    x[r] = src[pad_add(pj, r * NB1)];
-            } else {
-#pragma unroll
-                for (int r = 0; r < 16; r++)
-                    x[r] = src[pad(j + r * NB1)];
-            }
-            Dft<16, +1>::run(x);
-            const int pq = pad((j >> 3) * 128 + (j & 7));
-#pragma unroll
-            for (int r = 0; r < 16; r++)
-                dst[pad_add(pq, r * 8)] = x[r];
-        }
-        __syncthreads();
-        // stage 2: radix R2 (Ns = 128), butterflies j = tid, tid + T, ... < 128
-        // of both
-#pragma unroll
-        for (int jb = 0; jb < 128; jb += T) {
-            const int j = jb + tid;
-            if (128 % T == 0 || j < 128) {
-                Cp v[R2];
-                const int pj = pad(j);
-#pragma unroll
-                for (int r = 0; r < R2; r++) {
-                    const float2 e = outE[pad_add(pj, r * 128)], o = outO[pad_add(pj, r * 128)];
-                    v[r].re = make_float2(e.x, o.x);
-                    v[r].im = make_float2(e.y, o.y);
-                }
-#pragma unroll
-                for (int r = 1; r < R2; r++)
-                    v[r] = pmul_conj(v[r], __ldg(tw2 + r * 128 + j));
-                if constexpr (R2 == 8)
-                    pdft8(v);
-                else
-                    pdft5(v);
-                // outputs 2 m and 2 m + 1, m = j + 128 r: the lane pair of
-                // powers is one 8-byte store (offset and numrs are even)
-#pragma unroll
-                for (int r = 0; r < R2; r++) {
-                    const int kk = 2 * (j + 128 * r) - offset;
-                    float2 pw = fma2(v[r].re, v[r].re, mul2(v[r].im, v[r].im));
-                    if constexpr (!IsPow2<N>::value)
-                        pw = mul2(pw, bc(norm));
-                    if ((unsigned)kk < (unsigned)numrs)
-                        *reinterpret_cast<float2 *>(outp + kk) = pw;
-                }
-            }
-        }
-        // no barrier: the next rstep's stage 0 writes bufE / bufO, last read
-        // in stage 1 before the barrier above, and its stage 1 writes outE /
-        // outO only after the barrier that follows its stage 0
-    }
-}
-
-// Set-up shared by both launch forms: carve shared memory, start the first
-// data-row copy, stage the twiddles, load this thread's folded values, then
-// run the rstep loop.
-template <int N>
-__device__ __forceinline__ void fold_cta(const SubDev &sd, const float2 *prepped,
-                                         const StepDev *steps, int nsubs, float *planes,
-                                         int lrow, const float2 *__restrict__ Fr,
-                                         const float2 *__restrict__ ftw, int b0, int b1,
-                                         unsigned *status)
-{
-    using F = Fold<N>;
-    constexpr int T = F::T, H = F::H;
-    extern __shared__ __align__(16) float2 smf[];
-    __shared__ uint64_t s_bar;
-    float2 *tws = smf + 4 * F::Plane;
-    float2 *dsm = tws + kFoldTw1;
-    const int tid = threadIdx.x;
-    const float2 *D0 = prepped + sd.data_off;
-    constexpr unsigned kRowBytes = H * sizeof(float2);
-
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (tid == 0 && b0 < b1)
-        bulk_row_load(dsm, D0 + (long long)b0 * N, kRowBytes, &s_bar);
-    for (int i = tid; i < kFoldTw1; i += T)
-        tws[i] = ftw[i];
-    float2 kr[8], ki[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-        const float2 a = Fr[tid + T * r], bb = Fr[H + tid + T * r];
-        kr[r] = make_float2(a.x, bb.x);
-        ki[r] = make_float2(a.y, bb.y);
-    }
-    __syncthreads();
-    fold_rsteps<N>(smf, smf + F::Plane, smf + 2 * F::Plane, smf + 3 * F::Plane, tws,
-                   ftw + kFoldTw1, dsm, &s_bar, kr, ki, D0, steps, nsubs,
-                   planes + sd.plane_off + (long long)lrow * sd.stride, sd.plane_size,
-                   sd.halfwidth * 2, sd.pownorm, b0, b1, status);
-}
-
-// A plan's own launch at a folded length: one CTA per kernel row
-// (blockIdx.x) of the group, rsteps of chunk blockIdx.y of gridDim.y; F: the
-// group's folded rows in launch order; ftw: the two twiddle tables.
-template <int N>
-__global__ void __launch_bounds__(Fold<N>::T, Fold<N>::Occ)
-    corr_fold_kernel(const __grid_constant__ SearchDev P, const __grid_constant__ RowGroup G,
-                     const float2 *__restrict__ F, const float2 *__restrict__ ftw)
-{
-    const int row = blockIdx.x;
-    int gi = 0;
-    while (gi + 1 < G.n && row >= G.rowstart[gi + 1])
-        gi++;
-    const int s = G.sub[gi];
-    const int bchunk = (P.nb + (int)gridDim.y - 1) / (int)gridDim.y;
-    const int b0 = min(P.nb, (int)blockIdx.y * bchunk), b1 = min(P.nb, b0 + bchunk);
-    fold_cta<N>(P.subs[s], P.prepped, P.steps + P.first_rstep * P.nsubs + s, P.nsubs, P.planes,
-                row - G.rowstart[gi], F + (long long)row * N, ftw, b0, b1, P.status);
-}
-
-template <int N>
-__global__ void __launch_bounds__(Fold<N>::T, Fold<N>::Occ)
-    corr_fold_group_kernel(const __grid_constant__ GroupLaunch M)
-{
-    const int i = group_plan(M, blockIdx.x);
-    const int local = blockIdx.x - M.cta0[i];
-    const int ny = M.ny[i];
-    int b0, b1;
-    rstep_chunk(M.P[i].nb, ny, local % ny, &b0, &b1);
-    const SearchDev &P = M.P[i];
-    const RowGroup &G = M.G[i];
-    const int row = local / ny;
-    int gi = 0;
-    while (gi + 1 < G.n && row >= G.rowstart[gi + 1])
-        gi++;
-    const int s = G.sub[gi];
-    fold_cta<N>(P.subs[s], P.prepped, P.steps + P.first_rstep * P.nsubs + s, P.nsubs, P.planes,
-                row - G.rowstart[gi], M.fold[i] + (long long)row * N, M.fold_tw[i], b0, b1,
-                P.status);
-}
-
-template <class K>
-static cudaError_t fold_attrs(K kernel, int smem)
-{
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
-    return e;
-}
-
-// A wave's plans at a folded length (M.fold, M.fold_tw set).
-template <int N>
-static cudaError_t launch_corr_fold_group_n(GroupLaunch M, cudaStream_t st)
-{
-    using F = Fold<N>;
-    if (M.n < 1 || M.n > kMaxGroupPlans)
-        return cudaErrorInvalidValue;
-    cudaError_t e = fold_attrs(corr_fold_group_kernel<N>, F::Smem);
-    if (e != cudaSuccess)
-        return e;
-    const int wave = sm_count() * F::Occ;
-    long long total = 0;
-    for (int i = 0; i < M.n; i++)
-        total += M.G[i].rowstart[M.G[i].n];
-    long long x = 0;
-    for (int i = 0; i < M.n; i++) {
-        const int rows = M.G[i].rowstart[M.G[i].n];
-        const int split = total >= 2 * wave ? 1
-                          : std::max(1, std::min(M.P[i].nb, (int)((2 * wave + total - 1) / total)));
-        M.cta0[i] = (int)x;
-        M.ny[i] = split;
-        x += (long long)rows * split;
-    }
-    if (x >= (1ll << 31))
-        return cudaErrorInvalidValue;
-    M.cta0[M.n] = (int)x;
-    corr_fold_group_kernel<N><<<(unsigned)x, F::T, F::Smem, st>>>(M);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_corr_fold_group(int N, GroupLaunch M, cudaStream_t st)
-{
-    return N == 2048 ? launch_corr_fold_group_n<2048>(M, st)
-           : N == 1280 ? launch_corr_fold_group_n<1280>(M, st)
-                       : cudaErrorInvalidValue;
-}
-
-template <int N>
-static cudaError_t launch_corr_fold_n(const SearchDev &P, const RowGroup &G, int rows,
-                                      const float2 *Fr, const float2 *ftw, cudaStream_t st)
-{
-    using F = Fold<N>;
-    cudaError_t e = fold_attrs(corr_fold_kernel<N>, F::Smem);
-    if (e != cudaSuccess)
-        return e;
-    const int wave = sm_count() * F::Occ;
-    const int split = rows >= 2 * wave ? 1 : std::max(1, std::min(P.nb, (2 * wave + rows - 1) / rows));
-    corr_fold_kernel<N><<<dim3(rows, split), F::T, F::Smem, st>>>(P, G, Fr, ftw);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_corr_fold(int N, const SearchDev &P, const RowGroup &G, int rows,
-                             const float2 *F, const float2 *ftw, cudaStream_t st)
-{
-    return N == 2048 ? launch_corr_fold_n<2048>(P, G, rows, F, ftw, st)
-           : N == 1280 ? launch_corr_fold_n<1280>(P, G, rows, F, ftw, st)
-                       : cudaErrorInvalidValue;
 }
 
 // ---------------------------------------------------------------------------
@@ -1325,7 +796,7 @@ __global__ void __launch_bounds__(kHarmThreads, HarmOcc<S, 4>::value)
 {
     const int i = group_plan(M, blockIdx.x);
     const int local = blockIdx.x - M.cta0[i];
-    const int nx = M.ny[i], nw = M.P[i].numw0;
+    const int nx = M.nx[i], nw = M.P[i].numw0;
     harmsum_body<S, 4, false>(M.P[i], nullptr, local % nx, (local / nx) % nw, local / (nx * nw));
 }
 
@@ -1539,16 +1010,20 @@ static size_t prep_bytes_n()
     return sizeof(float2) * (size_t)(prep_buf_len<N>() + TW + M) + sizeof(float) * (size_t)M;
 }
 
-size_t prep_smem_bytes(int maxfft)
+// Shared memory of a prep CTA for one subharmonic's length.
+size_t prep_smem_bytes(int fftlen, bool folded)
 {
-    size_t b = 0;
-#define JERK_PB(NN)                                  \
-    if (NN <= maxfft && prep_bytes_n<NN>() > b)      \
-        b = prep_bytes_n<NN>();
+    if (folded) {
+        const int M = fftlen / 2;
+        return sizeof(float2) * (size_t)(prep_folded_buf(M) + M) + sizeof(float) * (size_t)M;
+    }
+    switch (fftlen) {
+#define JERK_PB(NN) case NN: return prep_bytes_n<NN>();
     JERK_PB(128) JERK_PB(192) JERK_PB(256) JERK_PB(384) JERK_PB(512) JERK_PB(768)
     JERK_PB(1024) JERK_PB(1280) JERK_PB(2048) JERK_PB(4096) JERK_PB(5120) JERK_PB(7680) JERK_PB(10240) JERK_PB(15360)
 #undef JERK_PB
-    return b;
+    default: return 0;
+    }
 }
 
 // twiddle tables of every supported fftlen's plan (host)
@@ -1557,6 +1032,7 @@ int fft_twiddle_size(int N)
     switch (N) {
 #define JERK_TS(NN) case NN: return FftPlan<NN>::twsize();
     JERK_TS(128) JERK_TS(192) JERK_TS(256) JERK_TS(384) JERK_TS(512) JERK_TS(768)
+    JERK_TS(640) JERK_TS(1536) JERK_TS(1792)
     JERK_TS(1024) JERK_TS(1280) JERK_TS(2048) JERK_TS(4096) JERK_TS(5120) JERK_TS(7680) JERK_TS(10240) JERK_TS(15360)
 #undef JERK_TS
     default: return -1;
@@ -1568,67 +1044,69 @@ void fft_twiddle_table(int N, float2 *out)
     switch (N) {
 #define JERK_TT(NN) case NN: fft_stage_twiddles<NN>(out); break;
     JERK_TT(128) JERK_TT(192) JERK_TT(256) JERK_TT(384) JERK_TT(512) JERK_TT(768)
+    JERK_TT(640) JERK_TT(1536) JERK_TT(1792)
     JERK_TT(1024) JERK_TT(1280) JERK_TT(2048) JERK_TT(4096) JERK_TT(5120) JERK_TT(7680) JERK_TT(10240) JERK_TT(15360)
 #undef JERK_TT
     default: break;
     }
 }
 
-int prep_threads(int maxfft)
+static int prep_threads(int maxfft)
 {
-    // at least the widest FFT plan's thread count, and at least 256
     int t = 256;
 #define JERK_PT(NN)                                  \
     if (NN <= maxfft && FftPlan<NN>::T > t)          \
         t = FftPlan<NN>::T;
-    JERK_PT(128) JERK_PT(192) JERK_PT(256) JERK_PT(384) JERK_PT(512) JERK_PT(768)
-    JERK_PT(1024) JERK_PT(1280) JERK_PT(2048) JERK_PT(4096) JERK_PT(5120) JERK_PT(7680) JERK_PT(10240) JERK_PT(15360)
+    JERK_PT(4096) JERK_PT(5120) JERK_PT(7680) JERK_PT(10240) JERK_PT(15360)
 #undef JERK_PT
     return (t + 31) / 32 * 32;
 }
 
-cudaError_t launch_prep(const SearchDev &P, int maxfft, cudaStream_t st)
+// Function attributes are set when a plan is made (and by the plan-free entry
+// point), not at every launch.
+cudaError_t prep_attrs(int maxfft)
 {
-    const size_t smem = prep_smem_bytes(maxfft);
-    cudaError_t e = cudaFuncSetAttribute(prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess)
-        return e;
-    prep_kernel<<<dim3(P.nb, P.nsubs), prep_threads(maxfft), smem, st>>>(P);
-    return cudaGetLastError();
+    cudaError_t e = cudaSuccess;
+    if (maxfft > kPrepLong) {
+        e = smem_attrs(prep_kernel<true>, false);
+        return e == cudaSuccess ? smem_attrs(prep_group_kernel<true>, false) : e;
+    }
+    e = smem_attrs(prep_kernel<false>, false);
+    return e == cudaSuccess ? smem_attrs(prep_group_kernel<false>, false) : e;
 }
 
-// SMs of the current device (queried once; every B200 has 148)
-static int sm_count()
+// maxfft, smem: the longest fftlen of the launch and the largest
+// prep_smem_bytes over its subharmonics
+cudaError_t launch_prep(const SearchDev &P, int maxfft, size_t smem, cudaStream_t st)
 {
-    static int n = 0;
-    if (n <= 0) {
-        int dev = 0, v = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0)
-            n = v;
-        else
-            return 148;
-    }
-    return n;
+    const dim3 grid(P.nb, P.nsubs);
+    if (maxfft > kPrepLong)
+        prep_kernel<true><<<grid, prep_threads(maxfft), smem, st>>>(P);
+    else
+        prep_kernel<false><<<grid, 256, smem, st>>>(P);
+    return cudaGetLastError();
 }
 
 template <int N>
 static cudaError_t launch_corr_n(const SearchDev &P, const RowGroup &G, int rows, cudaStream_t st)
 {
     const size_t smem = sizeof(float2) * CorrSmem<N>::value;
-    cudaError_t e = cudaFuncSetAttribute(corr_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(corr_kernel<N>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess)
-        return e;
     // a group with fewer rows than two waves of CTAs also splits its rsteps
     const int wave = sm_count() * CorrOcc<N>::value;
     const int split = rows >= 2 * wave ? 1 : std::max(1, std::min(P.nb, (2 * wave + rows - 1) / rows));
     corr_kernel<N><<<dim3(rows, split), FftPlan<N>::T, smem, st>>>(P, G);
     return cudaGetLastError();
+}
+
+cudaError_t corr_attrs(int fftlen)
+{
+    switch (fftlen) {
+#define JERK_CA(NN) case NN: return smem_attrs(corr_kernel<NN>, true);
+    JERK_CA(128) JERK_CA(192) JERK_CA(256) JERK_CA(384) JERK_CA(512) JERK_CA(768) JERK_CA(1024)
+    JERK_CA(1280) JERK_CA(2048) JERK_CA(4096) JERK_CA(5120) JERK_CA(7680) JERK_CA(10240) JERK_CA(15360)
+#undef JERK_CA
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 bool fftlen_supported(int n)
@@ -1668,10 +1146,6 @@ template <int S, bool PF>
 static cudaError_t launch_harmsum_s(const SearchDev &P, const HarmTma &T, cudaStream_t st)
 {
     const size_t smem = harmsum_smem_bytes(P.nsubs, P.numz0);
-    cudaError_t e = cudaFuncSetAttribute(harmsum_kernel<S, 4, PF>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess)
-        return e;
     const dim3 grid((P.corr_uselen + kHarmThreads - 1) / kHarmThreads, P.numw0, P.nb);
     harmsum_kernel<S, 4, PF><<<grid, kHarmThreads, smem, st>>>(P, T);
     return cudaGetLastError();
@@ -1703,89 +1177,26 @@ cudaError_t launch_harmsum(const SearchDev &P, const HarmTma &T, bool prefetch, 
 // plans.  The caller fills M.n, M.P and (corr) M.G; the launchers fill the
 // CTA ranges.
 
-cudaError_t launch_prep_group(GroupLaunch M, int maxfft, cudaStream_t st)
+cudaError_t launch_prep_group(GroupLaunch M, int maxfft, size_t smem, cudaStream_t st)
 {
     if (M.n < 1 || M.n > kMaxGroupPlans)
         return cudaErrorInvalidValue;
     int x = 0;
     for (int i = 0; i < M.n; i++) {
         M.cta0[i] = x;
-        M.ny[i] = 1;
         x += M.P[i].nb * M.P[i].nsubs;
     }
     M.cta0[M.n] = x;
-    const size_t smem = prep_smem_bytes(maxfft);
-    cudaError_t e = cudaFuncSetAttribute(prep_group_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess)
-        return e;
-    prep_group_kernel<<<x, prep_threads(maxfft), smem, st>>>(M);
+    if (maxfft > kPrepLong)
+        prep_group_kernel<true><<<x, prep_threads(maxfft), smem, st>>>(M);
+    else
+        prep_group_kernel<false><<<x, 256, smem, st>>>(M);
     return cudaGetLastError();
-}
-
-template <int N>
-static cudaError_t launch_corr_group_n(GroupLaunch &M, cudaStream_t st)
-{
-    const size_t smem = sizeof(float2) * CorrSmem<N>::value;
-    cudaError_t e = cudaFuncSetAttribute(corr_group_kernel<N>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(corr_group_kernel<N>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess)
-        return e;
-    // the single-plan rule, applied to the wave's rows together: fewer rows
-    // than two waves of CTAs also split their rsteps
-    const int wave = sm_count() * CorrGroupOcc<N>::value;
-    long long total = 0;
-    for (int i = 0; i < M.n; i++)
-        total += M.G[i].rowstart[M.G[i].n];
-    long long x = 0;
-    for (int i = 0; i < M.n; i++) {
-        const int rows = M.G[i].rowstart[M.G[i].n];
-        const int split = total >= 2 * wave ? 1
-                          : std::max(1, std::min(M.P[i].nb, (int)((2 * wave + total - 1) / total)));
-        M.cta0[i] = (int)x;
-        M.ny[i] = split;
-        x += (long long)rows * split;
-    }
-    if (x >= (1ll << 31))
-        return cudaErrorInvalidValue;
-    M.cta0[M.n] = (int)x;
-    corr_group_kernel<N><<<(unsigned)x, FftPlan<N>::T, smem, st>>>(M);
-    return cudaGetLastError();
-}
-
-// CTAs of one full wave of the single-plan correlation / harmonic sum
-int corr_wave_ctas(int fftlen)
-{
-    switch (fftlen) {
-#define JERK_CW(NN) case NN: return sm_count() * (fold_length(NN) ? fold_occ(NN) : CorrOcc<NN>::value);
-    JERK_CW(128) JERK_CW(192) JERK_CW(256) JERK_CW(384) JERK_CW(512) JERK_CW(768)
-    JERK_CW(1024) JERK_CW(1280) JERK_CW(2048) JERK_CW(4096) JERK_CW(5120) JERK_CW(7680)
-    JERK_CW(10240) JERK_CW(15360)
-#undef JERK_CW
-    default: return sm_count();
-    }
 }
 
 int harmsum_wave_ctas(int nstages)
 {
     return sm_count() * (nstages <= 5 ? HarmOcc<5, 4>::value : HarmOcc<6, 4>::value);
-}
-
-cudaError_t launch_corr_group(GroupLaunch M, int fftlen, cudaStream_t st)
-{
-    if (M.n < 1 || M.n > kMaxGroupPlans)
-        return cudaErrorInvalidValue;
-    switch (fftlen) {
-#define JERK_CG(NN) case NN: return launch_corr_group_n<NN>(M, st);
-    JERK_CG(128) JERK_CG(192) JERK_CG(256) JERK_CG(384) JERK_CG(512) JERK_CG(768)
-    JERK_CG(1024) JERK_CG(1280) JERK_CG(2048) JERK_CG(4096) JERK_CG(5120) JERK_CG(7680)
-    JERK_CG(10240) JERK_CG(15360)
-#undef JERK_CG
-    default: return cudaErrorInvalidValue;
-    }
 }
 
 template <int S>
@@ -1797,16 +1208,12 @@ static cudaError_t launch_harmsum_group_s(GroupLaunch &M, cudaStream_t st)
         const SearchDev &P = M.P[i];
         smem = std::max(smem, harmsum_smem_bytes(P.nsubs, P.numz0));
         M.cta0[i] = (int)x;
-        M.ny[i] = (P.corr_uselen + kHarmThreads - 1) / kHarmThreads;
-        x += (long long)M.ny[i] * P.numw0 * P.nb;
+        M.nx[i] = (P.corr_uselen + kHarmThreads - 1) / kHarmThreads;
+        x += (long long)M.nx[i] * P.numw0 * P.nb;
     }
     if (x >= (1ll << 31))
         return cudaErrorInvalidValue;
     M.cta0[M.n] = (int)x;
-    cudaError_t e = cudaFuncSetAttribute(harmsum_group_kernel<S>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess)
-        return e;
     harmsum_group_kernel<S><<<(unsigned)x, kHarmThreads, smem, st>>>(M);
     return cudaGetLastError();
 }
@@ -1836,14 +1243,6 @@ template <int S, int ZT>
 static cudaError_t launch_harmsum_tma_s(const SearchDev &P, const HarmTma &T, cudaStream_t st)
 {
     const size_t smem = harmsum_tma_smem_bytes(T, P.nsubs, P.numz0);
-    cudaError_t e = cudaFuncSetAttribute(harmsum_tma_kernel<S, ZT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(harmsum_tma_kernel<S, ZT>,
-                                 cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess)
-        return e;
     const dim3 grid((P.corr_uselen + kHarmThreads - 1) / kHarmThreads, P.numw0, P.nb);
     harmsum_tma_kernel<S, ZT><<<grid, kHarmThreads, smem, st>>>(P, T);
     return cudaGetLastError();
@@ -1859,6 +1258,30 @@ static cudaError_t launch_harmsum_tma_z(const SearchDev &P, const HarmTma &T, cu
     case 4: return launch_harmsum_tma_s<4, ZT>(P, T, st);
     case 5: return launch_harmsum_tma_s<5, ZT>(P, T, st);
     case 6: return launch_harmsum_tma_s<6, ZT>(P, T, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+template <int S>
+static cudaError_t harmsum_attrs_s(int harm_mode)
+{
+    // (the gather forms keep the default carveout: their gathers live in L1)
+    cudaError_t e = harm_mode >= 4   ? smem_attrs(harmsum_tma_kernel<S, 16>, true)
+                    : harm_mode == 3 ? smem_attrs(harmsum_tma_kernel<S, 8>, true)
+                    : harm_mode == 2 ? smem_attrs(harmsum_kernel<S, 4, true>, false)
+                                     : smem_attrs(harmsum_kernel<S, 4, false>, false);
+    return e == cudaSuccess ? smem_attrs(harmsum_group_kernel<S>, false) : e;
+}
+
+cudaError_t harmsum_attrs(int nstages, int harm_mode)
+{
+    switch (nstages) {
+    case 1: return harmsum_attrs_s<1>(harm_mode);
+    case 2: return harmsum_attrs_s<2>(harm_mode);
+    case 3: return harmsum_attrs_s<3>(harm_mode);
+    case 4: return harmsum_attrs_s<4>(harm_mode);
+    case 5: return harmsum_attrs_s<5>(harm_mode);
+    case 6: return harmsum_attrs_s<6>(harm_mode);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -2002,7 +1425,7 @@ extern "C" int jerk_volume_static(const void *spectrum, long long numbins, long 
         return static_fail(JERK_EINVAL, "null argument");
     const int N = sub->fftlen;
     const int tws = fft_twiddle_size(N);
-    if (N > kStaticMaxFft || tws < 0 || (size_t)tws * sizeof(float2) > kOffData - kOffTw)
+    if (N > kStaticMaxFft || !fftlen_supported(N) || tws < 0 || (size_t)tws * sizeof(float2) > kOffData - kOffTw)
         return static_fail(JERK_EINVAL, "fftlen beyond the static scratch (at most 7680, and supported)");
     if (corr_uselen <= 0 || corr_uselen % 2 || corr_uselen > kStaticMaxUselen)
         return static_fail(JERK_EINVAL, "corr_uselen beyond the static scratch (even, at most 16384)");
@@ -2092,7 +1515,11 @@ extern "C" int jerk_volume_static(const void *spectrum, long long numbins, long 
     P.first_rstep = 0;
     P.nb = 1;
     if (e == cudaSuccess)
-        e = launch_prep(P, N, st);
+        e = prep_attrs(N);
+    if (e == cudaSuccess)
+        e = corr_attrs(N);
+    if (e == cudaSuccess)
+        e = launch_prep(P, N, prep_smem_bytes(N, false), st);
     if (e == cudaSuccess) {
         RowGroup G{};
         G.n = 1;

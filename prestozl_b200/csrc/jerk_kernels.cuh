@@ -6,6 +6,8 @@
 
 #include <cstdint>
 
+#include "jerk.h"
+
 namespace jerk {
 
 constexpr int kMaxSubs = 32;      // numharm <= 32 -> 1 + 31 subharmonic planes
@@ -28,7 +30,43 @@ struct SubDev {
     long long data_off;       // offset (float2) of the b = 0 prepared chunk
     int zinds_off;            // offset of zinds (u16, fundamental numz entries)
     int wind_off;             // offset of wind (int, fundamental numw entries)
+    int cls0, ncls;           // this subharmonic's FoldClass entries (0: not folded)
 };
+
+// Half lengths of the folded correlation (jerk_fold.cu), and the FFT lengths
+// that take it (each of whose halves is among them).
+constexpr int kFoldLens[] = {256, 384, 512, 640, 768, 1024, 1280, 1536, 1792, 2048};
+constexpr int kNumFoldLens = sizeof(kFoldLens) / sizeof(int);
+inline bool folded_fftlen(int N)
+{
+    return N == 512 || N == 768 || N == 1024 || N == 1280 || N == 2048 || N == 4096;
+}
+
+// The rows of one subharmonic that share a half length: they correlate with
+// the transform of `len` consecutive bins of its normalised chunk.
+struct FoldClass {
+    int sub, len;
+    int wstart;               // first bin of the window in the chunk
+    int out0;                 // window position of the good bins' first even output
+    int twoff;                // offset (float2) of FftPlan<len>'s twiddles
+    int stride;               // the subharmonic's plane row stride,
+    long long plane_off;      // b = 0 volume
+    long long plane_size;     // and volume size
+    long long data_off;       // offset (float2) of the b = 0 prepared window
+};
+
+// The kernel rows of one length of a plan, n of them.
+//   folded (len > 0, the half length): row i as [A (len) | B (len)];
+//     map[i] = (class, w * numz + z), class -1 on padding rows;
+//   short, unfolded (len < 0, the negated fftlen): rows of the bank,
+//     map[i] = (subharmonic, w * numz + z).
+struct FoldRows {
+    int len, n;
+    const float2 *rows;
+    const int2 *map;
+    const float2 *tw;         // folded: the half length's two twiddle tables
+};
+constexpr int kMaxRowSets = 16;  // row sets of one plan
 
 // One (rstep, subharmonic): where its chunk starts and how many r it yields.
 struct StepDev {
@@ -56,6 +94,8 @@ struct SearchDev {
     const StepDev *steps;     // [rstep][nsubs], whole spectrum
     const float2 *bank;
     const float2 *twiddles;
+    const FoldClass *classes;
+    const FoldRows *rowsets;
     const uint16_t *zinds;
     const int *wind;
     // per-batch work
@@ -72,6 +112,13 @@ struct SearchDev {
     unsigned int *status;     // bit 0: a subharmonic r index fell outside its row
                               // (or its TMA box); bit 1: a bounded wait on a bulk
                               // or tensor copy gave up
+};
+
+// A bank row to fold (jerk_fold.cu): offset (float2) in the bank, -1 for a
+// padding row; its fftlen; its support, -1 to fold the row's own values.
+struct FoldSrc {
+    long long off;
+    int N, h;
 };
 
 // Tensor maps of the harmonic sum's TMA path: subharmonic s's batch volumes
@@ -108,22 +155,36 @@ struct RowGroup {
 // flat CTA index x belongs to plan i for cta0[i] <= x < cta0[i + 1], and
 // that plan's part runs exactly the CTAs its own launch would run, with its
 // own arguments, so every plan's results are bitwise those of its own
-// launches.  ny[i]: corr -- rstep chunks per kernel row; harmsum -- r blocks
-// per w row.  Passed by value as a __grid_constant__ parameter.
+// launches.  nx[i]: harmsum -- r blocks per w row.  Passed by value as a
+// __grid_constant__ parameter.
 constexpr int kMaxGroupPlans = 12;
 struct GroupLaunch {
     int n;
     int cta0[kMaxGroupPlans + 1];
-    int ny[kMaxGroupPlans];
+    int nx[kMaxGroupPlans];
     SearchDev P[kMaxGroupPlans];
-    RowGroup G[kMaxGroupPlans];
-    const float2 *fold[kMaxGroupPlans];     // corr at fftlen 2048: folded kernel rows
-    const float2 *fold_tw[kMaxGroupPlans];  // and their twiddle tables
 };
-static_assert(sizeof(GroupLaunch) <= 30000, "kernel parameter space");
+
+// The merged correlation launch: CTAs [seg[j].cta0, seg[j + 1].cta0) run row
+// set `set` of plan `plan`, ny rstep chunks per row group.
+struct MultiSeg {
+    int cta0;
+    short plan, set;
+    int ny;
+};
+template <int NP>
+struct MultiLaunch {
+    int n;
+    SearchDev P[NP];
+    MultiSeg seg[NP * kMaxRowSets];
+};
+static_assert(sizeof(GroupLaunch) <= 30000 && sizeof(MultiLaunch<kMaxGroupPlans>) <= 30000,
+              "kernel parameter space");
 
 // Records msg as the text jerk_last_error returns and passes code back.
 int set_error(int code, const char *msg);
+// Bytes of a plan's folded rows of one subharmonic of the generated bank.
+long long fold_bytes(const jerk_subharm &s, int maxnumrs);
 // w_resp_halfwidth(z, w, LOWACC) (src/responses.c:49-84).
 int w_resp_halfwidth_lowacc(double z, double w);
 

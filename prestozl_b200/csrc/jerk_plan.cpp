@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <functional>
 #include <cmath>
 #include <cstdint>
@@ -27,38 +28,37 @@
 #include "jerk_kernels.cuh"
 
 namespace jerk {
-size_t prep_smem_bytes(int maxfft);
-cudaError_t launch_prep(const SearchDev &P, int maxfft, cudaStream_t st);
+size_t prep_smem_bytes(int fftlen, bool folded);
+cudaError_t prep_attrs(int maxfft);
+cudaError_t launch_prep(const SearchDev &P, int maxfft, size_t smem, cudaStream_t st);
+cudaError_t corr_attrs(int fftlen);
 cudaError_t launch_corr(const SearchDev &P, int fftlen, const RowGroup &G, int rows,
                         cudaStream_t st);
+cudaError_t harmsum_attrs(int nstages, int harm_mode);
 cudaError_t launch_harmsum(const SearchDev &P, const HarmTma &T, bool prefetch, cudaStream_t st);
 cudaError_t launch_harmsum_tma(const SearchDev &P, const HarmTma &T, int zt, cudaStream_t st);
 size_t harmsum_tma_smem_bytes(const HarmTma &T, int nsubs, int numz0);
 bool fftlen_supported(int n);
-cudaError_t launch_prep_group(GroupLaunch M, int maxfft, cudaStream_t st);
-cudaError_t launch_corr_group(GroupLaunch M, int fftlen, cudaStream_t st);
+cudaError_t launch_prep_group(GroupLaunch M, int maxfft, size_t smem, cudaStream_t st);
 cudaError_t launch_harmsum_group(GroupLaunch M, int nstages, cudaStream_t st);
 cudaError_t launch_wait_probe(unsigned int *status, cudaStream_t st);
-int corr_wave_ctas(int fftlen);
-bool fold_length(int N);
-int fold_twiddle_size(int N);
-void fold_twiddle_table(int N, float2 *out);
-cudaError_t launch_fold_rows(int N, const float2 *bank, const long long *src, float2 *out,
-                             int nrows, cudaStream_t st);
-cudaError_t launch_corr_fold(int N, const SearchDev &P, const RowGroup &G, int rows,
-                             const float2 *F, const float2 *ftw, cudaStream_t st);
-cudaError_t launch_corr_fold_group(int N, GroupLaunch M, cudaStream_t st);
-
-// The FFT lengths whose correlation runs on folded kernel rows, and a
-// length's slot in a plan's per-length fold arrays (-1: not folded).
-constexpr int kFoldLens[2] = {2048, 1280};
-static int fold_slot(int N)
-{
-    for (int i = 0; i < 2; i++)
-        if (kFoldLens[i] == N)
-            return i;
-    return -1;
-}
+cudaError_t fold_plan_attrs();
+cudaError_t launch_fold_roots(double2 *roots, int n, cudaStream_t st);
+cudaError_t launch_fold_support(const float2 *bank, const long long *src, int nrows, int N,
+                                const double2 *rootsN, int *half, cudaStream_t st);
+cudaError_t launch_fold_rows(const float2 *bank, const FoldSrc *src, int nrows, int L, int maxN,
+                             const double2 *roots, const int *roots_at, float2 *out,
+                             cudaStream_t st);
+int fold_twiddle_size(int L);
+void fold_twiddle_table(int L, float2 *out);
+cudaError_t fold_attrs(int L);
+cudaError_t launch_corr_fold(int L, const SearchDev &P, const FoldRows &R, cudaStream_t st);
+bool multi_takes(const FoldRows &R);
+cudaError_t multi_attrs();
+cudaError_t launch_corr_multi(const SearchDev *P, int np, const int (*sets)[2],
+                              const FoldRows *const *rows, int nsets, cudaStream_t st);
+int fold_cta_rows(int L);
+int fold_wave_ctas(int L);
 int harmsum_wave_ctas(int nstages);
 int fft_twiddle_size(int N);
 void fft_twiddle_table(int N, float2 *out);
@@ -713,6 +713,52 @@ extern "C" int jerk_bank_generate(const jerk_subharm *subs, int nsubs, void *dev
 }
 
 // ---------------------------------------------------------------------------
+// Half lengths of the folded correlation (jerk_fold.cu)
+
+// The window of half length L of a subharmonic whose chunk holds M = fftlen/2
+// bins with the good outputs from bin H (the halfwidth) on, nr/2 of each
+// parity: its first bin (the good bins in the middle, inside the chunk), and
+// the widest support it holds.  L = M holds any row.
+static int fold_window(int M, int H, int nr, int L, int *hmax)
+{
+    const int w = std::max(0, std::min(H - (L - nr / 2) / 2, M - L));
+    *hmax = L >= M ? 1 << 30 : std::min(H - w, L - nr / 2 - (H - w));
+    return w;
+}
+
+// The shortest half length (index into kFoldLens) for a row of support h.
+static int fold_choose(int fftlen, int H, int nr, int h)
+{
+    const int M = fftlen / 2;
+    int hmax = 0;
+    for (int i = 0; i < kNumFoldLens; i++) {
+        fold_window(M, H, nr, kFoldLens[i], &hmax);
+        if (kFoldLens[i] >= M || h <= hmax)
+            return i;
+    }
+    return kNumFoldLens - 1;
+}
+
+// Bytes of the folded rows of one subharmonic whose rows are the generated
+// bank's (jerk_bank_generate), each as wide as its response.
+long long jerk::fold_bytes(const jerk_subharm &s, int maxnumrs)
+{
+    if (!folded_fftlen(s.fftlen))
+        return 0;
+    std::map<int, long long> rows;
+    for (int ii = 0; ii < s.numw; ii++)
+        for (int jj = 0; jj < s.numz; jj++)
+            rows[kFoldLens[fold_choose(s.fftlen, s.halfwidth, maxnumrs,
+                                       w_resp_halfwidth(-s.zmax + jj * kDZ, -s.wmax + ii * kDW))]]++;
+    long long b = 0;
+    for (auto &kv : rows) {
+        const long long per = fold_cta_rows(kv.first);
+        b += (kv.second + per - 1) / per * per * 2 * kv.first * (long long)sizeof(float2);
+    }
+    return b;
+}
+
+// ---------------------------------------------------------------------------
 // The plan
 
 // per kernel class: launches, device time (CUDA events on the plan's stream,
@@ -734,6 +780,7 @@ struct jerk_plan {
     bool own_stream = false;
     jerk_obs obs{};
     int nsubs = 0, maxfft = 0, batch = 8;
+    size_t prep_smem = 0;
     // harmonic-sum kernel (jerk_config.harm_mode, resolved): 1 gather,
     // 2 gather + TMA L2 prefetch, 3 / 4 TMA tiles of harm_tile (8 / 16) rows;
     // tma holds the tensor maps of modes 2-4
@@ -751,16 +798,20 @@ struct jerk_plan {
     std::vector<jerk_subharm> subs;
     std::vector<SubDev> hsubs;
     std::vector<StepDev> hsteps;  // [nrsteps][nsubs]
-    std::map<int, std::vector<int>> groups;  // fftlen -> subs
+    std::map<int, std::vector<int>> groups;  // fftlen -> subs, the long unfolded lengths
+    std::vector<FoldRows> rowsets;  // folded half lengths, then short unfolded lengths
+    std::vector<char> own_launch;   // per row set: fills the GPU in a launch of its own
+    FoldRows *d_rowsets = nullptr;
+    std::vector<FoldClass> fold_classes;
+    std::vector<std::vector<double>> class_rows;  // [half length index][class] live rows
     // device
     float2 *d_bank = nullptr;
     bool own_bank = false;
     float2 *d_tw = nullptr;
-    // per folded length (kFoldLens): the rows folded for the half-length
-    // correlation, and the offset of its twiddle tables in d_tw
-    float2 *d_fold[2] = {nullptr, nullptr};
-    long long fold_floats2[2] = {0, 0};
-    int fold_twoff[2] = {-1, -1};
+    float2 *d_fold = nullptr;   // every half length's folded rows
+    int2 *d_foldmap = nullptr;  // and their maps
+    long long fold_f2 = 0;
+    FoldClass *d_classes = nullptr;
     SubDev *d_subs = nullptr;
     StepDev *d_steps = nullptr;
     uint16_t *d_zinds = nullptr;
@@ -919,8 +970,10 @@ static void plan_free_device(jerk_plan *p)
     if (p->own_bank)
         cudaFree(p->d_bank);
     cudaFree(p->d_tw);
-    cudaFree(p->d_fold[0]);
-    cudaFree(p->d_fold[1]);
+    cudaFree(p->d_fold);
+    cudaFree(p->d_foldmap);
+    cudaFree(p->d_classes);
+    cudaFree(p->d_rowsets);
     cudaFree(p->d_subs);
     cudaFree(p->d_steps);
     cudaFree(p->d_zinds);
@@ -1065,6 +1118,203 @@ static int build_harm_tma(jerk_plan *p, bool in_smem)
     return JERK_OK;
 }
 
+// The plan's row sets.  Fold the bank's rows of every folded length: measure
+// each row's support, choose its half length, lay out the classes (their
+// prepared windows from *data_off on) and write the folded rows, class after
+// class, longest half length first; then the maps of the short lengths that
+// do not fold (fftlen 128 to 384).
+static int fold_bank(jerk_plan *p, const std::vector<int> &maxnumrs, long long *data_off)
+{
+    std::map<int, std::vector<int>> subs_of;  // fftlen -> subharmonics
+    for (int s = 0; s < p->nsubs; s++)
+        if (folded_fftlen(p->subs[s].fftlen))
+            subs_of[p->subs[s].fftlen].push_back(s);
+    cudaStream_t st = p->stream;
+    JERK_CUDA(fold_plan_attrs());
+
+    // root tables of every length the folding may take
+    int roots_at[4096 / 128 + 1];
+    int nroots = 0, maxN = 0;
+    std::fill(std::begin(roots_at), std::end(roots_at), -1);
+    std::vector<int> lens(std::begin(kFoldLens), std::end(kFoldLens));
+    for (auto &kv : subs_of) {
+        lens.push_back(kv.first);
+        maxN = std::max(maxN, kv.first);
+    }
+    for (int n : lens)
+        if (n <= maxN && roots_at[n / 128] < 0) {
+            roots_at[n / 128] = nroots;
+            nroots += n;
+        }
+
+    // supports
+    long long nrows = 0;
+    for (auto &kv : subs_of)
+        for (int s : kv.second)
+            nrows += (long long)p->subs[s].numw * p->subs[s].numz;
+    if (nrows > INT_MAX)
+        return fail(JERK_EUNSUPPORTED, "too many kernel rows");
+    std::vector<long long> src;
+    src.reserve(nrows);
+    std::vector<long long> first_row(p->nsubs, 0);
+    for (auto &kv : subs_of)
+        for (int s : kv.second) {
+            first_row[s] = (long long)src.size();
+            const long long n = (long long)p->subs[s].numw * p->subs[s].numz;
+            for (long long r = 0; r < n; r++)
+                src.push_back(p->hsubs[s].kern_off + r * kv.first);
+        }
+    // scratch of this function: roots, supports, then the row sources (the
+    // padding adds at most three rows a class); freed on every path (cudaFree
+    // waits for the kernels reading it)
+    struct Scratch {
+        char *p = nullptr;
+        ~Scratch() { cudaFree(p); }
+    } sc;
+    const size_t pad_rows = 4 * (size_t)kNumFoldLens * p->nsubs;
+    const size_t b_roots = sizeof(double2) * nroots, b_at = 256,
+                 b_src = sizeof(long long) * (size_t)nrows,
+                 b_fsrc = sizeof(FoldSrc) * ((size_t)nrows + pad_rows),
+                 b_half = sizeof(int) * (size_t)nrows;
+    static_assert(sizeof(roots_at) <= 256, "roots_at");
+    JERK_CUDA(cudaMalloc(&sc.p, b_roots + b_at + b_src + b_fsrc + b_half + 16));
+    double2 *d_roots = (double2 *)sc.p;
+    int *d_roots_at = (int *)(sc.p + b_roots);
+    long long *d_src = (long long *)(sc.p + b_roots + b_at);
+    FoldSrc *d_fsrc = (FoldSrc *)(sc.p + b_roots + b_at + b_src);
+    int *d_half = (int *)(sc.p + b_roots + b_at + b_src + b_fsrc);
+    for (int n : lens)
+        if (n <= maxN && roots_at[n / 128] >= 0)
+            JERK_CUDA(launch_fold_roots(d_roots + roots_at[n / 128], n, st));
+    JERK_CUDA(cudaMemcpyAsync(d_roots_at, roots_at, sizeof(roots_at), cudaMemcpyHostToDevice, st));
+    JERK_CUDA(cudaMemcpyAsync(d_src, src.data(), sizeof(long long) * nrows, cudaMemcpyHostToDevice,
+                              st));
+    for (auto &kv : subs_of) {
+        const long long at = first_row[kv.second.front()];
+        long long n = 0;
+        for (int s : kv.second)
+            n += (long long)p->subs[s].numw * p->subs[s].numz;
+        JERK_CUDA(launch_fold_support(p->d_bank, d_src + at, (int)n, kv.first,
+                                      d_roots + roots_at[kv.first / 128], d_half + at, st));
+    }
+    std::vector<int> half(nrows);
+    JERK_CUDA(cudaMemcpyAsync(half.data(), d_half, sizeof(int) * nrows, cudaMemcpyDeviceToHost, st));
+    JERK_CUDA(cudaStreamSynchronize(st));
+
+    // classes: a subharmonic's rows of one half length
+    struct Built {
+        std::vector<FoldSrc> src;
+        std::vector<int2> map;
+        int maxN = 0;
+    };
+    std::vector<Built> built(kNumFoldLens);
+    p->class_rows.assign(kNumFoldLens, {});
+    for (int s = 0; s < p->nsubs; s++) {
+        const jerk_subharm &sh = p->subs[s];
+        if (!folded_fftlen(sh.fftlen))
+            continue;
+        SubDev &d = p->hsubs[s];
+        const int M = sh.fftlen / 2, rows = sh.numw * sh.numz;
+        const int *h = half.data() + first_row[s];
+        std::vector<std::vector<int>> of(kNumFoldLens);
+        for (int r = 0; r < rows; r++)
+            of[fold_choose(sh.fftlen, sh.halfwidth, maxnumrs[s], h[r])].push_back(r);
+        d.cls0 = (int)p->fold_classes.size();
+        for (int i = 0; i < kNumFoldLens; i++) {
+            if (of[i].empty())
+                continue;
+            FoldClass c{};
+            int hmax = 0;
+            c.sub = s;
+            c.len = kFoldLens[i];
+            c.wstart = fold_window(M, sh.halfwidth, maxnumrs[s], c.len, &hmax);
+            c.out0 = sh.halfwidth - c.wstart;
+            c.stride = d.stride;
+            c.plane_off = d.plane_off;
+            c.plane_size = d.plane_size;
+            c.data_off = *data_off;
+            *data_off += (long long)c.len * p->batch;
+            const int ci = (int)p->fold_classes.size();
+            Built &B = built[i];
+            B.maxN = std::max(B.maxN, sh.fftlen);
+            for (int r : of[i]) {
+                B.src.push_back({d.kern_off + (long long)r * sh.fftlen, sh.fftlen,
+                                 c.len == M ? -1 : h[r]});
+                B.map.push_back(make_int2(ci, r));
+            }
+            while (B.src.size() % fold_cta_rows(c.len)) {
+                B.src.push_back({-1, sh.fftlen, -1});
+                B.map.push_back(make_int2(-1, 0));
+            }
+            p->fold_classes.push_back(c);
+            p->class_rows[i].resize(p->fold_classes.size(), 0.0);
+            p->class_rows[i][ci] = (double)of[i].size();
+        }
+        d.ncls = (int)p->fold_classes.size() - d.cls0;
+    }
+
+    std::map<int, std::vector<int2>> shorts;  // unfolded fftlen -> map
+    for (int s = 0; s < p->nsubs; s++) {
+        const jerk_subharm &sh = p->subs[s];
+        if (!folded_fftlen(sh.fftlen) && sh.fftlen < 512)
+            for (int r = 0; r < sh.numw * sh.numz; r++)
+                shorts[sh.fftlen].push_back(make_int2(s, r));
+    }
+    long long total = 0, f2 = 0;
+    for (int i = 0; i < kNumFoldLens; i++) {
+        total += (long long)built[i].src.size();
+        f2 += (long long)built[i].src.size() * 2 * kFoldLens[i];
+    }
+    for (auto &kv : shorts)
+        total += (long long)kv.second.size();
+    p->fold_f2 = f2;
+    if (f2)
+        JERK_CUDA(cudaMalloc(&p->d_fold, sizeof(float2) * f2));
+    if (total)
+        JERK_CUDA(cudaMalloc(&p->d_foldmap, sizeof(int2) * total));
+    long long row = 0, at = 0;
+    for (int i = kNumFoldLens - 1; i >= 0; i--) {
+        const Built &B = built[i];
+        const long long n = (long long)B.src.size();
+        if (!n)
+            continue;
+        const int L = kFoldLens[i];
+        JERK_CUDA(cudaMemcpyAsync(d_fsrc + row, B.src.data(), sizeof(FoldSrc) * n,
+                                  cudaMemcpyHostToDevice, st));
+        JERK_CUDA(cudaMemcpyAsync(p->d_foldmap + row, B.map.data(), sizeof(int2) * n,
+                                  cudaMemcpyHostToDevice, st));
+        JERK_CUDA(launch_fold_rows(p->d_bank, d_fsrc + row, (int)n, L, B.maxN, d_roots, d_roots_at,
+                                   p->d_fold + at, st));
+        FoldRows R{};
+        R.len = L;
+        R.n = (int)n;
+        R.rows = p->d_fold + at;
+        R.map = p->d_foldmap + row;
+        p->rowsets.push_back(R);
+        // two waves of CTAs by themselves gain nothing from the merged launch
+        p->own_launch.push_back(!multi_takes(R) ||
+                                n / fold_cta_rows(L) >= 2 * fold_wave_ctas(L));
+        row += n;
+        at += n * 2 * L;
+    }
+    for (auto kv = shorts.rbegin(); kv != shorts.rend(); ++kv) {
+        const long long n = (long long)kv->second.size();
+        JERK_CUDA(cudaMemcpyAsync(p->d_foldmap + row, kv->second.data(), sizeof(int2) * n,
+                                  cudaMemcpyHostToDevice, st));
+        FoldRows R{};
+        R.len = -kv->first;
+        R.n = (int)n;
+        R.map = p->d_foldmap + row;
+        p->rowsets.push_back(R);
+        p->own_launch.push_back(0);
+        row += n;
+    }
+    if (p->rowsets.size() > (size_t)kMaxRowSets)
+        return fail(JERK_EUNSUPPORTED, "too many row sets");
+    // the host tables above are pageable: copied before these calls returned
+    return JERK_OK;
+}
+
 extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk_subharm *subs,
                                 int nsubs, const jerk_config *cfg)
 {
@@ -1186,18 +1436,21 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
         d.zlo = calc_required_z(d.harm_fract, obs->zlo);
         d.wlo = calc_required_w(d.harm_fract, obs->wlo);
         d.pownorm = (float)(1.0 / (double)(sh.fftlen * sh.fftlen));
-        if (!twoff.count(sh.fftlen)) {
+        const bool folded = folded_fftlen(sh.fftlen);
+        if (!folded && !twoff.count(sh.fftlen)) {
             twoff[sh.fftlen] = twtotal;
             twtotal += fft_twiddle_size(sh.fftlen);
         }
-        d.twoff = twoff[sh.fftlen];
+        d.twoff = folded ? 0 : twoff[sh.fftlen];
+        d.cls0 = d.ncls = 0;  // set with the folded rows below
         d.kern_off = kern_off;
         kern_off += (long long)sh.numw * sh.numz * sh.fftlen;
         d.plane_size = (long long)sh.numw * sh.numz * d.stride;
         d.plane_off = plane_off;
         plane_off += d.plane_size * p->batch;
         d.data_off = data_off;
-        data_off += (long long)sh.fftlen * p->batch;
+        if (!folded)
+            data_off += (long long)sh.fftlen * p->batch;
         d.zinds_off = zinds_off;
         d.wind_off = wind_off;
         // zinds (src/accel_utils.c:1124-1130) and wind (src/accel_utils.c:1362-1364)
@@ -1220,33 +1473,13 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
         zinds_off += obs->numz;
         wind_off += subs[0].numw;
         p->maxfft = std::max(p->maxfft, sh.fftlen);
-        p->groups[sh.fftlen].push_back(s);
+        p->prep_smem = std::max(p->prep_smem, prep_smem_bytes(sh.fftlen, folded));
+        if (!folded && sh.fftlen > 512)
+            p->groups[sh.fftlen].push_back(s);
     }
     p->plane_floats = plane_off;
-    p->prepped_f2 = data_off;
     if (plane_off >= (1LL << 32))
         return bail(fail(JERK_EINVAL, "ffdot volumes of one batch exceed 2^32 floats: lower batch_rsteps"));
-
-    // twiddles: exp(-2 pi i m / N), double on the host
-    std::vector<float2> tw;
-    {
-        std::vector<std::pair<int, int>> byoff;
-        for (auto &kv : twoff)
-            byoff.push_back({kv.second, kv.first});
-        std::sort(byoff.begin(), byoff.end());
-        for (auto &o : byoff)
-            append_twiddles(o.second, tw);
-    }
-    for (int f = 0; f < 2; f++) {
-        const int N = kFoldLens[f];
-        if (!p->groups.count(N))
-            continue;
-        twtotal += twtotal & 1;  // 16-byte aligned tables
-        p->fold_twoff[f] = twtotal;
-        tw.resize(twtotal + fold_twiddle_size(N));
-        fold_twiddle_table(N, tw.data() + twtotal);
-        twtotal += fold_twiddle_size(N);
-    }
 
 #define JERK_CUDA_B(call)                                \
     do {                                                 \
@@ -1270,40 +1503,56 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
                                         sizeof(float2) * n, cudaMemcpyHostToDevice, p->stream));
         }
     }
-    JERK_CUDA_B(cudaMalloc(&p->d_tw, sizeof(float2) * twtotal));
-    JERK_CUDA_B(cudaMemcpyAsync(p->d_tw, tw.data(), sizeof(float2) * twtotal,
-                                cudaMemcpyHostToDevice, p->stream));
-    // folded lengths: fold the bank's rows once for the half-length
-    // correlation (the bank must be complete when the plan is made;
+    // folded rows (the bank must be complete when the plan is made;
     // jerk_bank_generate returns once it is)
-    std::vector<long long> fold_src[2];
-    // device copies of the source-row tables, freed when this function
-    // returns on any path (cudaFree waits for the fold kernels reading them)
-    struct FoldSrc {
-        long long *d[2] = {nullptr, nullptr};
-        ~FoldSrc()
-        {
-            cudaFree(d[0]);
-            cudaFree(d[1]);
-        }
-    } d_fold_src;
-    for (int f = 0; f < 2; f++) {
-        const int N = kFoldLens[f];
-        if (p->fold_twoff[f] < 0)
+    {
+        const int rc = fold_bank(p, maxnumrs, &data_off);
+        if (rc != JERK_OK)
+            return bail(rc);
+    }
+    p->prepped_f2 = data_off;
+
+    // twiddles: exp(-2 pi i m / N), double on the host
+    std::vector<float2> tw;
+    {
+        std::vector<std::pair<int, int>> byoff;
+        for (auto &kv : twoff)
+            byoff.push_back({kv.second, kv.first});
+        std::sort(byoff.begin(), byoff.end());
+        for (auto &o : byoff)
+            append_twiddles(o.second, tw);
+    }
+    std::map<int, int> fold_tw;
+    for (const FoldRows &R : p->rowsets) {
+        if (R.len < 0)
             continue;
-        for (int s : p->groups[N]) {
-            const long long nrow = (long long)subs[s].numw * subs[s].numz;
-            for (long long r = 0; r < nrow; r++)
-                fold_src[f].push_back(p->hsubs[s].kern_off + r * N);
-        }
-        p->fold_floats2[f] = (long long)fold_src[f].size() * N;
-        JERK_CUDA_B(cudaMalloc(&p->d_fold[f], sizeof(float2) * p->fold_floats2[f]));
-        JERK_CUDA_B(cudaMalloc(&d_fold_src.d[f], sizeof(long long) * fold_src[f].size()));
-        JERK_CUDA_B(cudaMemcpyAsync(d_fold_src.d[f], fold_src[f].data(),
-                                    sizeof(long long) * fold_src[f].size(), cudaMemcpyHostToDevice,
+        const int at = (int)tw.size();
+        for (FoldClass &c : p->fold_classes)
+            if (c.len == R.len)
+                c.twoff = at;
+        append_twiddles(R.len, tw);
+        tw.resize(tw.size() + (tw.size() & 1));  // 16-byte aligned tables
+        fold_tw[R.len] = (int)tw.size();
+        tw.resize(tw.size() + fold_twiddle_size(R.len));
+        fold_twiddle_table(R.len, tw.data() + fold_tw[R.len]);
+    }
+    JERK_CUDA_B(cudaMalloc(&p->d_tw, sizeof(float2) * (tw.size() + 1)));
+    JERK_CUDA_B(cudaMemcpyAsync(p->d_tw, tw.data(), sizeof(float2) * tw.size(),
+                                cudaMemcpyHostToDevice, p->stream));
+    for (FoldRows &R : p->rowsets)
+        if (R.len > 0)
+            R.tw = p->d_tw + fold_tw[R.len];
+    if (!p->rowsets.empty()) {
+        JERK_CUDA_B(cudaMalloc(&p->d_rowsets, sizeof(FoldRows) * p->rowsets.size()));
+        JERK_CUDA_B(cudaMemcpyAsync(p->d_rowsets, p->rowsets.data(),
+                                    sizeof(FoldRows) * p->rowsets.size(), cudaMemcpyHostToDevice,
                                     p->stream));
-        JERK_CUDA_B(launch_fold_rows(N, p->d_bank, d_fold_src.d[f], p->d_fold[f],
-                                     (int)fold_src[f].size(), p->stream));
+    }
+    if (!p->fold_classes.empty()) {
+        JERK_CUDA_B(cudaMalloc(&p->d_classes, sizeof(FoldClass) * p->fold_classes.size()));
+        JERK_CUDA_B(cudaMemcpyAsync(p->d_classes, p->fold_classes.data(),
+                                    sizeof(FoldClass) * p->fold_classes.size(), cudaMemcpyHostToDevice,
+                                    p->stream));
     }
     JERK_CUDA_B(cudaMalloc(&p->d_subs, sizeof(SubDev) * nsubs));
     JERK_CUDA_B(cudaMemcpyAsync(p->d_subs, p->hsubs.data(), sizeof(SubDev) * nsubs,
@@ -1335,6 +1584,14 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
         if (!p->tma)
             p->harm_mode = 1;  // no tensor maps here: the plain gather kernel
     }
+    JERK_CUDA_B(prep_attrs(p->maxfft));
+    JERK_CUDA_B(harmsum_attrs(obs->numharmstages, p->harm_mode));
+    for (auto &kv : p->groups)
+        JERK_CUDA_B(corr_attrs(kv.first));
+    for (const FoldRows &R : p->rowsets)
+        if (R.len > 0)
+            JERK_CUDA_B(fold_attrs(R.len));
+    JERK_CUDA_B(multi_attrs());
     JERK_CUDA_B(cudaEventCreateWithFlags(&p->ev_done, cudaEventDisableTiming));
     for (int i = 0; i < jerk_plan::kRing; i++)
         JERK_CUDA_B(cudaEventCreateWithFlags(&p->ev_batch[i], cudaEventDisableTiming));
@@ -1393,6 +1650,8 @@ static SearchDev make_args(const jerk_plan *p, const float2 *spec)
     a.steps = p->d_steps;
     a.bank = p->d_bank;
     a.twiddles = p->d_tw;
+    a.classes = p->d_classes;
+    a.rowsets = p->d_rowsets;
     a.zinds = p->d_zinds;
     a.wind = p->d_wind;
     a.prepped = p->d_prepped;
@@ -1412,16 +1671,34 @@ static inline double fft_flops(int n)
     return 5.0 * n * log2((double)n);
 }
 
-// The plan's own correlation launch for one FFT length (the folded form at
-// the folded lengths).
-static cudaError_t launch_corr_of(const jerk_plan *p, const SearchDev &a, int N, const RowGroup &G,
-                                  cudaStream_t st)
+// algorithmic traffic and operations of one row set over a batch: each row
+// read once, each prepared window once, every good power written once; the
+// product and the transforms
+static void rowset_work(const jerk_plan *p, const SearchDev &a, const FoldRows &R, double *bytes,
+                        double *flops)
 {
-    const int f = fold_slot(N);
-    if (f >= 0 && p->d_fold[f])
-        return launch_corr_fold(N, a, G, G.rowstart[G.n], p->d_fold[f], p->d_tw + p->fold_twoff[f],
-                                st);
-    return launch_corr(a, N, G, G.rowstart[G.n], st);
+    auto add = [&](double rows, int sub, double row_f2, double fl) {
+        double numrs = 0;
+        for (int b = 0; b < a.nb; b++)
+            numrs += p->hsteps[(size_t)(a.first_rstep + b) * p->nsubs + sub].numrs;
+        *bytes += rows * row_f2 * 8.0 + a.nb * row_f2 * 4.0 + rows * numrs * 4.0;
+        *flops += rows * (a.nb * fl + numrs * 3.0);
+    };
+    if (R.len < 0) {
+        for (int s = 0; s < p->nsubs; s++)
+            if (p->subs[s].fftlen == -R.len)
+                add((double)p->subs[s].numw * p->subs[s].numz, s, -R.len,
+                    fft_flops(-R.len) + 6.0 * -R.len);
+        return;
+    }
+    int li = 0;
+    while (kFoldLens[li] != R.len)
+        li++;
+    const std::vector<double> &rows = p->class_rows[li];
+    for (size_t c = 0; c < rows.size(); c++)
+        if (rows[c] > 0.0)
+            add(rows[c], p->fold_classes[c].sub, 2.0 * R.len,
+                2 * (fft_flops(R.len) + 6.0 * R.len));
 }
 
 // The rows of the subharmonics subs (one fftlen), numbered consecutively.
@@ -1450,7 +1727,7 @@ static int run_volumes(jerk_plan *p, SearchDev &a)
             flops += (double)a.nb * fft_flops(N);
         }
         const int tok = launch_begin(p, kclass(p, "prep"), bytes, flops);
-        cudaError_t e = launch_prep(a, p->maxfft, p->stream);
+        cudaError_t e = launch_prep(a, p->maxfft, p->prep_smem, p->stream);
         launch_end(p, tok);
         if (e != cudaSuccess)
             return cuda_fail(e, "prep_kernel");
@@ -1472,10 +1749,40 @@ static int run_volumes(jerk_plan *p, SearchDev &a)
             flops += nrow * a.nb * (fft_flops(N) + 6.0 * N) + nrow * numrs * 3.0;
         }
         const int tok = launch_begin(p, kclass(p, "corr_" + std::to_string(N)), bytes, flops);
-        e = launch_corr_of(p, a, N, G, p->stream);
+        e = launch_corr(a, N, G, G.rowstart[G.n], p->stream);
         launch_end(p, tok);
         if (e != cudaSuccess)
             return cuda_fail(e, "corr_kernel");
+    }
+    int sets[kMaxRowSets][2], nsets = 0;
+    const FoldRows *rows[kMaxRowSets];
+    double mbytes = 0, mflops = 0;
+    for (size_t i = 0; i < p->rowsets.size(); i++) {
+        const FoldRows &R = p->rowsets[i];
+        if (!p->own_launch[i]) {
+            if (p->profiling)
+                rowset_work(p, a, R, &mbytes, &mflops);
+            sets[nsets][0] = 0;
+            sets[nsets][1] = (int)i;
+            rows[nsets++] = &R;
+            continue;
+        }
+        double bytes = 0, flops = 0;
+        if (p->profiling)
+            rowset_work(p, a, R, &bytes, &flops);
+        const int tok = launch_begin(p, kclass(p, "corr_fold_" + std::to_string(R.len)), bytes,
+                                     flops);
+        e = launch_corr_fold(R.len, a, R, p->stream);
+        launch_end(p, tok);
+        if (e != cudaSuccess)
+            return cuda_fail(e, "corr_fold_kernel");
+    }
+    if (nsets) {
+        const int tok = launch_begin(p, kclass(p, "corr_multi"), mbytes, mflops);
+        e = launch_corr_multi(&a, 1, sets, rows, nsets, p->stream);
+        launch_end(p, tok);
+        if (e != cudaSuccess)
+            return cuda_fail(e, "corr_multi_kernel");
     }
     return JERK_OK;
 }
@@ -1791,6 +2098,7 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
     cudaStream_t st = p0->stream;
     const int n = (int)W.size();
     int maxfft = 0;
+    size_t prep_smem = 0;
     double pbytes = 0, pflops = 0;
     for (jerk_plan *p : W) {
         jerk_plan::Pass &ps = p->pass;
@@ -1800,6 +2108,7 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
         a.planes = p->d_planes;
         a.rinds = p->d_rinds;
         maxfft = std::max(maxfft, p->maxfft);
+        prep_smem = std::max(prep_smem, p->prep_smem);
         for (int s = 0; s < p->nsubs; s++) {
             const int N = p->subs[s].fftlen;
             pbytes += (double)a.nb * (N / 2 * 8.0 + N / 2 * 8.0);
@@ -1817,63 +2126,55 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
     for (int i = 0; i < n; i++)
         M.P[i] = W[i]->pass.a;
     int tok = launch_begin(p0, kclass(p0, "wave_prep"), pbytes, pflops);
-    cudaError_t e = launch_prep_group(M, maxfft, st);
+    cudaError_t e = launch_prep_group(M, maxfft, prep_smem, st);
     launch_end(p0, tok);
     if (e != cudaSuccess)
         return fail_all(e, "prep_group_kernel");
 
-    // correlation: one launch per FFT length over every plan that has it; a
-    // plan whose rows of that length fill the GPU twice over by themselves
-    // gains nothing from merging and takes its own (faster) launch
-    std::map<int, std::vector<int>> byN;
+    // correlation: the row sets that fill the GPU twice over by themselves
+    // (and the long unfolded lengths) in their plan's own launches, all the
+    // others of every plan in one
+    int sets[kMaxGroupPlans * kMaxRowSets][2], nsets = 0;
+    const FoldRows *rows[kMaxGroupPlans * kMaxRowSets];
+    double mbytes = 0, mflops = 0;
     for (int i = 0; i < n; i++) {
         jerk_plan *p = W[i];
+        const SearchDev &a = p->pass.a;
         for (auto &kv : p->groups) {
             const RowGroup G = row_group(p, kv.second);
-            if (G.rowstart[G.n] < 2 * corr_wave_ctas(kv.first)) {
-                byN[kv.first].push_back(i);
-                continue;
-            }
             tok = launch_begin(p0, kclass(p0, "wave_corr_" + std::to_string(kv.first)), 0.0, 0.0);
-            e = launch_corr_of(p, p->pass.a, kv.first, G, st);
+            e = launch_corr(a, kv.first, G, G.rowstart[G.n], st);
             launch_end(p0, tok);
             if (e != cudaSuccess)
                 return fail_all(e, "corr_kernel");
         }
-    }
-    for (auto &kv : byN) {
-        const int N = kv.first;
-        GroupLaunch C{};
-        C.n = (int)kv.second.size();
-        double bytes = 0, flops = 0;
-        const int f = fold_slot(N);
-        bool fold = f >= 0;
-        for (int j = 0; j < C.n; j++) {
-            jerk_plan *p = W[kv.second[j]];
-            const SearchDev &a = p->pass.a;
-            C.P[j] = a;
-            C.G[j] = row_group(p, p->groups.at(N));
-            // at a folded length every plan has folded rows (made with the
-            // plan), so the merged launch computes exactly what the plan's
-            // own launch does
-            fold = fold && p->d_fold[f];
-            C.fold[j] = f >= 0 ? p->d_fold[f] : nullptr;
-            C.fold_tw[j] = f >= 0 && p->d_fold[f] ? p->d_tw + p->fold_twoff[f] : nullptr;
-            for (int g = 0; g < C.G[j].n; g++) {
-                const int s = C.G[j].sub[g];
-                const double nrow = (double)p->subs[s].numw * p->subs[s].numz;
-                double numrs = 0;
-                for (int b = 0; b < a.nb; b++)
-                    numrs += p->hsteps[(size_t)(a.first_rstep + b) * p->nsubs + s].numrs;
-                bytes += nrow * N * 8.0 + a.nb * N / 2 * 8.0 + nrow * numrs * 4.0;
-                flops += nrow * a.nb * (fft_flops(N) + 6.0 * N) + nrow * numrs * 3.0;
+        for (size_t k = 0; k < p->rowsets.size(); k++) {
+            const FoldRows &R = p->rowsets[k];
+            double bytes = 0, flops = 0;
+            if (p0->profiling)
+                rowset_work(p, a, R, &bytes, &flops);
+            if (!p->own_launch[k]) {
+                sets[nsets][0] = i;
+                sets[nsets][1] = (int)k;
+                rows[nsets++] = &R;
+                mbytes += bytes;
+                mflops += flops;
+                continue;
             }
+            tok = launch_begin(p0, kclass(p0, "wave_corr_fold_" + std::to_string(R.len)), bytes,
+                               flops);
+            e = launch_corr_fold(R.len, a, R, st);
+            launch_end(p0, tok);
+            if (e != cudaSuccess)
+                return fail_all(e, "corr_fold_kernel");
         }
-        tok = launch_begin(p0, kclass(p0, "wave_corr_" + std::to_string(N)), bytes, flops);
-        e = fold ? launch_corr_fold_group(N, C, st) : launch_corr_group(C, N, st);
+    }
+    if (nsets) {
+        tok = launch_begin(p0, kclass(p0, "wave_corr_multi"), mbytes, mflops);
+        e = launch_corr_multi(M.P, n, sets, rows, nsets, st);
         launch_end(p0, tok);
         if (e != cudaSuccess)
-            return fail_all(e, "corr_group_kernel");
+            return fail_all(e, "corr_multi_kernel");
     }
 
     // harmonic sums: the gather form merged per stage count; plans tuned to
@@ -2196,7 +2497,7 @@ extern "C" long long jerk_plan_device_bytes(const jerk_plan *p)
                        sizeof(float2) * p->prepped_f2 +
                        (sizeof(unsigned long long) + sizeof(float)) * p->max_hits +
                        sizeof(StepDev) * p->hsteps.size() + sizeof(float2) * p->spec_cap +
-                       sizeof(float2) * (p->fold_floats2[0] + p->fold_floats2[1]) +
+                       sizeof(float2) * p->fold_f2 +
                        (p->own_bank ? sizeof(float2) * jerk_bank_elements(p->subs.data(), p->nsubs)
                                     : 0));
 }
