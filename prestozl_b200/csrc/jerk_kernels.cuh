@@ -12,6 +12,7 @@ namespace jerk {
 
 constexpr int kMaxSubs = 32;      // numharm <= 32 -> 1 + 31 subharmonic planes
 constexpr int kMaxStages = 6;
+constexpr int kPlaneAlign = 8;    // volume rows start on 32-byte sectors
 
 // One subharmonic (harmnum / numharm) as laid out on the device.
 struct SubDev {
@@ -20,7 +21,7 @@ struct SubDev {
     int numz, numw;           // kernel grid (numkern_zdim, numkern_wdim)
     int fftlen;
     int halfwidth;            // kern[0][0].kern_half_width (bins)
-    int stride;               // plane row stride in floats (>= max numrs, multiple of 4)
+    int stride;               // plane row stride in floats (>= max numrs, multiple of kPlaneAlign)
     int zlo, wlo;             // lowest z / w of this subharmonic's volume
     float pownorm;            // (float)(1.0 / (fftlen * fftlen))
     int twoff;                // offset (float2) of this fftlen's twiddle table

@@ -36,6 +36,10 @@ cudaError_t launch_corr(const SearchDev &P, int fftlen, const RowGroup &G, int r
                         cudaStream_t st);
 cudaError_t harmsum_attrs(int nstages, int harm_mode);
 cudaError_t launch_harmsum(const SearchDev &P, const HarmTma &T, bool prefetch, cudaStream_t st);
+cudaError_t harm_ring_attrs(int nstages);
+cudaError_t launch_harm_ring(const SearchDev &P, cudaStream_t st);
+bool harm_ring_wins(double bytes);
+cudaError_t launch_harm_ring_group(const GroupLaunch &M, int nstages, cudaStream_t st);
 cudaError_t launch_harmsum_tma(const SearchDev &P, const HarmTma &T, int zt, cudaStream_t st);
 size_t harmsum_tma_smem_bytes(const HarmTma &T, int nsubs, int numz0);
 bool fftlen_supported(int n);
@@ -769,6 +773,8 @@ struct KernelClass {
     double ms = 0.0, bytes = 0.0, flops = 0.0;
 };
 
+constexpr int kHarmRing = 5;  // the default harmonic sum
+
 struct PendingTiming {
     int cls;
     cudaEvent_t start, stop;
@@ -781,10 +787,11 @@ struct jerk_plan {
     jerk_obs obs{};
     int nsubs = 0, maxfft = 0, batch = 8;
     size_t prep_smem = 0;
-    // harmonic-sum kernel (jerk_config.harm_mode, resolved): 1 gather,
-    // 2 gather + TMA L2 prefetch, 3 / 4 TMA tiles of harm_tile (8 / 16) rows;
-    // tma holds the tensor maps of modes 2-4
-    int harm_mode = 1;
+    // harmonic-sum kernel (jerk_config.harm_mode, 0 resolved to kHarmRing):
+    // 1 gather, 2 gather + TMA L2 prefetch, 3 / 4 TMA tiles of harm_tile
+    // (8 / 16) rows, kHarmRing the ring of row copies (jerk_harm.cu); tma
+    // holds the tensor maps of modes 2-4
+    int harm_mode = kHarmRing;
     int harm_tile = 16;
     std::unique_ptr<HarmTma> tma;
     // graph mode: a whole pass captured once per (first, count) and replayed;
@@ -1315,6 +1322,8 @@ static int fold_bank(jerk_plan *p, const std::vector<int> &maxnumrs, long long *
     return JERK_OK;
 }
 
+static int plane_stride(int numrs) { return (numrs + kPlaneAlign - 1) / kPlaneAlign * kPlaneAlign; }
+
 extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk_subharm *subs,
                                 int nsubs, const jerk_config *cfg)
 {
@@ -1344,10 +1353,9 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
         delete p;
         return fail(JERK_EINVAL, "jerk_plan_create: harm_mode must be 0 .. 4");
     }
-    // default: plain gathers, measured fastest at the paper configuration
-    // (57.3 us per rstep against 69.6 with L2 prefetch and 93.7 with 16-row
-    // TMA tiles)
-    p->harm_mode = hm == 0 ? 1 : hm;
+    // the ring up to 16 harmonics; at 32 its registers would hold one cell a
+    // thread, and the gathers stay
+    p->harm_mode = hm != 0 ? hm : obs->numharmstages <= 5 ? kHarmRing : 1;
     p->harm_tile = p->harm_mode == 3 ? 8 : 16;
     p->use_graph = cfg && cfg->use_graph;
     const long long want_hits = (cfg && cfg->max_hits > 0) ? cfg->max_hits : (1LL << 22);
@@ -1403,7 +1411,7 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
     {
         long long per_rstep = 0;
         for (int s = 0; s < nsubs; s++)
-            per_rstep += (long long)subs[s].numw * subs[s].numz * ((maxnumrs[s] + 3) & ~3);
+            per_rstep += (long long)subs[s].numw * subs[s].numz * plane_stride(maxnumrs[s]);
         const long long cap = per_rstep > 0 ? ((1LL << 32) - 1) / per_rstep : p->batch;
         if (cap < 1)
             return bail(fail(JERK_EUNSUPPORTED, "ffdot volumes of one rstep exceed 2^32 floats"));
@@ -1432,7 +1440,7 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
         d.numw = sh.numw;
         d.fftlen = sh.fftlen;
         d.halfwidth = sh.halfwidth;
-        d.stride = (maxnumrs[s] + 3) & ~3;
+        d.stride = plane_stride(maxnumrs[s]);
         d.zlo = calc_required_z(d.harm_fract, obs->zlo);
         d.wlo = calc_required_w(d.harm_fract, obs->wlo);
         d.pownorm = (float)(1.0 / (double)(sh.fftlen * sh.fftlen));
@@ -1577,7 +1585,7 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
     JERK_CUDA_B(cudaMalloc(&p->d_planes, sizeof(float) * p->plane_floats));
     JERK_CUDA_B(cudaMalloc(&p->d_rinds, sizeof(uint16_t) * (size_t)p->batch * nsubs *
                                             obs->corr_uselen));
-    if (p->harm_mode >= 2) {
+    if (p->harm_mode >= 2 && p->harm_mode <= 4) {
         const int rc = build_harm_tma(p, p->harm_mode >= 3);
         if (rc != JERK_OK)
             return bail(rc);
@@ -1585,7 +1593,9 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
             p->harm_mode = 1;  // no tensor maps here: the plain gather kernel
     }
     JERK_CUDA_B(prep_attrs(p->maxfft));
-    JERK_CUDA_B(harmsum_attrs(obs->numharmstages, p->harm_mode));
+    JERK_CUDA_B(harmsum_attrs(obs->numharmstages, p->harm_mode == kHarmRing ? 1 : p->harm_mode));
+    if (p->harm_mode == kHarmRing)
+        JERK_CUDA_B(harm_ring_attrs(obs->numharmstages));
     for (auto &kv : p->groups)
         JERK_CUDA_B(corr_attrs(kv.first));
     for (const FoldRows &R : p->rowsets)
@@ -1817,10 +1827,20 @@ static long long pass_done_batches(jerk_plan *p)
     return ps.ndone;
 }
 
+// Whether a batch takes the ring of row copies: the default form, on volumes
+// large enough for it.
+static bool use_ring(const jerk_plan *p, const SearchDev &a)
+{
+    return p->harm_mode == kHarmRing &&
+           harm_ring_wins(4.0 * (double)p->plane_floats / p->batch * a.nb);
+}
+
 // The plan's own harmonic-sum launch for batch arguments a.
 static cudaError_t launch_harmsum_of(const jerk_plan *p, const SearchDev &a, cudaStream_t st)
 {
     static const HarmTma no_maps{};
+    if (p->harm_mode == kHarmRing)
+        return use_ring(p, a) ? launch_harm_ring(a, st) : launch_harmsum(a, no_maps, false, st);
     return p->harm_mode >= 3 ? launch_harmsum_tma(a, *p->tma, p->harm_tile, st)
            : p->harm_mode == 2 ? launch_harmsum(a, *p->tma, true, st)
                                : launch_harmsum(a, no_maps, false, st);
@@ -2177,15 +2197,20 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
             return fail_all(e, "corr_multi_kernel");
     }
 
-    // harmonic sums: the gather form merged per stage count; plans tuned to
-    // another form launch their own
-    std::map<int, std::vector<int>> byS;
+    // harmonic sums: the ring and the gather form merged per stage count;
+    // plans that fill the GPU twice over, or are tuned to another form, launch
+    // their own
+    std::map<std::pair<int, bool>, std::vector<int>> byS;  // (stages, ring)
     for (int i = 0; i < n; i++) {
         jerk_plan *p = W[i];
         const SearchDev &a = p->pass.a;
+        // (the ring splits its rows evenly over the resident CTAs, alone or
+        // merged; the gather form merges what does not fill two waves)
+        const bool ring = use_ring(p, a);
         const long long ctas = (long long)((a.corr_uselen + 127) / 128) * a.numw0 * a.nb;
-        if (p->harm_mode <= 1 && ctas < 2 * harmsum_wave_ctas(a.nstages)) {
-            byS[p->obs.numharmstages].push_back(i);
+        if (ring || ((p->harm_mode <= 1 || p->harm_mode == kHarmRing) &&
+                     ctas < 2 * harmsum_wave_ctas(a.nstages))) {
+            byS[{p->obs.numharmstages, ring}].push_back(i);
             continue;
         }
         double bytes = 0, flops = 0;
@@ -2206,7 +2231,8 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
             harmsum_work(p, p->pass.a, &bytes, &flops);
         }
         tok = launch_begin(p0, kclass(p0, "wave_harmsum"), bytes, flops);
-        e = launch_harmsum_group(H, kv.first, st);
+        e = kv.first.second ? launch_harm_ring_group(H, kv.first.first, st)
+                            : launch_harmsum_group(H, kv.first.first, st);
         launch_end(p0, tok);
         if (e != cudaSuccess)
             return fail_all(e, "harmsum_group_kernel");
