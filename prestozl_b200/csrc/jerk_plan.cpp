@@ -189,10 +189,9 @@ static int fftlen_from_kernwidth(int kw)
 // summed until a term drops below 1e-15.
 static double log_upper_gamma_large_z(double a, double z)
 {
-    double sum = 1.0, coef = 1.0, term = 1.0;
+    double sum = 1.0, term = 1.0;
     for (int k = 1; fabs(term) > 1e-15; k++) {
-        coef *= (a - k);
-        term = coef / pow(z, k);
+        term *= (a - k) / z;
         sum += term;
     }
     return (a - 1.0) * log(z) - z + log(sum);
@@ -233,23 +232,25 @@ static double chi2_logp(double chi2, double dof)
     return log(q_gamma_int((int)(0.5 * dof + 0.5), 0.5 * chi2));
 }
 
-// x with 1 - Phi(x) = q, full double precision
-static double upper_normal_quantile(double q)
+// The rational approximation of the upper normal quantile, Abramowitz &
+// Stegun 26.2.23, on log p for p <= 1/2 (|error| < 4.5e-4)
+static double normal_quantile_rational(double logp)
 {
-    double lo = -40.0, hi = 40.0, x = 0.0;
-    for (int it = 0; it < 200; it++) {
-        x = 0.5 * (lo + hi);
-        if (0.5 * erfc(x / M_SQRT2) > q)
-            lo = x;
-        else
-            hi = x;
-        if (hi - lo < 1e-15 * (fabs(x) + 1.0))
-            break;
-    }
-    for (int it = 0; it < 3; it++) {
+    const double t = sqrt(-2.0 * logp);
+    const double num = 2.515517 + t * (0.802853 + t * 0.010328);
+    const double den = 1.0 + t * (1.432788 + t * (0.189269 + t * 0.001308));
+    return t - num / den;
+}
+
+// x with 1 - Phi(x) = q for 0 < q < 1/2, full double precision: Newton steps
+// from the rational approximation (three square its error, up to x = 35, away
+// below the last bit; the fourth settles rounding).  A search has thousands
+// of hits, and a bisection with 55 erfc calls each took 2 us a hit.
+static double upper_normal_quantile(double logq, double q)
+{
+    double x = normal_quantile_rational(logq);
+    for (int it = 0; it < 4; it++) {
         const double dens = exp(-0.5 * x * x) / sqrt(2.0 * M_PI);
-        if (dens <= 0.0)
-            break;
         x += (0.5 * erfc(x / M_SQRT2) - q) / dens;
     }
     return x;
@@ -257,24 +258,16 @@ static double upper_normal_quantile(double q)
 
 static double equivalent_gaussian_sigma(double logp)
 {
-    double x;
-    if (logp < -600.0) {
-        // the rational approximation of the normal quantile, Abramowitz &
-        // Stegun 26.2.23, on log p (|error| < 4.5e-4)
-        const double t = sqrt(-2.0 * logp);
-        const double num = 2.515517 + t * (0.802853 + t * 0.010328);
-        const double den = 1.0 + t * (1.432788 + t * (0.189269 + t * 0.001308));
-        x = t - num / den;
-    } else {
-        const double q = exp(logp);
-        /* p = 1 - q < 0 has no normal quantile: the reference's cdfnor2 gives
-           NaN there, and -inf (clamped to 0) at q == 1 */
-        if (q > 1.0)
-            return NAN;
-        if (q == 1.0)
-            return 0.0;
-        x = upper_normal_quantile(q);
-    }
+    if (logp < -600.0)
+        return std::max(0.0, normal_quantile_rational(logp));
+    const double q = exp(logp);
+    /* p = 1 - q < 0 has no normal quantile: the reference's cdfnor2 gives
+       NaN there; at q >= 1/2 the quantile is not positive, which is 0 */
+    if (q > 1.0)
+        return NAN;
+    if (!(q < 0.5))
+        return 0.0;
+    const double x = upper_normal_quantile(logp, q);
     return x < 0.0 ? 0.0 : x;
 }
 
@@ -2340,14 +2333,39 @@ struct HitGeom {
 // r; src/accel_utils_cu.c:857-929) -- decoded into candidates with their
 // sigma and inserted with the reference's rule.  order receives the sorted
 // permutation of the input.
+// order[i]: the index of the i-th key in ascending order.  Keys are distinct;
+// many are sorted by 11-bit digits of the bits they use.
+static void sort_keys(const unsigned long long *keys, uint32_t n, std::vector<uint32_t> &order)
+{
+    order.resize(n);
+    for (uint32_t i = 0; i < n; i++)
+        order[i] = i;
+    if (n < 4096) {
+        std::sort(order.begin(), order.end(),
+                  [&](uint32_t x, uint32_t y) { return keys[x] < keys[y]; });
+        return;
+    }
+    unsigned long long used = 0;
+    for (uint32_t i = 0; i < n; i++)
+        used |= keys[i];
+    constexpr int kBits = 11, kBins = 1 << kBits;
+    std::vector<uint32_t> other(n), start(kBins + 1);
+    for (int shift = 0; shift < 64 && used >> shift; shift += kBits) {
+        std::fill(start.begin(), start.end(), 0u);
+        for (uint32_t i = 0; i < n; i++)
+            start[(keys[i] >> shift & (kBins - 1)) + 1]++;
+        for (int d = 0; d < kBins; d++)
+            start[d + 1] += start[d];
+        for (uint32_t i = 0; i < n; i++)
+            other[start[keys[order[i]] >> shift & (kBins - 1)]++] = order[i];
+        order.swap(other);
+    }
+}
+
 static void hits_to_list(const HitGeom &g, const unsigned long long *keys, const float *pows,
                          uint32_t nh, std::vector<uint32_t> &order, CandList &L)
 {
-    order.resize(nh);
-    for (uint32_t i = 0; i < nh; i++)
-        order[i] = i;
-    std::sort(order.begin(), order.end(),
-              [&](uint32_t x, uint32_t y) { return keys[x] < keys[y]; });
+    sort_keys(keys, nh, order);
     // decode + sigma per hit (independent, so spread over host threads when
     // there are many), then the insertions in key order (sequential: each
     // depends on the list the earlier ones left)
@@ -2373,8 +2391,9 @@ static void hits_to_list(const HitGeom &g, const unsigned long long *keys, const
             c.w = (g.wlo0 + ii * (double)kDW) / (double)nhm;
         }
     };
-    const uint32_t nthr =
-        nh < 8192 ? 1u : std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    // about 0.4 us a hit, some 20 us to start a thread
+    const uint32_t nthr = std::max(
+        1u, std::min({16u, std::thread::hardware_concurrency(), nh / 1024u}));
     if (nthr == 1) {
         decode(0, nh);
     } else {
