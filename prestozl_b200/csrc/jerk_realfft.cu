@@ -11,7 +11,9 @@
 //   1. columns: for each m2 < R2, the R1-point FFT over m1 of z[m2 + R2 m1],
 //      times exp(-2 pi i m2 k1 / M), stored as row k1 of an R1 x R2 scratch;
 //   2. rows: for each k1 < R1, the R2-point FFT of that row, stored to
-//      Z[k1 + R1 k2] in the output;
+//      Z[k1 + R1 k2] in the output (a CTA of either takes up to four
+//      neighbouring columns or rows, so that the strided side moves whole
+//      32-byte sectors);
 //   3. in place on the output: X[k] = (Z[k] + conj Z[M-k]) / 2
 //      - (i/2) exp(-2 pi i k / n) (Z[k] - conj Z[M-k]), one thread per
 //      pair (k, M-k) in double, and X[0] = (DC, Nyquist) packed as the
@@ -28,7 +30,7 @@
 // as runs of blocks of equal length (about 130 runs cover 2^31 bins), passed
 // to the kernels by value.  One warp per block takes the median power (the
 // value of rank (n-1)/2, which the reference's quickselect returns) over
-// ln 2 (a bitonic sort in registers); one warp per segment between block
+// ln 2 (a selection by ballots); one warp per segment between block
 // midpoints then scales its bins by
 // invsqrtf of the linearly interpolated level, in the reference's float and
 // double steps.
@@ -56,87 +58,106 @@ constexpr int kRfSizes[] = {128, 192, 256, 384, 512, 768, 1024, 1280, 2048,
 // ---------------------------------------------------------------------------
 // real FFT kernels
 
-// Entry i of the per-stage twiddle tables of FftPlan<N> (the layout
-// fft_stage_twiddles writes on the host), computed in double.
-template <int N, int S>
-__device__ __forceinline__ void stage_twiddle(int i, float2 *tw)
+// The radices of one FFT plan, and where its tables go.
+struct RfTable {
+    int n, size;
+    int r[8];
+    float2 *tw;
+};
+
+// The per-stage twiddle tables of both block FFTs in one launch (the layout
+// fft_stage_twiddles writes on the host: stage s >= 1 of radix R after ns
+// points holds W_{ns R}^(r k) at [r ns + k]), computed in double.
+__global__ void rf_twiddle_kernel(RfTable A, RfTable B)
 {
-    using P = FftPlan<N>;
-    if constexpr (S < P::nstages) {
-        constexpr int R = P::radices[S];
-        constexpr int OFF = P::twoff(S);
-        constexpr int NS = (P::twoff(S + 1) - OFF) / R;
-        if (i < OFF + NS * R) {
-            const int r = (i - OFF) / NS, k = (i - OFF) % NS;
-            double s, c;
-            sincospi(-2.0 * (double)(r * k) / (double)(NS * R), &s, &c);
-            tw[i] = make_float2((float)c, (float)s);
-        } else {
-            stage_twiddle<N, S + 1>(i, tw);
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const RfTable &t = i < A.size ? A : B;
+    if (i >= A.size)
+        i -= A.size;
+    if (i >= t.size)
+        return;
+    int off = 0, ns = t.r[0];
+    for (int s = 1; s < t.n; s++) {
+        const int size = ns * t.r[s];
+        if (i < off + size) {
+            const int r = (i - off) / ns, k = (i - off) % ns;
+            double sn, cs;
+            sincospi(-2.0 * (double)(r * k) / (double)size, &sn, &cs);
+            t.tw[i] = make_float2((float)cs, (float)sn);
+            return;
         }
+        off += size;
+        ns *= t.r[s];
     }
 }
 
-template <int N>
-__global__ void rf_twiddle_kernel(float2 *tw)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < FftPlan<N>::twsize())
-        stage_twiddle<N, 1>(i, tw);
-}
+// Columns (rows) of a CTA: four where their threads fit in one CTA, whose
+// 8-byte accesses then make whole sectors on the strided side.  The buffers
+// lie 4 banks of 8 bytes apart, so that a half warp (four columns of four
+// neighbouring threads) touches every bank once.  At 2^25 samples one column
+// per CTA took 230 us and one row 161 (a quarter of each sector used).
+template <int R>
+struct RfShape {
+    static constexpr int T = FftPlan<R>::T;
+    static constexpr int C = T <= 256 ? 4 : T <= 512 ? 2 : 1;
+    static constexpr int Pitch = (fft_buf_len<R>() + 15) / 16 * 16 + 4;  // float2
+    static constexpr int Smem = C * Pitch * 8;
+};
 
-// Step 1: CTA m2 transforms column m2 of z (stride R2) and stores row k1 of
+// Step 1: a CTA transforms columns m2 of z (stride R2) and stores row k1 of
 // the scratch at a[k1 * R2 + m2], times exp(-2 pi i m2 k1 / M).  The twiddle
-// is the double product of two per-CTA tables, exp(-2 pi i m2 lo / M) and
+// is the double product of two per-column tables, exp(-2 pi i m2 lo / M) and
 // exp(-2 pi i m2 64 hi / M) for k1 = 64 hi + lo (exponents reduced mod M
 // exactly), rounded once to float.
 constexpr int kTwLo = 64;
 template <int R1>
-__global__ void __launch_bounds__(FftPlan<R1>::T)
+__global__ void __launch_bounds__(RfShape<R1>::T * RfShape<R1>::C)
     rf_column_kernel(const float2 *__restrict__ z, int R2, const float2 *__restrict__ tw,
                      float2 *__restrict__ a)
 {
-    constexpr int T = FftPlan<R1>::T;
+    using H = RfShape<R1>;
+    constexpr int T = H::T, C = H::C;
     constexpr int NHI = (R1 + kTwLo - 1) / kTwLo;
     extern __shared__ float2 rf_buf[];
-    __shared__ double2 t_lo[kTwLo], t_hi[NHI];
-    const int tid = threadIdx.x;
-    const int m2 = blockIdx.x;
+    __shared__ double2 t_lo[kTwLo][C], t_hi[NHI][C];
+    const int c = threadIdx.x % C, tid = threadIdx.x / C;
+    const int m2 = blockIdx.x * C + c;
     const long long M = (long long)R1 * R2;
     for (int i = tid; i < kTwLo + NHI; i += T) {
         const long long e = i < kTwLo ? ((long long)m2 * i) % M
                                       : ((long long)m2 * kTwLo * (i - kTwLo)) % M;
-        double s, c;
-        sincospi(-2.0 * (double)e / (double)M, &s, &c);
+        double sn, cs;
+        sincospi(-2.0 * (double)e / (double)M, &sn, &cs);
         if (i < kTwLo)
-            t_lo[i] = make_double2(c, s);
+            t_lo[i][c] = make_double2(cs, sn);
         else
-            t_hi[i - kTwLo] = make_double2(c, s);
+            t_hi[i - kTwLo][c] = make_double2(cs, sn);
     }
     // fft_block's first barrier orders these writes before the reads in out()
     auto in = [&](int r) -> float2 { return z[m2 + (size_t)R2 * (size_t)(tid + r * T)]; };
     auto out = [&](int k1, float2 y) {
-        const double2 u = t_hi[k1 / kTwLo], v = t_lo[k1 % kTwLo];
+        const double2 u = t_hi[k1 / kTwLo][c], v = t_lo[k1 % kTwLo][c];
         const float2 w = make_float2((float)(u.x * v.x - u.y * v.y), (float)(u.x * v.y + u.y * v.x));
         a[(size_t)k1 * R2 + m2] = cmul(y, w);
     };
-    fft_block<R1, -1>(rf_buf, tw, tid, in, out);
+    fft_block<R1, -1>(rf_buf + c * H::Pitch, tw, tid, in, out);
 }
 
-// Step 2: CTA k1 transforms row k1 of the scratch and stores Z[k1 + R1 k2].
+// Step 2: a CTA transforms rows k1 of the scratch and stores Z[k1 + R1 k2].
 template <int R2>
-__global__ void __launch_bounds__(FftPlan<R2>::T)
+__global__ void __launch_bounds__(RfShape<R2>::T * RfShape<R2>::C)
     rf_row_kernel(const float2 *__restrict__ a, int R1, const float2 *__restrict__ tw,
                   float2 *__restrict__ zout)
 {
-    constexpr int T = FftPlan<R2>::T;
+    using H = RfShape<R2>;
+    constexpr int T = H::T, C = H::C;
     extern __shared__ float2 rf_buf[];
-    const int tid = threadIdx.x;
-    const int k1 = blockIdx.x;
+    const int c = threadIdx.x % C, tid = threadIdx.x / C;
+    const int k1 = blockIdx.x * C + c;
     const float2 *row = a + (size_t)k1 * R2;
     auto in = [&](int r) -> float2 { return row[tid + r * T]; };
     auto out = [&](int k2, float2 y) { zout[k1 + (size_t)R1 * k2] = y; };
-    fft_block<R2, -1>(rf_buf, tw, tid, in, out);
+    fft_block<R2, -1>(rf_buf + c * H::Pitch, tw, tid, in, out);
 }
 
 // Step 3, in place: thread k (0 <= k <= M/2) turns Z[k], Z[M-k] into X[k],
@@ -168,35 +189,27 @@ __global__ void rf_post_kernel(float2 *x, long long M)
     }
 }
 
-template <int R>
-cudaError_t rf_launch_twiddles(float2 *tw, cudaStream_t st)
-{
-    constexpr int n = FftPlan<R>::twsize();
-    rf_twiddle_kernel<R><<<(n + 255) / 256, 256, 0, st>>>(tw);
-    return cudaGetLastError();
-}
-
 template <int R1>
 cudaError_t rf_launch_columns(const float2 *z, int R2, const float2 *tw, float2 *a, cudaStream_t st)
 {
-    const int smem = (int)(sizeof(float2) * fft_buf_len<R1>());
+    using H = RfShape<R1>;
     cudaError_t e = cudaFuncSetAttribute(rf_column_kernel<R1>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, H::Smem);
     if (e != cudaSuccess)
         return e;
-    rf_column_kernel<R1><<<R2, FftPlan<R1>::T, smem, st>>>(z, R2, tw, a);
+    rf_column_kernel<R1><<<R2 / H::C, H::T * H::C, H::Smem, st>>>(z, R2, tw, a);
     return cudaGetLastError();
 }
 
 template <int R2>
 cudaError_t rf_launch_rows(const float2 *a, int R1, const float2 *tw, float2 *zout, cudaStream_t st)
 {
-    const int smem = (int)(sizeof(float2) * fft_buf_len<R2>());
+    using H = RfShape<R2>;
     cudaError_t e = cudaFuncSetAttribute(rf_row_kernel<R2>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, H::Smem);
     if (e != cudaSuccess)
         return e;
-    rf_row_kernel<R2><<<R1, FftPlan<R2>::T, smem, st>>>(a, R1, tw, zout);
+    rf_row_kernel<R2><<<R1 / H::C, H::T * H::C, H::Smem, st>>>(a, R1, tw, zout);
     return cudaGetLastError();
 }
 
@@ -222,8 +235,17 @@ cudaError_t rf_dispatch(int R, A... args)
     default: return cudaErrorInvalidValue;
     }
 }
-template <int R> struct RfTw {
-    static cudaError_t run(float2 *tw, cudaStream_t st) { return rf_launch_twiddles<R>(tw, st); }
+template <int R> struct RfRadices {
+    static cudaError_t run(RfTable *t)
+    {
+        using P = FftPlan<R>;
+        static_assert(P::nstages <= 8, "radices");
+        t->n = P::nstages;
+        t->size = P::twsize();
+        for (int i = 0; i < P::nstages; i++)
+            t->r[i] = P::radices[i];
+        return cudaSuccess;
+    }
 };
 template <int R> struct RfCol {
     static cudaError_t run(const float2 *z, int R2, const float2 *tw, float2 *a, cudaStream_t st)
@@ -295,7 +317,8 @@ struct DrRuns {
 };
 static_assert(sizeof(DrRuns) <= 4000, "kernel parameter space");
 
-__device__ __forceinline__ int2 dr_block(const DrRuns &R, int b)
+// the run that holds block b
+__device__ __forceinline__ int dr_run(const DrRuns &R, int b)
 {
     int lo = 0, hi = R.n - 1;
     while (lo < hi) {
@@ -305,8 +328,7 @@ __device__ __forceinline__ int2 dr_block(const DrRuns &R, int b)
         else
             hi = mid - 1;
     }
-    const DrRun &u = R.r[lo];
-    return make_int2(u.start + (b - u.first) * u.len, u.len);
+    return lo;
 }
 
 __device__ __forceinline__ float dr_power(float2 v)
@@ -316,67 +338,110 @@ __device__ __forceinline__ float dr_power(float2 v)
 
 constexpr int kDrWarps = 8;
 
-// Ascending bitonic sort of 128 values held 4 per lane (value e = lane + 32 j
-// in v[j]) across one warp.
-__device__ __forceinline__ void warp_sort128(float (&v)[4], int lane)
+// The k-th smallest (0-based) of the first n <= 128 values held 4 per lane
+// (value e = lane + 32 j as bit pattern u[j], ~0 past n; non-negative floats
+// order as their bits do), by one warp: thresholds -- first where the median
+// of exponential noise of this mean would lie, then steps by that density --
+// until the count below one is k or k + 1, whose neighbour is the value; ties
+// and other distributions end in a walk over the values from the lower bound.
+// The thresholds only set the speed.  (For 2^24 bins: 71 us; sorting in
+// registers, a hundred shuffles a block, 110; a quickselect by ballots 119.)
+__device__ __forceinline__ int warp_count_below(const unsigned (&u)[4], unsigned t)
 {
-#pragma unroll
-    for (int s = 2; s <= 128; s <<= 1) {
-#pragma unroll
-        for (int d = s >> 1; d > 0; d >>= 1) {
-            if (d >= 32) {
-                const int dj = d >> 5;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    if ((j & dj) == 0) {
-                        const bool asc = ((lane + 32 * j) & s) == 0;
-                        const float a = v[j], b = v[j | dj];
-                        v[j] = asc ? fminf(a, b) : fmaxf(a, b);
-                        v[j | dj] = asc ? fmaxf(a, b) : fminf(a, b);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int e = lane + 32 * j;
-                    const float o = __shfl_xor_sync(0xffffffffu, v[j], d);
-                    const bool keep_min = (((e & s) == 0) == ((e & d) == 0));
-                    v[j] = keep_min ? fminf(v[j], o) : fmaxf(v[j], o);
-                }
-            }
+    const unsigned c = (u[0] < t) + (u[1] < t) + (u[2] < t) + (u[3] < t);
+    return (int)__reduce_add_sync(0xffffffffu, c);
+}
+
+__device__ __forceinline__ unsigned warp_select(const unsigned (&u)[4], float mean, int n, int k)
+{
+    // counts below flo and fhi: cl <= k < ch
+    float flo = 0.f, fhi = __int_as_float(0x7f800000);
+    int cl = 0, ch = n;
+    float p = 0.69314718f * mean;
+    const float step = 2.0f * mean / (float)n;  // one rank at the median
+#pragma unroll 1
+    for (int round = 0; round < 7 && cl < k && ch > k + 1; round++) {
+        const int c = warp_count_below(u, __float_as_uint(p));
+        if (c <= k) {
+            flo = p;
+            cl = c;
+        } else {
+            fhi = p;
+            ch = c;
         }
+        // the next threshold aims half a rank past the one wanted
+        const float d = ((float)(k - c) + 0.5f) * step;
+        const float q = p + d;
+        p = q > flo && q < fhi ? q : 0.5f * (flo + fhi);
+    }
+    if (ch == k + 1) {  // the largest value below fhi
+        unsigned m = 0u;
+        const unsigned t = __float_as_uint(fhi);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            m = max(m, u[j] < t ? u[j] : 0u);
+        return __reduce_max_sync(0xffffffffu, m);
+    }
+    unsigned lo = __float_as_uint(flo);
+    for (;;) {  // the smallest value from lo on, until its rank passes k
+        unsigned m = ~0u;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            m = min(m, u[j] >= lo ? u[j] : ~0u);
+        m = __reduce_min_sync(0xffffffffu, m);
+        if (cl == k || m == ~0u || warp_count_below(u, m + 1u) > k)
+            return m;
+        lo = m + 1u;
+        cl = -1;
     }
 }
 
-// One warp per block: level[b] = median power / ln 2.  Blocks are at most 128
-// bins long below 2^31 bins ((int)(6 ln 2^31) = 128): sorted in registers,
-// padded with +inf; the value at sorted position (n-1)/2 is the one the
-// reference's quickselect returns.  (Longer blocks, which the walk never
-// makes, would take the stable-rank count.)
+// One warp per block: level[b] = median power / ln 2, its middle bin and
+// its length.  Blocks are at most 128 bins long below 2^31 bins ((int)(6 ln
+// 2^31) = 128); the value of rank (n-1)/2 is the one the reference's
+// quickselect returns.  (Longer blocks, which the walk never makes, would take
+// the stable-rank count.)
 __global__ void __launch_bounds__(32 * kDrWarps)
     dr_level_kernel(const float2 *__restrict__ x, const __grid_constant__ DrRuns runs, int nb,
-                    double ln2, float *__restrict__ level)
+                    double ln2, float *__restrict__ level, int *__restrict__ mid, int *__restrict__ len)
 {
     __shared__ float pw[kDrWarps][kDrMax];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.x * kDrWarps + w;
+    // the run of the CTA's first block, once; the others step on from it
+    __shared__ int s_run;
+    if (threadIdx.x == 0)
+        s_run = dr_run(runs, blockIdx.x * kDrWarps);
+    __syncthreads();
     if (b >= nb)
         return;  // whole warps leave; only warp-level syncs below
-    const int2 blk = dr_block(runs, b);
+    int run = s_run;
+    while (run + 1 < runs.n && runs.r[run + 1].first <= b)
+        run++;
+    const int2 blk = make_int2(runs.r[run].start + (b - runs.r[run].first) * runs.r[run].len,
+                               runs.r[run].len);
     const int n = blk.y;
     const int k = (n - 1) / 2;
+    if (lane == 0) {
+        mid[b] = blk.x + n / 2;
+        len[b] = n;
+    }
     if (n <= 128) {
-        float v[4];
+        unsigned u[4];
+        float sum = 0.f;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int i = lane + 32 * j;
-            v[j] = i < n ? dr_power(x[blk.x + i]) : INFINITY;
+            const float p = i < n ? dr_power(x[blk.x + i]) : 0.f;
+            u[j] = i < n ? __float_as_uint(p) : ~0u;
+            sum += p;
         }
-        warp_sort128(v, lane);
-        const float m0 = __shfl_sync(0xffffffffu, v[0], k & 31);
-        const float m1 = __shfl_sync(0xffffffffu, v[1], k & 31);
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1)
+            sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        const float med = __uint_as_float(warp_select(u, sum / (float)n, n, k));
         if (lane == 0)
-            level[b] = (float)((double)(k < 32 ? m0 : m1) / ln2);
+            level[b] = (float)((double)med / ln2);
         return;
     }
     float *p = pw[w];
@@ -399,50 +464,47 @@ __global__ void __launch_bounds__(32 * kDrWarps)
 // constant level[0]; segment s is [mid(s-1), mid(s)) (mid(nb) = numamps)
 // running from level[s-1] with the slope toward level[s] (the tail keeps the
 // last slope, or 1 when there is one block).  mid(b) = start + len / 2.
-// Bin 0 becomes (1, bin0_imag).
+// Bin 0 becomes (1, bin0_imag).  A segment is about a hundred bins: its loads
+// go out together, and the blocks' places come from the level pass (the walk
+// over the runs three times a warp, and one load at a time, took 97 us for
+// 2^24 bins).
 __global__ void __launch_bounds__(32 * kDrWarps)
-    dr_scale_kernel(float2 *__restrict__ x, const __grid_constant__ DrRuns runs, int nb,
-                    int numamps, const float *__restrict__ level, float bin0_imag)
+    dr_scale_kernel(float2 *__restrict__ x, int nb, int numamps, const float *__restrict__ level,
+                    const int *__restrict__ mid, const int *__restrict__ len, float bin0_imag)
 {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int s = blockIdx.x * kDrWarps + w;
     if (s > nb)
         return;
-    int lo, hi;
-    float base, slope = 0.0f;
     const bool flat = s == 0;
+    const int lo = flat ? 1 : mid[s - 1];
+    const int hi = s < nb ? mid[s] : numamps;
+    const float base = level[flat ? 0 : s - 1];
+    float slope = 0.0f;
     if (flat) {
-        const int2 b0 = dr_block(runs, 0);
-        lo = 1;
-        hi = b0.x + b0.y / 2;
-        base = level[0];
         if (lane == 0)
             x[0] = make_float2(1.0f, bin0_imag);
     } else {
-        const int2 prev = dr_block(runs, s - 1);
-        lo = prev.x + prev.y / 2;
-        base = level[s - 1];
-        if (s < nb) {
-            const int2 cur = dr_block(runs, s);
-            hi = cur.x + cur.y / 2;
-        } else {
-            hi = numamps;
-        }
         const int bb = s < nb ? s : nb - 1;
-        if (bb >= 1) {
-            const int la = dr_block(runs, bb - 1).y, lb = dr_block(runs, bb).y;
-            slope = (float)((double)__fsub_rn(level[bb], level[bb - 1]) / (0.5 * (double)(la + lb)));
-        } else {
-            slope = 1.0f;
-        }
+        slope = bb >= 1 ? (float)((double)__fsub_rn(level[bb], level[bb - 1]) /
+                                  (0.5 * (double)(len[bb - 1] + len[bb])))
+                        : 1.0f;
     }
-    for (int ind = lo + lane; ind < hi; ind += 32) {
-        const float lv = flat ? base : __fadd_rn(base, __fmul_rn(slope, (float)(ind - lo)));
-        const float nrm = invsqrtf_ref(lv);
-        float2 v = x[ind];
-        v.x = __fmul_rn(v.x, nrm);
-        v.y = __fmul_rn(v.y, nrm);
-        x[ind] = v;
+    for (int i0 = lo + lane; i0 < hi; i0 += 128) {
+        float2 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (i0 + 32 * j < hi)
+                v[j] = x[i0 + 32 * j];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int ind = i0 + 32 * j;
+            if (ind >= hi)
+                break;
+            const float lv = flat ? base : __fadd_rn(base, __fmul_rn(slope, (float)(ind - lo)));
+            const float nrm = invsqrtf_ref(lv);
+            x[ind] = make_float2(__fmul_rn(v[j].x, nrm), __fmul_rn(v[j].y, nrm));
+        }
     }
 }
 
@@ -509,55 +571,63 @@ int dr_layout(int numamps, DrRuns *out)
 
 size_t dr_scratch(int numamps)
 {
-    return align256(sizeof(float) * (size_t)(numamps / kDrInit + 2));
+    return 3 * align256(sizeof(float) * (size_t)(numamps / kDrInit + 2));  // level, mid, len
 }
 
 // ---------------------------------------------------------------------------
 // birdie zapping (zapbirds from memory, src/zapping.c:29-81)
 
 constexpr int kZapBins = 200;  // MEDIANBINS (src/zapping.c:3)
-constexpr int kZapThreads = 256;
+constexpr int kZapThreads = 512;
+constexpr int kZapGroup = 128;
 
-// One birdie.  The median powers (rank 99 of 200) of the bins
+struct ZapGroup {
+    double lo[kZapGroup], hi[kZapGroup];
+};
+
+// One birdie per CTA.  The median powers (rank 99 of 200) of the bins
 // [lobin - 300, lobin - 100) and [hibin - 100, hibin + 100), read before any
 // bin is written (bins at or past numamps read as zeros, as the reference's
 // zero-padded buffer gives them), set avgamp = sqrt(0.5 (mlo + mhi) / ln 2);
-// bins [floor(lobin), ceil(hibin)) become (avgamp, 0).
+// bins [floor(lobin), ceil(hibin)) become (avgamp, 0).  The birdies of a
+// launch touch no bin that another writes (one launch per birdie, as the
+// order of the list would have it, took 7 us each).
 __global__ void __launch_bounds__(kZapThreads)
-    zap_kernel(float2 *__restrict__ x, long long numamps, double lobin, double hibin,
+    zap_kernel(float2 *__restrict__ x, long long numamps, const __grid_constant__ ZapGroup g,
                double neg_log_half)
 {
-    __shared__ float p[2][kZapBins];
+    __shared__ __align__(16) float p[2][kZapBins];
     __shared__ float med[2];
-    const int tid = threadIdx.x;
-    const long long first[2] = {(long long)(lobin - 3 * kZapBins / 2),
-                                (long long)(hibin - kZapBins / 2)};
-#pragma unroll
-    for (int w = 0; w < 2; w++)
-        for (int i = tid; i < kZapBins; i += kZapThreads) {
-            const long long b = first[w] + i;
-            const float2 v = (b >= 0 && b < numamps) ? x[b] : make_float2(0.f, 0.f);
-            p[w][i] = dr_power(v);
-        }
+    const double lobin = g.lo[blockIdx.x], hibin = g.hi[blockIdx.x];
+    const int w = threadIdx.x / 256, i = threadIdx.x % 256;
+    const long long first = w == 0 ? (long long)(lobin - 3 * kZapBins / 2)
+                                   : (long long)(hibin - kZapBins / 2);
+    float v = 0.f;
+    if (i < kZapBins) {
+        const long long b = first + i;
+        v = dr_power((b >= 0 && b < numamps) ? x[b] : make_float2(0.f, 0.f));
+        p[w][i] = v;
+    }
     __syncthreads();
     constexpr int k = (kZapBins - 1) / 2;
-#pragma unroll
-    for (int w = 0; w < 2; w++)
-        for (int i = tid; i < kZapBins; i += kZapThreads) {
-            const float v = p[w][i];
-            int pos = 0;
-            for (int j = 0; j < kZapBins; j++) {
-                const float u = p[w][j];
-                pos += (u < v) | ((u == v) & (j < i));
-            }
-            if (pos == k)
-                med[w] = v;
+    if (i < kZapBins) {
+        int pos = 0;
+#pragma unroll 5
+        for (int j = 0; j < kZapBins; j += 4) {
+            const float4 u = *reinterpret_cast<const float4 *>(&p[w][j]);
+            pos += (u.x < v) | ((u.x == v) & (j < i));
+            pos += (u.y < v) | ((u.y == v) & (j + 1 < i));
+            pos += (u.z < v) | ((u.z == v) & (j + 2 < i));
+            pos += (u.w < v) | ((u.w == v) & (j + 3 < i));
         }
+        if (pos == k)
+            med[w] = v;
+    }
     __syncthreads();
     const float avgamp =
         (float)__dsqrt_rn(__ddiv_rn(0.5 * (double)__fadd_rn(med[0], med[1]), neg_log_half));
     const long long lo = (long long)floor(lobin), hi = (long long)ceil(hibin);
-    for (long long b = lo + tid; b < hi; b += kZapThreads)
+    for (long long b = lo + threadIdx.x; b < hi; b += kZapThreads)
         if (b >= 0 && b < numamps)
             x[b] = make_float2(avgamp, 0.f);
 }
@@ -596,9 +666,13 @@ extern "C" int jerk_realfft(const float *timeseries, long long n, void *spectrum
     float2 *tw1 = (float2 *)(base + align256(sizeof(float2) * (size_t)R1 * R2));
     float2 *tw2 = (float2 *)((unsigned char *)tw1 + align256(sizeof(float2) * rf_twsize(R1)));
     float2 *out = (float2 *)spectrum;
-    cudaError_t e = rf_dispatch<RfTw>(R1, tw1, st);
-    if (e == cudaSuccess)
-        e = rf_dispatch<RfTw>(R2, tw2, st);
+    RfTable t1{}, t2{};
+    rf_dispatch<RfRadices>(R1, &t1);
+    rf_dispatch<RfRadices>(R2, &t2);
+    t1.tw = tw1;
+    t2.tw = tw2;
+    rf_twiddle_kernel<<<(t1.size + t2.size + 255) / 256, 256, 0, st>>>(t1, t2);
+    cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
         e = rf_dispatch<RfCol>(R1, (const float2 *)timeseries, R2, (const float2 *)tw1, a, st);
     if (e == cudaSuccess)
@@ -640,13 +714,17 @@ int deredden_impl(void *spectrum, long long numamps, void *scratch, long long sc
     if (nb < 1)
         return set_error(JERK_EUNSUPPORTED, "jerk_deredden: block layout too long");
     cudaStream_t st = (cudaStream_t)stream;
+    const size_t part = align256(sizeof(float) * (size_t)(numamps / kDrInit + 2));
     float *level = (float *)scratch;
+    int *mid = (int *)((unsigned char *)scratch + part);
+    int *len = (int *)((unsigned char *)scratch + 2 * part);
     float2 *x = (float2 *)spectrum;
     const int threads = 32 * kDrWarps;
     dr_level_kernel<<<(nb + kDrWarps - 1) / kDrWarps, threads, 0, st>>>(x, runs, nb, std::log(2.0),
-                                                                       level);
+                                                                       level, mid, len);
     dr_scale_kernel<<<(nb + 1 + kDrWarps - 1) / kDrWarps, threads, 0, st>>>(
-        x, runs, nb, (int)numamps, level, bin0_imag);
+        x, nb, (int)numamps, level, mid, len,
+        bin0_imag);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return set_error(JERK_ECUDA, cudaGetErrorString(e));
@@ -692,14 +770,35 @@ extern "C" int jerk_zap_birdies(void *spectrum, long long numbins, long long N,
     cudaStream_t st = (cudaStream_t)stream;
     const double top = (double)(N / 2);
     const double neg_log_half = -std::log(0.5);
+    // birdies in list order; a launch takes as many as touch none of each
+    // other's bins: a birdie reads within [lo - 301, lo - 99) and [hi - 101,
+    // hi + 101) and writes within [lo - 1, hi + 1)
+    ZapGroup g;
+    int n = 0;
+    auto flush = [&] {
+        if (n)
+            zap_kernel<<<n, kZapThreads, 0, st>>>((float2 *)spectrum, numbins, g, neg_log_half);
+        n = 0;
+    };
+    auto clear_of = [](double alo, double ahi, double blo, double bhi) {  // a's bins, b's writes
+        return std::min(alo - 302.0, ahi - 102.0) >= bhi + 1.0 ||
+               std::max(alo - 99.0, ahi + 102.0) <= blo - 1.0;
+    };
     for (int i = 0; i < nbirds; i++) {
         if (lobins[i] >= top)
             break;
         const double lo = lobins[i], hi = hibins[i] >= top ? top - 1 : hibins[i];
         if (!(lo - 1.5 * kZapBins > 1))
             continue;
-        zap_kernel<<<1, kZapThreads, 0, st>>>((float2 *)spectrum, numbins, lo, hi, neg_log_half);
+        bool apart = n < kZapGroup;
+        for (int j = 0; j < n && apart; j++)
+            apart = clear_of(lo, hi, g.lo[j], g.hi[j]) && clear_of(g.lo[j], g.hi[j], lo, hi);
+        if (!apart)
+            flush();
+        g.lo[n] = lo;
+        g.hi[n++] = hi;
     }
+    flush();
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return set_error(JERK_ECUDA, cudaGetErrorString(e));
