@@ -21,11 +21,10 @@
 //                            npts samples, zero-padded to 8 npts, real FFT
 //                            (an M = 4 npts point complex FFT in shared memory
 //                            and the real split of the numkern bins needed)
-//   pk_fft_kernel<N>         forward FFT of every kernel row, in place
-//   pd_data_kernel<N>        each harmonic's data window spread by 8, FFT'd
-//   pc_corr_kernel<N>        per kernel row: times conj(kernel) / fftlen,
-//                            inverse FFT, power at the 24 r positions over
-//                            the local power
+//   pd_data_kernel           each harmonic's data window spread by 8, FFT'd
+//   pc_corr_kernel           per kernel row: its forward FFT, the data times
+//                            its conjugate / fftlen, inverse FFT, power at the
+//                            24 r positions over the local power
 //   ps_argmax_kernel         sum over harmonics in the reference's order,
 //                            first strict maximum
 // The local powers (get_localpower3d, src/characteristics.c:75-135) come in
@@ -44,6 +43,7 @@
 #include <vector>
 
 #include "jerk.h"
+#include "jerk_async.cuh"
 #include "jerk_fft.cuh"
 #include "jerk_kernels.cuh"
 #include "jerk_resp.cuh"
@@ -227,29 +227,22 @@ __global__ void __launch_bounds__(FftPlan<M>::T)
 // ---------------------------------------------------------------------------
 // kernel-row FFTs, data windows, correlations
 
-template <int N>
-__global__ void __launch_bounds__(FftPlan<N>::T)
-    pk_fft_kernel(const PolishRow *__restrict__ rows, int first, const float2 *__restrict__ tw,
-                  float2 *__restrict__ bank)
-{
-    constexpr int T = FftPlan<N>::T;
-    extern __shared__ float2 pk_buf[];
-    float2 *row = bank + rows[first + blockIdx.x].off;
-    const int tid = threadIdx.x;
-    auto in = [&](int r) -> float2 { return row[tid + r * T]; };
-    auto out = [&](int m, float2 y) { row[m] = y; };
-    fft_block<N, -1>(pk_buf, tw, tid, in, out);
-}
+// The harmonics of a candidate have a few FFT lengths; one launch covers them
+// all (CTAs of the widest plan's threads, whose surplus only joins the
+// barriers): a launch per length and step took 89 us of a 16-harmonic
+// candidate, nine launches that each left most of the GPU idle.
+struct PolishTw {
+    const float2 *tw;
+    int off[7];  // kSizes
+};
 
 // spread_no_pad (src/corr_prep.c:37-74) by 8, then the forward FFT
 template <int N>
-__global__ void __launch_bounds__(FftPlan<N>::T)
-    pd_data_kernel(const PolishHarm *__restrict__ harms, int first, const float2 *__restrict__ tw,
-                   const float2 *__restrict__ windows, float2 *__restrict__ dfft)
+__device__ __forceinline__ void pd_data(const PolishHarm &H, const float2 *tw,
+                                        const float2 *__restrict__ windows,
+                                        float2 *__restrict__ dfft, float2 *buf)
 {
     constexpr int T = FftPlan<N>::T;
-    extern __shared__ float2 pd_buf[];
-    const PolishHarm H = harms[first + blockIdx.x];
     const float2 *src = windows + H.win;
     float2 *dst = dfft + H.data;
     const int tid = threadIdx.x;
@@ -258,27 +251,43 @@ __global__ void __launch_bounds__(FftPlan<N>::T)
         return (m % kNb) == 0 ? src[m / kNb] : make_float2(0.f, 0.f);
     };
     auto out = [&](int m, float2 y) { dst[m] = y; };
-    fft_block<N, -1>(pd_buf, tw, tid, in, out);
+    fft_block<N, -1>(buf, tw, tid, in, out);
 }
 
-// complex_corr_conv (src/correlations.c:3-55, CORR) and the chop of
-// corr_complex: amplitude i of the volume is y[khw * 8 + i]
+__global__ void __launch_bounds__(512)
+    pd_data_kernel(const PolishHarm *__restrict__ harms, const PolishTw W,
+                   const float2 *__restrict__ windows, float2 *__restrict__ dfft)
+{
+    extern __shared__ float2 p_smem[];
+    const PolishHarm &H = harms[blockIdx.x];
+    switch (H.fftlen) {
+#define JERK_PD(NN, I) case NN: pd_data<NN>(H, W.tw + W.off[I], windows, dfft, p_smem); break;
+    JERK_PD(128, 0) JERK_PD(256, 1) JERK_PD(512, 2) JERK_PD(1024, 3) JERK_PD(2048, 4)
+    JERK_PD(4096, 5) JERK_PD(8192, 6)
+#undef JERK_PD
+    default: break;
+    }
+}
+
+// The kernel row's forward FFT (kept in shared memory), then complex_corr_conv
+// (src/correlations.c:3-55, CORR) and the chop of corr_complex: amplitude i of
+// the volume is y[khw * 8 + i]
 template <int N>
-__global__ void __launch_bounds__(FftPlan<N>::T)
-    pc_corr_kernel(const PolishRow *__restrict__ rows, int first,
-                   const PolishHarm *__restrict__ harms, const float2 *__restrict__ tw,
-                   const float2 *__restrict__ bank, const float2 *__restrict__ dfft,
-                   float *__restrict__ terms, float *__restrict__ tails)
+__device__ __forceinline__ void pc_corr(const PolishHarm &H, const float2 *__restrict__ kresp,
+                                        long long rowi, const float2 *tw,
+                                        const float2 *__restrict__ dfft, float *__restrict__ terms,
+                                        float *__restrict__ tails, float2 *buf, float *pw)
 {
     constexpr int T = FftPlan<N>::T;
-    extern __shared__ float2 pc_buf[];
-    __shared__ float pw[kWin];
-    const int rowi = first + blockIdx.x;
-    const PolishRow R = rows[rowi];
-    const PolishHarm &H = harms[R.harm];
-    const float2 *krow = bank + R.off;
+    float2 *krow = buf + fft_buf_len<N>();
     const float2 *d = dfft + H.data;
     const int tid = threadIdx.x;
+    {
+        auto in = [&](int r) -> float2 { return kresp[tid + r * T]; };
+        auto out = [&](int m, float2 y) { krow[m] = y; };
+        fft_block<N, -1>(buf, tw, tid, in, out);
+    }
+    __syncthreads();
     const float normal = 1.0f / (float)N;
     auto in = [&](int r) -> float2 {
         const int m = tid + r * T;
@@ -295,30 +304,52 @@ __global__ void __launch_bounds__(FftPlan<N>::T)
             pw[i] = p;
         const int t = m - tail0;
         if (t >= 0 && t < kTail)
-            tails[(long long)rowi * kTail + t] = p;
+            tails[rowi * kTail + t] = p;
     };
-    fft_block<N, +1>(pc_buf, tw, tid, in, out);
+    fft_block<N, +1>(buf, tw, tid, in, out);
     __syncthreads();
     if (tid < kNumR && H.rind[tid] >= 0)
-        terms[(long long)rowi * kNumR + tid] = __fdiv_rn(pw[H.rind[tid] - H.rmin], H.locpow);
+        terms[rowi * kNumR + tid] = __fdiv_rn(pw[H.rind[tid] - H.rmin], H.locpow);
+}
+
+__global__ void __launch_bounds__(512)
+    pc_corr_kernel(const PolishRow *__restrict__ rows, const PolishHarm *__restrict__ harms,
+                   const PolishTw W, const float2 *__restrict__ bank,
+                   const float2 *__restrict__ dfft, float *__restrict__ terms,
+                   float *__restrict__ tails)
+{
+    extern __shared__ float2 p_smem[];
+    __shared__ float pw[kWin];
+    const long long rowi = blockIdx.x;
+    const PolishRow &R = rows[rowi];
+    const PolishHarm &H = harms[R.harm];
+    switch (H.fftlen) {
+#define JERK_PC(NN, I)                                                                       \
+    case NN:                                                                                 \
+        pc_corr<NN>(H, bank + R.off, rowi, W.tw + W.off[I], dfft, terms, tails, p_smem, pw); \
+        break;
+    JERK_PC(128, 0) JERK_PC(256, 1) JERK_PC(512, 2) JERK_PC(1024, 3) JERK_PC(2048, 4)
+    JERK_PC(4096, 5) JERK_PC(8192, 6)
+#undef JERK_PC
+    default: break;
+    }
 }
 
 // powsum[w][z][r] = sum over harmonics (highest first) of the terms; the first
-// strict maximum above 0 in (w, z, r) order.  One CTA.
-constexpr int kArgThreads = 1024;
+// strict maximum above 0 in (w, z, r) order: the largest (power, ~position) in
+// *best, which starts at 0.  (One CTA for all 6936 sums took 66 us.)
+constexpr int kArgThreads = 128;
 __global__ void __launch_bounds__(kArgThreads)
     ps_argmax_kernel(const float *__restrict__ terms, const float *__restrict__ tails,
-                     const PolishHarm *__restrict__ harms, int numharm, int *__restrict__ best,
-                     float *__restrict__ bestpow)
+                     const PolishHarm *__restrict__ harms, int numharm,
+                     unsigned long long *__restrict__ best)
 {
-    __shared__ float sv[kArgThreads / 32];
-    __shared__ int si[kArgThreads / 32];
-    const int tid = threadIdx.x;
-    float bv = 0.0f;
-    int bi = 0x7fffffff;
-    for (int c = tid; c < kCells * kNumR; c += kArgThreads) {
+    const int c = blockIdx.x * kArgThreads + threadIdx.x;
+    unsigned long long key = 0;
+    if (c < kCells * kNumR) {
         const int cell = c / kNumR, kk = c % kNumR;
         float s = 0.0f;
+#pragma unroll 4
         for (int h = 0; h < numharm; h++) {
             const int ri = harms[h].rind[kk];
             const long long row = (long long)h * kCells + cell;
@@ -331,40 +362,13 @@ __global__ void __launch_bounds__(kArgThreads)
                 t = 0.0f;
             s = __fadd_rn(s, t);
         }
-        if (s > bv) {  // cells visited in increasing order per thread
-            bv = s;
-            bi = c;
-        }
+        if (s > 0.0f)
+            key = (unsigned long long)__float_as_uint(s) << 32 | (0xffffffffu - (unsigned)c);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_down_sync(0xffffffffu, bv, o);
-        const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-        if (ov > bv || (ov == bv && oi < bi)) {
-            bv = ov;
-            bi = oi;
-        }
-    }
-    if ((tid & 31) == 0) {
-        sv[tid >> 5] = bv;
-        si[tid >> 5] = bi;
-    }
-    __syncthreads();
-    if (tid < 32) {
-        bv = sv[tid];
-        bi = si[tid];
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_down_sync(0xffffffffu, bv, o);
-            const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-            if (ov > bv || (ov == bv && oi < bi)) {
-                bv = ov;
-                bi = oi;
-            }
-        }
-        if (tid == 0) {
-            *best = bi == 0x7fffffff ? 0 : bi;
-            *bestpow = bv;
-        }
-    }
+    for (int o = 16; o > 0; o >>= 1)
+        key = max(key, __shfl_down_sync(0xffffffffu, key, o));
+    if ((threadIdx.x & 31) == 0 && key)
+        atomicMax(best, key);
 }
 
 // per-stage twiddles of every power-of-two plan 128..8192, in double
@@ -457,48 +461,6 @@ template <int M> struct PW {
         return cudaGetLastError();
     }
 };
-template <int N> struct PK {
-    static cudaError_t run(const PolishRow *rows, int first, int count, const float2 *tw,
-                           float2 *bank, cudaStream_t st)
-    {
-        const int smem = (int)(sizeof(float2) * fft_buf_len<N>());
-        cudaError_t e = cudaFuncSetAttribute(pk_fft_kernel<N>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-        pk_fft_kernel<N><<<count, FftPlan<N>::T, smem, st>>>(rows, first, tw, bank);
-        return cudaGetLastError();
-    }
-};
-template <int N> struct PD {
-    static cudaError_t run(const PolishHarm *harms, int first, int count, const float2 *tw,
-                           const float2 *windows, float2 *dfft, cudaStream_t st)
-    {
-        const int smem = (int)(sizeof(float2) * fft_buf_len<N>());
-        cudaError_t e = cudaFuncSetAttribute(pd_data_kernel<N>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-        pd_data_kernel<N><<<count, FftPlan<N>::T, smem, st>>>(harms, first, tw, windows, dfft);
-        return cudaGetLastError();
-    }
-};
-template <int N> struct PC {
-    static cudaError_t run(const PolishRow *rows, int first, int count, const PolishHarm *harms,
-                           const float2 *tw, const float2 *bank, const float2 *dfft,
-                           float *terms, float *tails, cudaStream_t st)
-    {
-        const int smem = (int)(sizeof(float2) * fft_buf_len<N>());
-        cudaError_t e = cudaFuncSetAttribute(pc_corr_kernel<N>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-        pc_corr_kernel<N><<<count, FftPlan<N>::T, smem, st>>>(rows, first, harms, tw, bank, dfft,
-                                                              terms, tails);
-        return cudaGetLastError();
-    }
-};
-
 long long next2(long long x)
 {
     long long n = 1;
@@ -506,6 +468,17 @@ long long next2(long long x)
         n <<= 1;
     return n;
 }
+
+struct InterpPoint {
+    long long win;  // float2 offset of the staged data window (numkern bins)
+    double frac, z, w;
+    int numkern;    // 2 kern_half_width
+    int npts;       // w responses: the cosine series' length (M = npts / 2)
+};
+
+__global__ void interp_w_kernel(const InterpPoint *__restrict__ pts, const int *__restrict__ list,
+                                const PolishTw W, const float2 *__restrict__ windows,
+                                float2 *__restrict__ ans);
 
 // One run of spectrum values read from a spectrum held on the device:
 // count values from index src (zero outside [0, numdata)) to dst[off] with
@@ -565,12 +538,19 @@ struct jerk_polisher {
     WinSeg *d_segs = nullptr;  // window runs of a spectrum held on the device
     long long segs_cap = 0;
     PolishHarm *d_harms = nullptr;
-    int *d_best = nullptr;
-    float *d_bestpow = nullptr;
+    unsigned long long *d_best = nullptr;
     // pinned staging: rows, lists, harms, windows
     unsigned char *h_stage = nullptr;
     long long stage_cap = 0;
     long long candidates = 0;
+    PolishTw tables() const
+    {
+        PolishTw W;
+        W.tw = tw;
+        for (int i = 0; i < kNumSizes; i++)
+            W.off[i] = twoff[i];
+        return W;
+    }
 };
 
 namespace {
@@ -626,9 +606,13 @@ extern "C" int jerk_polisher_create(jerk_polisher **out, void *stream)
     if (e == cudaSuccess)
         e = cudaMalloc(&p->d_harms, sizeof(PolishHarm) * kMaxHarm);
     if (e == cudaSuccess)
-        e = cudaMalloc(&p->d_best, sizeof(int));
+        e = cudaMalloc(&p->d_best, sizeof(unsigned long long));
     if (e == cudaSuccess)
-        e = cudaMalloc(&p->d_bestpow, sizeof(float));
+        e = smem_attrs(pc_corr_kernel, false);
+    if (e == cudaSuccess)
+        e = smem_attrs(pd_data_kernel, false);
+    if (e == cudaSuccess)
+        e = smem_attrs(interp_w_kernel, false);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(p->stream);
     if (e != cudaSuccess) {
@@ -656,7 +640,6 @@ extern "C" void jerk_polisher_destroy(jerk_polisher *p)
     cudaFree(p->d_segs);
     cudaFree(p->d_harms);
     cudaFree(p->d_best);
-    cudaFree(p->d_bestpow);
     if (p->h_stage)
         cudaFreeHost(p->h_stage);
     if (p->own_stream && p->stream)
@@ -893,38 +876,38 @@ extern "C" int jerk_polish_rzw(jerk_polisher *p, const void *spectrum, long long
             e = p_dispatch<PW>(kSizes[s], (const PolishRow *)p->d_rows,
                                (const int *)p->d_lists + mfirst[s], mcount[s],
                                (const float2 *)(p->tw + p->twoff[s]), p->bank, maxkern[s], st);
-    // harmonics of equal fftlen are consecutive rows and consecutive harmonics
-    for (int hind = 0; hind < numharm && e == cudaSuccess;) {
-        int hend = hind + 1;
-        while (hend < numharm && H[hend].fftlen == H[hind].fftlen)
-            hend++;
-        const int N = H[hind].fftlen;
-        const int si = size_index(N);
-        const float2 *tw = p->tw + p->twoff[si];
-        const int first = (int)H[hind].row0, count = (hend - hind) * kCells;
-        e = p_dispatch<PK>(N, (const PolishRow *)p->d_rows, first, count, tw, p->bank, st);
-        if (e == cudaSuccess)
-            e = p_dispatch<PD>(N, (const PolishHarm *)p->d_harms, hind, hend - hind, tw,
-                               (const float2 *)p->windows, p->dfft, st);
-        if (e == cudaSuccess)
-            e = p_dispatch<PC>(N, (const PolishRow *)p->d_rows, first, count,
-                               (const PolishHarm *)p->d_harms, tw, (const float2 *)p->bank,
-                               (const float2 *)p->dfft, p->terms, p->tails, st);
-        hind = hend;
+    if (e == cudaSuccess) {
+        int N = 0;
+        for (const PolishHarm &h : H)
+            N = std::max(N, h.fftlen);
+        const PolishTw W = p->tables();
+        const int threads = N / 16 < 64 ? 64 : N / 16;  // the widest plan's (512 and less: 64)
+        const size_t b_buf = sizeof(float2) * (size_t)fft_buf_len_rt(N);
+        e = cudaMemsetAsync(p->d_best, 0, sizeof(unsigned long long), st);
+        if (e == cudaSuccess) {
+            pd_data_kernel<<<numharm, threads, b_buf, st>>>(p->d_harms, W, p->windows, p->dfft);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) {
+            pc_corr_kernel<<<(unsigned)nrows, threads, b_buf + sizeof(float2) * N, st>>>(
+                p->d_rows, p->d_harms, W, p->bank, p->dfft, p->terms, p->tails);
+            e = cudaGetLastError();
+        }
     }
     if (e == cudaSuccess) {
-        ps_argmax_kernel<<<1, kArgThreads, 0, st>>>(p->terms, p->tails, p->d_harms, numharm,
-                                                    p->d_best, p->d_bestpow);
+        ps_argmax_kernel<<<(kCells * kNumR + kArgThreads - 1) / kArgThreads, kArgThreads, 0, st>>>(
+            p->terms, p->tails, p->d_harms, numharm, p->d_best);
         e = cudaGetLastError();
     }
-    int best = 0;
-    float bpow = 0.0f;
+    unsigned long long key = 0;
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&best, p->d_best, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&bpow, p->d_bestpow, sizeof(float), cudaMemcpyDeviceToHost, st);
+        e = cudaMemcpyAsync(&key, p->d_best, sizeof(key), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(st);
+    const int best = key ? (int)(0xffffffffu - (unsigned)key) : 0;
+    float bpow = 0.0f;
+    const unsigned bits = (unsigned)(key >> 32);
+    memcpy(&bpow, &bits, sizeof bpow);
     if (e != cudaSuccess)
         return p_cuda(e, "jerk_polish_rzw");
     p->candidates++;
@@ -954,13 +937,6 @@ extern "C" int jerk_polish_rzw(jerk_polisher *p, const void *spectrum, long long
 namespace jerk {
 namespace {
 
-struct InterpPoint {
-    long long win;  // float2 offset of the staged data window (numkern bins)
-    double frac, z, w;
-    int numkern;    // 2 kern_half_width
-    int npts;       // w responses: the cosine series' length (M = npts / 2)
-};
-
 constexpr int kInterpThreads = 256;
 
 template <int NT>
@@ -972,7 +948,7 @@ __device__ __forceinline__ void block_sum2(double &a, double &b)
         b += __shfl_down_sync(0xffffffffu, b, o);
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
+    if (lane == 0 && wid < NT / 32) {  // a CTA may have more threads than the sum's NT
         red[0][wid] = a;
         red[1][wid] = b;
     }
@@ -1073,17 +1049,12 @@ __global__ void __launch_bounds__(kInterpThreads)
 // the numkern bins around M / 2 split out of the window that the last stage
 // drops into shared memory; then the correlation with the data window.
 template <int M>
-__global__ void __launch_bounds__(FftPlan<M>::T)
-    interp_w_kernel(const InterpPoint *__restrict__ pts, const int *__restrict__ list,
-                    const float2 *__restrict__ tw, const float2 *__restrict__ windows,
-                    float2 *__restrict__ ans)
+__device__ __forceinline__ void interp_w(const InterpPoint &P, int pi, const float2 *tw,
+                                         const float2 *__restrict__ windows,
+                                         float2 *__restrict__ ans, float2 *buf)
 {
     constexpr int T = FftPlan<M>::T;
-    extern __shared__ float2 iw_smem[];
-    float2 *buf = iw_smem;
-    float2 *win = iw_smem + fft_buf_len<M>();
-    const int pi = list[blockIdx.x];
-    const InterpPoint P = pts[pi];
+    float2 *win = buf + fft_buf_len<M>();
     const int tid = threadIdx.x, numkern = P.numkern, npts = P.npts;
     const double z = P.z, w = P.w;
     const double dt = 1.0 / (double)npts;
@@ -1114,7 +1085,7 @@ __global__ void __launch_bounds__(FftPlan<M>::T)
     __syncthreads();
     const float2 *d = windows + P.win;
     double ar = 0.0, ai = 0.0;
-    for (int k = tid; k < numkern; k += T) {
+    for (int k = tid < T ? tid : numkern; k < numkern; k += T) {
         const int kc = lo + k;
         const float2 a = win[k], b = win[numkern - k];
         const double hx = 0.5 * ((double)a.x + (double)b.x);
@@ -1131,19 +1102,25 @@ __global__ void __launch_bounds__(FftPlan<M>::T)
         ans[pi] = make_float2((float)ar, (float)ai);
 }
 
-template <int M> struct PI {
-    static cudaError_t run(const InterpPoint *pts, const int *list, int count, const float2 *tw,
-                           const float2 *windows, float2 *ans, int maxkern, cudaStream_t st)
-    {
-        const int smem = (int)(sizeof(float2) * (fft_buf_len<M>() + maxkern + 1));
-        cudaError_t e = cudaFuncSetAttribute(interp_w_kernel<M>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-        interp_w_kernel<M><<<count, FftPlan<M>::T, smem, st>>>(pts, list, tw, windows, ans);
-        return cudaGetLastError();
+// Every w point of a call in one launch, whatever its series' length (CTAs of
+// the longest one's threads; the first T of them form the sum).  A launch per
+// length took 32 us a call, three calls a candidate.
+__global__ void __launch_bounds__(512)
+    interp_w_kernel(const InterpPoint *__restrict__ pts, const int *__restrict__ list,
+                    const PolishTw W, const float2 *__restrict__ windows, float2 *__restrict__ ans)
+{
+    extern __shared__ float2 p_smem[];
+    const int pi = list[blockIdx.x];
+    const InterpPoint &P = pts[pi];
+    switch (P.npts / 2) {
+#define JERK_IW(MM, I) \
+    case MM: interp_w<MM>(P, pi, W.tw + W.off[I], windows, ans, p_smem); break;
+    JERK_IW(128, 0) JERK_IW(256, 1) JERK_IW(512, 2) JERK_IW(1024, 3) JERK_IW(2048, 4)
+    JERK_IW(4096, 5) JERK_IW(8192, 6)
+#undef JERK_IW
+    default: break;
     }
-};
+}
 
 int whw_high(double z, double w) { return w_resp_halfwidth_lowacc(z, w) + 32; }
 
@@ -1209,9 +1186,8 @@ int interp_points(jerk_polisher *p, const float2 *data, long long numdata, int n
         }
     }
     std::vector<int> lists(zr);
-    int wfirst[kNumSizes], wcount[kNumSizes];
-    for (int s = 0; s < kNumSizes; s++) {
-        wfirst[s] = (int)lists.size();
+    int wcount[kNumSizes];
+    for (int s = kNumSizes - 1; s >= 0; s--) {  // the longest first
         lists.insert(lists.end(), wl[s].begin(), wl[s].end());
         wcount[s] = (int)wl[s].size();
     }
@@ -1278,11 +1254,18 @@ int interp_points(jerk_polisher *p, const float2 *data, long long numdata, int n
                                                                      p->dfft);
         e = cudaGetLastError();
     }
-    for (int s = 0; s < kNumSizes && e == cudaSuccess; s++)
-        if (wcount[s])
-            e = p_dispatch<PI>(kSizes[s], d_pts, (const int *)p->d_lists + wfirst[s], wcount[s],
-                               (const float2 *)(p->tw + p->twoff[s]), (const float2 *)p->windows,
-                               p->dfft, maxkern[s], st);
+    const int nw = (int)(lists.size() - zr.size());
+    if (e == cudaSuccess && nw) {
+        int M = 0, smem = 0;
+        for (int s = 0; s < kNumSizes; s++)
+            if (wcount[s]) {
+                M = kSizes[s];
+                smem = std::max(smem, fft_buf_len_rt(M) + maxkern[s] + 1);
+            }
+        interp_w_kernel<<<nw, M / 16 < 64 ? 64 : M / 16, sizeof(float2) * smem, st>>>(
+            d_pts, p->d_lists + zr.size(), p->tables(), p->windows, p->dfft);
+        e = cudaGetLastError();
+    }
     float2 *hans = (float2 *)(hs + o_ans);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(hans, p->dfft, b_ans, cudaMemcpyDeviceToHost, st);
@@ -1314,39 +1297,107 @@ void localpower_points(double r, long long numdata, std::vector<double> &out)
         out.push_back(f);
 }
 
-int local_powers(jerk_polisher *p, const float2 *data, long long numdata, int n, const double *r,
-                 const double *z, const double *w, double *out)
+// Points whose interpolated values are asked for together.
+struct InterpList {
+    std::vector<double> r, z, w;
+    std::vector<int> khw;
+    std::vector<float2> a;
+    void add(double rr, double zz, double ww, int k)
+    {
+        r.push_back(rr);
+        z.push_back(zz);
+        w.push_back(ww);
+        khw.push_back(k);
+    }
+    int run(jerk_polisher *p, const float2 *data, long long numdata)
+    {
+        a.resize(r.size());
+        return r.empty() ? JERK_OK
+                         : interp_points(p, data, numdata, (int)r.size(), r.data(), z.data(),
+                                         w.data(), khw.data(), a.data());
+    }
+};
+
+// Local power of n points: their points, then from the values starting at
+// `first` the powers.
+void local_power_points(InterpList &L, long long numdata, int n, const double *r, const double *z,
+                        const double *w, std::vector<int> &owner)
 {
-    std::vector<double> pr, pz, pw;
-    std::vector<int> pk, owner;
     for (int i = 0; i < n; i++) {
         std::vector<double> f;
         localpower_points(r[i], numdata, f);
         const int khw = w_resp_halfwidth_lowacc(z[i], w[i]);
         for (double v : f) {
-            pr.push_back(v);
-            pz.push_back(z[i]);
-            pw.push_back(w[i]);
-            pk.push_back(khw);
+            L.add(v, z[i], w[i], khw);
             owner.push_back(i);
         }
     }
-    std::vector<float2> a(pr.size());
-    if (!pr.empty()) {
-        const int rc = interp_points(p, data, numdata, (int)pr.size(), pr.data(), pz.data(),
-                                     pw.data(), pk.data(), a.data());
-        if (rc != JERK_OK)
-            return rc;
-    }
+}
+
+void local_power_values(const InterpList &L, size_t first, int n, const std::vector<int> &owner,
+                        double *out)
+{
     for (int i = 0; i < n; i++)
         out[i] = 0.0;
-    for (size_t j = 0; j < pr.size(); j++) {
-        const double ar = a[j].x, ai = a[j].y;
+    for (size_t j = 0; j < owner.size(); j++) {
+        const double ar = L.a[first + j].x, ai = L.a[first + j].y;
         out[owner[j]] += ar * ar + ai * ai;
     }
     for (int i = 0; i < n; i++)
         out[i] /= 20.0;  // NUMLOCPOWAVG
-    return JERK_OK;
+}
+
+int local_powers(jerk_polisher *p, const float2 *data, long long numdata, int n, const double *r,
+                 const double *z, const double *w, double *out)
+{
+    InterpList L;
+    std::vector<int> owner;
+    local_power_points(L, numdata, n, r, z, w, owner);
+    const int rc = L.run(p, data, numdata);
+    if (rc == JERK_OK)
+        local_power_values(L, 0, n, owner, out);
+    return rc;
+}
+
+// get_derivs3d (src/characteristics.c:138-191): 5 points 0.003 apart around r
+// at HIGHACC, powers and phases, finite differences.
+void derivs_points(InterpList &L, int n, const double *r, const double *z, const double *w)
+{
+    const double h = 0.003, twoh = 0.006;
+    for (int i = 0; i < n; i++) {
+        const int khw = whw_high(z[i], w[i]);
+        double f = r[i] - twoh;
+        for (int k = 0; k < 5; k++, f += h)
+            L.add(f, z[i], w[i], khw);
+    }
+}
+
+void derivs_values(const InterpList &L, size_t first, int n, const double *locpow,
+                   jerk_rderivs *out)
+{
+    const double twoh = 0.006, twohsqrd = 0.000036;
+    const double twopi = 6.2831853071795864769252867665590057683943387987502;
+    for (int i = 0; i < n; i++) {
+        double pwr[5], phs[5];
+        for (int k = 0; k < 5; k++) {
+            const float2 a = L.a[first + 5 * (size_t)i + k];
+            const double ar = a.x, ai = a.y;
+            pwr[k] = ar * ar + ai * ai;
+            const double t = atan2(ai, ar);
+            phs[k] = t > 0.0 ? t : t + twopi;
+        }
+        for (int k = 0; k < 4; k++)
+            if (fabs(phs[k + 1] - phs[k]) > M_PI)
+                phs[k + 1] -= twopi;
+        jerk_rderivs &d = out[i];
+        d.pow = pwr[2];
+        d.phs = phs[2];
+        d.dpow = (pwr[3] - pwr[1]) / twoh;
+        d.dphs = (phs[3] - phs[1]) / twoh;
+        d.d2pow = (pwr[4] - 2.0 * pwr[2] + pwr[0]) / twohsqrd;
+        d.d2phs = (phs[4] - 2.0 * phs[2] + phs[0]) / twohsqrd;
+        d.locpow = locpow[i];
+    }
 }
 
 }  // namespace
@@ -1365,50 +1416,12 @@ extern "C" int jerk_derivs(jerk_polisher *p, const void *spectrum, long long num
 {
     if (!p || !spectrum || n < 0 || (n && (!r || !z || !w || !locpow || !out)))
         return p_fail(JERK_EINVAL, "jerk_derivs: bad argument");
-    // get_derivs3d (src/characteristics.c:138-191): 5 points 0.003 apart
-    // around r at HIGHACC, powers and phases, finite differences
-    const double h = 0.003, twoh = 0.006, twohsqrd = 0.000036;
-    std::vector<double> pr(5 * (size_t)n), pz(5 * (size_t)n), pw(5 * (size_t)n);
-    std::vector<int> pk(5 * (size_t)n);
-    for (int i = 0; i < n; i++) {
-        const int khw = whw_high(z[i], w[i]);
-        double f = r[i] - twoh;
-        for (int k = 0; k < 5; k++, f += h) {
-            pr[5 * i + k] = f;
-            pz[5 * i + k] = z[i];
-            pw[5 * i + k] = w[i];
-            pk[5 * i + k] = khw;
-        }
-    }
-    std::vector<float2> a(pr.size());
-    if (n) {
-        const int rc = interp_points(p, (const float2 *)spectrum, numdata, 5 * n, pr.data(),
-                                     pz.data(), pw.data(), pk.data(), a.data());
-        if (rc != JERK_OK)
-            return rc;
-    }
-    const double twopi = 6.2831853071795864769252867665590057683943387987502;
-    for (int i = 0; i < n; i++) {
-        double pwr[5], phs[5];
-        for (int k = 0; k < 5; k++) {
-            const double ar = a[5 * i + k].x, ai = a[5 * i + k].y;
-            pwr[k] = ar * ar + ai * ai;
-            const double t = atan2(ai, ar);
-            phs[k] = t > 0.0 ? t : t + twopi;
-        }
-        for (int k = 0; k < 4; k++)
-            if (fabs(phs[k + 1] - phs[k]) > M_PI)
-                phs[k + 1] -= twopi;
-        jerk_rderivs &d = out[i];
-        d.pow = pwr[2];
-        d.phs = phs[2];
-        d.dpow = (pwr[3] - pwr[1]) / twoh;
-        d.dphs = (phs[3] - phs[1]) / twoh;
-        d.d2pow = (pwr[4] - 2.0 * pwr[2] + pwr[0]) / twohsqrd;
-        d.d2phs = (phs[4] - 2.0 * phs[2] + phs[0]) / twohsqrd;
-        d.locpow = locpow[i];
-    }
-    return JERK_OK;
+    InterpList L;
+    derivs_points(L, n, r, z, w);
+    const int rc = L.run(p, (const float2 *)spectrum, numdata);
+    if (rc == JERK_OK)
+        derivs_values(L, 0, n, locpow, out);
+    return rc;
 }
 
 // The whole default optimisation of one candidate on the GPU, as
@@ -1446,10 +1459,18 @@ extern "C" int jerk_optimize_cand(jerk_polisher *p, const void *spectrum, long l
         z[i] = rzw_out[1] * hh;
         w[i] = rzw_out[2] * hh;
     }
-    rc = jerk_local_power(p, spectrum, numdata, numharm, r, z, w, lp);
+    // the local powers and the derivatives at the polished point, one call
+    InterpList L;
+    std::vector<int> owner;
+    local_power_points(L, numdata, numharm, r, z, w, owner);
+    const size_t nlp = L.r.size();
+    derivs_points(L, numharm, r, z, w);
+    rc = L.run(p, (const float2 *)spectrum, numdata);
     if (rc != JERK_OK)
         return rc;
+    local_power_values(L, 0, numharm, owner, lp);
     for (int i = 0; i < numharm; i++)
         lp[i] = (double)(float)lp[i];  // a float there, as the reference holds it
-    return jerk_derivs(p, spectrum, numdata, numharm, r, z, w, lp, derivs);
+    derivs_values(L, nlp, numharm, lp, derivs);
+    return JERK_OK;
 }
