@@ -408,11 +408,12 @@ typedef struct jerk_dedisperser jerk_dedisperser;
 int jerk_dedisperser_create(jerk_dedisperser **dedisperser, int worklen, int nsub, int numdms,
                             const int *offsets);
 void jerk_dedisperser_destroy(jerk_dedisperser *dedisperser);
-/* the tiling chosen: DMs per CTA group and samples per tile */
+/* the tiling launched: DMs per CTA group and samples per tile */
 int jerk_dedisperser_shape(const jerk_dedisperser *dedisperser, int *group_dms, int *tile_samples);
-/* Host only (no CUDA call): the checks and the tiling choice of
- * jerk_dedisperser_create for a host offsets table, with the shared memory a
- * CTA takes. */
+/* Host only (no CUDA call): the checks of jerk_dedisperser_create for a host
+ * offsets table and a tiling that fits, with the shared memory a CTA takes.
+ * The dedisperser launches the tiling of least estimated time among those
+ * that leave two CTAs per SM, and this one where there is none. */
 int jerk_dedisp_plan(int worklen, int nsub, int numdms, const int *offsets, int *group_dms,
                      int *tile_samples, long long *smem_bytes);
 int jerk_dedisperser_matches(const jerk_dedisperser *dedisperser, int worklen, int nsub, int numdms,

@@ -538,9 +538,9 @@ def downsample_subbands(data, bs: int, out=None):
 
 
 def dedisp_plan(worklen: int, nsub: int, offsets) -> Tuple[int, int, int]:
-    """The tiling a Dedisperser would choose for these offsets (host only,
-    jerk_dedisp_plan): (DMs per CTA group, samples per tile, shared-memory
-    bytes per CTA).  Raises JerkError on offsets outside [0, worklen]."""
+    """A tiling that fits these offsets (host only, jerk_dedisp_plan; what a
+    Dedisperser launches is its .shape): (DMs per CTA group, samples per tile,
+    shared-memory bytes per CTA).  Raises JerkError on offsets outside [0, worklen]."""
     off = np.ascontiguousarray(offsets, dtype=np.int32)
     if off.ndim != 2 or off.shape[1] != nsub:
         raise JerkError(JERK_EINVAL, "dedisp_plan: offsets must be [numdms, nsub]")
