@@ -2,6 +2,7 @@
 // them, and the status bits the kernels report through.
 #pragma once
 
+#include <utility>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -72,6 +73,39 @@ inline cudaError_t smem_attrs(K kernel, bool carveout)
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  (int)cudaSharedmemCarveoutMaxShared);
     return e;
+}
+
+// Launches a kernel that may start while the one before it in the stream runs
+// (follow): its CTAs take the SMs that the other's last CTAs leave idle.  The
+// kernel before calls let_follow first thing, so that this one starts once
+// the other's CTAs have all started; this one calls wait_before at its end, so that
+// whatever is launched after it finds both complete.  Between let_follow and
+// wait_before the two must not depend on one another.
+template <class... Par, class... Arg>
+inline cudaError_t launch_follow(void (*kernel)(Par...), unsigned grid, unsigned block, size_t smem,
+                                 cudaStream_t st, bool follow, Arg &&...args)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = follow ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Arg>(args)...);
+}
+
+__device__ __forceinline__ void let_follow()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+__device__ __forceinline__ void wait_before()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // this CTA's rsteps: all of the batch, or a share of them when a small

@@ -56,11 +56,13 @@ cudaError_t launch_fold_rows(const float2 *bank, const FoldSrc *src, int nrows, 
 int fold_twiddle_size(int L);
 void fold_twiddle_table(int L, float2 *out);
 cudaError_t fold_attrs(int L);
-cudaError_t launch_corr_fold(int L, const SearchDev &P, const FoldRows &R, cudaStream_t st);
+cudaError_t launch_corr_fold(int L, const SearchDev &P, const FoldRows &R, bool follow,
+                             cudaStream_t st);
 bool multi_takes(const FoldRows &R);
 cudaError_t multi_attrs();
 cudaError_t launch_corr_multi(const SearchDev *P, int np, const int (*sets)[2],
-                              const FoldRows *const *rows, int nsets, cudaStream_t st);
+                              const FoldRows *const *rows, int nsets, bool follow,
+                              cudaStream_t st);
 int fold_cta_rows(int L);
 int fold_wave_ctas(int L);
 int harmsum_wave_ctas(int nstages);
@@ -800,7 +802,7 @@ struct jerk_plan {
     std::vector<StepDev> hsteps;  // [nrsteps][nsubs]
     std::map<int, std::vector<int>> groups;  // fftlen -> subs, the long unfolded lengths
     std::vector<FoldRows> rowsets;  // folded half lengths, then short unfolded lengths
-    std::vector<char> own_launch;   // per row set: fills the GPU in a launch of its own
+    std::vector<char> own_launch;   // per row set: launched by itself (own_launch_wins)
     FoldRows *d_rowsets = nullptr;
     std::vector<FoldClass> fold_classes;
     std::vector<std::vector<double>> class_rows;  // [half length index][class] live rows
@@ -1123,6 +1125,20 @@ static int build_harm_tma(jerk_plan *p, bool in_smem)
 // prepared windows from *data_off on) and write the folded rows, class after
 // class, longest half length first; then the maps of the short lengths that
 // do not fold (fftlen 128 to 384).
+// Whether a row set is launched by itself rather than merged with others: its
+// CTAs make two waves; or, for the half lengths whose rows leave a warp of the
+// merged launch's four idle (768, 640, 384), four waves over the rsteps --
+// the launches overlap, so that a last partial wave is no loss.  Measured (us
+// per pass; merged against own): 6 trials of 2^21 samples, zmax 50, wmax 150,
+// 8 harmonics 105900 / 101300; 2^22 samples, zmax 100, 16 harmonics 14660 /
+// 14500, and 15300 with its 359 rows of 1024 by themselves as well.
+static bool own_launch_wins(int L, long long n, int batch)
+{
+    const long long groups = n / fold_cta_rows(L), wave = fold_wave_ctas(L);
+    const bool idle = L == 768 || L == 640 || L == 384;
+    return groups >= 2 * wave || (idle && groups * batch >= 4 * wave);
+}
+
 static int fold_bank(jerk_plan *p, const std::vector<int> &maxnumrs, long long *data_off)
 {
     std::map<int, std::vector<int>> subs_of;  // fftlen -> subharmonics
@@ -1291,9 +1307,7 @@ static int fold_bank(jerk_plan *p, const std::vector<int> &maxnumrs, long long *
         R.rows = p->d_fold + at;
         R.map = p->d_foldmap + row;
         p->rowsets.push_back(R);
-        // two waves of CTAs by themselves gain nothing from the merged launch
-        p->own_launch.push_back(!multi_takes(R) ||
-                                n / fold_cta_rows(L) >= 2 * fold_wave_ctas(L));
+        p->own_launch.push_back(!multi_takes(R) || own_launch_wins(L, n, p->batch));
         row += n;
         at += n * 2 * L;
     }
@@ -1760,6 +1774,7 @@ static int run_volumes(jerk_plan *p, SearchDev &a)
     int sets[kMaxRowSets][2], nsets = 0;
     const FoldRows *rows[kMaxRowSets];
     double mbytes = 0, mflops = 0;
+    bool follow = false;  // a correlation launch of this batch runs before
     for (size_t i = 0; i < p->rowsets.size(); i++) {
         const FoldRows &R = p->rowsets[i];
         if (!p->own_launch[i]) {
@@ -1775,14 +1790,15 @@ static int run_volumes(jerk_plan *p, SearchDev &a)
             rowset_work(p, a, R, &bytes, &flops);
         const int tok = launch_begin(p, kclass(p, "corr_fold_" + std::to_string(R.len)), bytes,
                                      flops);
-        e = launch_corr_fold(R.len, a, R, p->stream);
+        e = launch_corr_fold(R.len, a, R, follow, p->stream);
+        follow = true;
         launch_end(p, tok);
         if (e != cudaSuccess)
             return cuda_fail(e, "corr_fold_kernel");
     }
     if (nsets) {
         const int tok = launch_begin(p, kclass(p, "corr_multi"), mbytes, mflops);
-        e = launch_corr_multi(&a, 1, sets, rows, nsets, p->stream);
+        e = launch_corr_multi(&a, 1, sets, rows, nsets, follow, p->stream);
         launch_end(p, tok);
         if (e != cudaSuccess)
             return cuda_fail(e, "corr_multi_kernel");
@@ -2150,6 +2166,7 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
     int sets[kMaxGroupPlans * kMaxRowSets][2], nsets = 0;
     const FoldRows *rows[kMaxGroupPlans * kMaxRowSets];
     double mbytes = 0, mflops = 0;
+    bool follow = false;  // a correlation launch of this wave runs before
     for (int i = 0; i < n; i++) {
         jerk_plan *p = W[i];
         const SearchDev &a = p->pass.a;
@@ -2176,7 +2193,8 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
             }
             tok = launch_begin(p0, kclass(p0, "wave_corr_fold_" + std::to_string(R.len)), bytes,
                                flops);
-            e = launch_corr_fold(R.len, a, R, st);
+            e = launch_corr_fold(R.len, a, R, follow, st);
+            follow = true;
             launch_end(p0, tok);
             if (e != cudaSuccess)
                 return fail_all(e, "corr_fold_kernel");
@@ -2184,7 +2202,7 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
     }
     if (nsets) {
         tok = launch_begin(p0, kclass(p0, "wave_corr_multi"), mbytes, mflops);
-        e = launch_corr_multi(M.P, n, sets, rows, nsets, st);
+        e = launch_corr_multi(M.P, n, sets, rows, nsets, follow, st);
         launch_end(p0, tok);
         if (e != cudaSuccess)
             return fail_all(e, "corr_multi_kernel");

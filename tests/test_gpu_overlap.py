@@ -1,0 +1,42 @@
+"""Overlapped launches of a batch: plain passes, passes replayed from a graph and
+passes with events between all launches (each then waits for the one before)
+give the same hits, bit for bit, also when repeated -- with row sets launched by
+themselves, merged, and both, and a short last batch."""
+
+import numpy as np
+import pytest
+
+from prestozl_b200 import jerk
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("zmax,wmax,numharm,batch,rsteps", [
+    (20, 60, 8, 8, 27), (100, 0, 16, 32, 70), (50, 140, 8, 32, 65), (150, 200, 4, 16, 20),
+    (260, 300, 1, 4, 9)])
+def test_overlapped_launches_equal_serial(zmax, wmax, numharm, batch, rsteps):
+    torch = pytest.importorskip("torch")
+    N = 1 << 21
+    g = torch.Generator(device="cuda")
+    g.manual_seed(zmax + numharm)
+    spec = torch.view_as_complex(torch.randn((N // 2, 2), generator=g, device="cuda"))
+    spec[40_000::3001] *= 12.0
+    obs, fftlen, _ = jerk.obs_from_params(N // 2, N, 64e-6, zmax, wmax, numharm, 3.0,
+                                          wmax_given=wmax > 0)
+    for i in range(obs.numharmstages):
+        obs.powcut[i] = 11.0 + 3.0 * (1 << i) ** 0.75
+    subs = jerk.subharm_sizes(obs, fftlen)
+    bank = jerk.DeviceBank(subs)
+    want = None
+    for profile, graph in ((True, False), (False, False), (False, True)):
+        plan = jerk.JerkPlan(obs, subs, batch=batch, device_bank=bank.ptr.value, use_graph=graph)
+        plan.set_profiling(profile)
+        for _ in range(1 if profile else 4):
+            got = plan.search(spec, 3, rsteps, want_hits=True)[1:]
+            if want is None:
+                want = got
+                assert len(want[0]) > 0
+            assert np.array_equal(got[0], want[0])
+            assert np.array_equal(got[1].view(np.uint32), want[1].view(np.uint32))
+        plan.close()
+    bank.close()
