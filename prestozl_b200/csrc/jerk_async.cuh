@@ -75,26 +75,29 @@ inline cudaError_t smem_attrs(K kernel, bool carveout)
     return e;
 }
 
-// Launches a kernel that may start while the one before it in the stream runs
-// (follow): its CTAs take the SMs that the other's last CTAs leave idle.  The
-// kernel before calls let_follow first thing, so that this one starts once
-// the other's CTAs have all started; this one calls wait_before at its end, so that
-// whatever is launched after it finds both complete.  Between let_follow and
-// wait_before the two must not depend on one another.
+// Launches a kernel that may start while the one before it in the stream runs:
+// its CTAs take the SMs that the other's last CTAs leave idle, and
+// the launch itself costs no gap.  The kernel before calls let_follow, so that
+// this one starts once all of the other's CTAs have; without the call, when
+// they have ended.  wait_before returns when the kernel before has ended and
+// its writes can be read.  A kernel that needs those calls wait_before first thing;
+// one that does not calls it last, so that whatever comes after it finds both
+// complete.  A kernel that waits first calls let_follow only after: the one
+// that follows may count on all that came before.
 template <class... Par, class... Arg>
-inline cudaError_t launch_follow(void (*kernel)(Par...), unsigned grid, unsigned block, size_t smem,
-                                 cudaStream_t st, bool follow, Arg &&...args)
+inline cudaError_t launch_follow(void (*kernel)(Par...), dim3 grid, unsigned block, size_t smem,
+                                 cudaStream_t st, Arg &&...args)
 {
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = &at;
-    cfg.numAttrs = follow ? 1 : 0;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Arg>(args)...);
 }
 

@@ -571,8 +571,10 @@ __device__ __forceinline__ void fold_cta(const SearchDev &P, const FoldRows &R, 
 template <int L>
 __global__ void __launch_bounds__(Fold<L>::Threads, Fold<L>::Occ)
     corr_fold_kernel(const __grid_constant__ SearchDev P, const __grid_constant__ FoldRows R,
-                     const int ny)
+                     const int ny, const bool first)
 {
+    if (first)  // of its batch: the rows come from the kernel before
+        wait_before();
     let_follow();
     int b0, b1;
     rstep_chunk(P.nb, ny, blockIdx.x % ny, &b0, &b1);
@@ -597,8 +599,10 @@ struct Multi {
 
 template <int NP>
 __global__ void __launch_bounds__(kMultiThreads, kMultiOcc)
-    corr_multi_kernel(const __grid_constant__ MultiLaunch<NP> M)
+    corr_multi_kernel(const __grid_constant__ MultiLaunch<NP> M, const bool first)
 {
+    if (first)
+        wait_before();
     let_follow();
     int j = 0;
     while (j + 1 < M.n && (int)blockIdx.x >= M.seg[j + 1].cta0)
@@ -646,12 +650,12 @@ template <int L>
 struct FoldOps {
     using F = Fold<L>;
     static cudaError_t attrs() { return smem_attrs(corr_fold_kernel<L>, true); }
-    static cudaError_t launch(const SearchDev &P, const FoldRows &R, bool follow, cudaStream_t st)
+    static cudaError_t launch(const SearchDev &P, const FoldRows &R, bool first, cudaStream_t st)
     {
         const int groups = R.n / F::Rows;
         const int split = fold_split(groups, sm_count() * F::Occ, P.nb);
         return launch_follow(corr_fold_kernel<L>, (unsigned)(groups * split), F::Threads, F::Smem,
-                             st, follow, P, R, split);
+                             st, P, R, split, first);
     }
 };
 
@@ -672,10 +676,10 @@ struct FoldOps {
 
 cudaError_t fold_attrs(int L) { JERK_FOLD_DISPATCH(L, attrs()) }
 
-cudaError_t launch_corr_fold(int L, const SearchDev &P, const FoldRows &R, bool follow,
+cudaError_t launch_corr_fold(int L, const SearchDev &P, const FoldRows &R, bool first,
                              cudaStream_t st)
 {
-    JERK_FOLD_DISPATCH(L, launch(P, R, follow, st))
+    JERK_FOLD_DISPATCH(L, launch(P, R, first, st))
 }
 
 // Row groups and shared memory of one row set in the merged launch; groups 0
@@ -717,7 +721,7 @@ cudaError_t multi_attrs()
 
 template <int NP>
 static cudaError_t launch_multi_n(const SearchDev *P, int np, const int (*sets)[2],
-                                  const FoldRows *const *rows, int nsets, bool follow,
+                                  const FoldRows *const *rows, int nsets, bool first,
                                   cudaStream_t st)
 {
     MultiLaunch<NP> M;
@@ -751,19 +755,20 @@ static cudaError_t launch_multi_n(const SearchDev *P, int np, const int (*sets)[
     }
     if (x <= 0 || x >= (1ll << 31))
         return cudaErrorInvalidValue;
-    return launch_follow(corr_multi_kernel<NP>, (unsigned)x, kMultiThreads, smem, st, follow, M);
+    return launch_follow(corr_multi_kernel<NP>, (unsigned)x, kMultiThreads, smem, st, M,
+                         first);
 }
 
 // Row sets sets[j] = (plan, row set), rows[j] their host copies; P the np
 // plans' arguments.
 cudaError_t launch_corr_multi(const SearchDev *P, int np, const int (*sets)[2],
-                              const FoldRows *const *rows, int nsets, bool follow,
+                              const FoldRows *const *rows, int nsets, bool first,
                               cudaStream_t st)
 {
     if (np < 1 || np > kMaxGroupPlans || nsets < 1 || nsets > np * kMaxRowSets)
         return cudaErrorInvalidValue;
-    return np == 1 ? launch_multi_n<1>(P, np, sets, rows, nsets, follow, st)
-                   : launch_multi_n<kMaxGroupPlans>(P, np, sets, rows, nsets, follow, st);
+    return np == 1 ? launch_multi_n<1>(P, np, sets, rows, nsets, first, st)
+                   : launch_multi_n<kMaxGroupPlans>(P, np, sets, rows, nsets, first, st);
 }
 
 // kernel rows a CTA takes, and CTAs of one full wave

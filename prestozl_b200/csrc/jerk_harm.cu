@@ -73,6 +73,12 @@ struct Ring {
     static constexpr int All = Threads + 32;
     static constexpr int C = Cols * Threads;  // r cells per tile
     static constexpr int Occ = RingShape<S>::Occ;
+    // whether the launch may come before the last correlation CTAs have ended:
+    // it saves the gap (zmax 200, wmax 300, 4 harmonics, 96 rsteps 5110 ->
+    // 4930 us a pass; zmax 100, 16 harmonics 14.33 -> 14.13 ms), but small
+    // CTAs that come in one by one lose more (1 harmonic 2935 -> 3240 us; zmax
+    // 300, wmax 600, 2 harmonics 12.34 -> 12.80 ms)
+    static constexpr bool Early = Occ < 3;
     // cells of subharmonic s that C fundamental cells can touch: the index
     // grows by at most floor((C - 1) hf) + 1, the piece starts on a multiple
     // of kPlaneAlign cells and ends on one (whole 32-byte sectors)
@@ -450,6 +456,7 @@ template <int S, int Q>
 __global__ void __launch_bounds__(Ring<S, Q>::All, Ring<S, Q>::Occ)
     harmsum_ring_kernel(const __grid_constant__ SearchDev P, const __grid_constant__ RingPlan W)
 {
+    wait_before();
     ring_body<S, Ring<S, Q>>(P, W, blockIdx.x, gridDim.x);
 }
 
@@ -463,6 +470,7 @@ template <int S, int Q>
 __global__ void __launch_bounds__(Ring<S, Q>::All, Ring<S, Q>::Occ)
     harmsum_ring_group_kernel(const __grid_constant__ RingGroup G)
 {
+    wait_before();
     int i = 0;
     while (i + 1 < G.M.n && (int)blockIdx.x >= G.M.cta0[i + 1])
         i++;
@@ -515,8 +523,10 @@ struct RingOps {
     static cudaError_t launch_q(const SearchDev &P, const RingPlan &W, cudaStream_t st)
     {
         using R = Ring<S, Q>;
-        harmsum_ring_kernel<S, Q>
-            <<<std::min(W.items, sm_count() * R::Occ), R::All, R::Smem, st>>>(P, W);
+        const int x = std::min(W.items, sm_count() * R::Occ);
+        if (R::Early)
+            return launch_follow(harmsum_ring_kernel<S, Q>, (unsigned)x, R::All, R::Smem, st, P, W);
+        harmsum_ring_kernel<S, Q><<<x, R::All, R::Smem, st>>>(P, W);
         return cudaGetLastError();
     }
     static cudaError_t launch(const SearchDev &P, cudaStream_t st)
@@ -552,6 +562,9 @@ struct RingOps {
             x += std::min(G.W[i].items, share);
         }
         G.M.cta0[M.n] = x;
+        if (R::Early)
+            return launch_follow(harmsum_ring_group_kernel<S, QMax>, (unsigned)x, R::All, R::Smem,
+                                 st, G);
         harmsum_ring_group_kernel<S, QMax><<<x, R::All, R::Smem, st>>>(G);
         return cudaGetLastError();
     }

@@ -365,6 +365,8 @@ template <bool LONG>
 __global__ void __launch_bounds__(LONG ? 1024 : 256, LONG ? 1 : 2)
     prep_kernel(const __grid_constant__ SearchDev P)
 {
+    wait_before();
+    let_follow();
     prep_dispatch<LONG>(P, blockIdx.x, blockIdx.y);
 }
 
@@ -381,6 +383,8 @@ template <bool LONG>
 __global__ void __launch_bounds__(LONG ? 1024 : 256, LONG ? 1 : 2)
     prep_group_kernel(const __grid_constant__ GroupLaunch M)
 {
+    wait_before();
+    let_follow();
     const int i = group_plan(M, blockIdx.x);
     const int local = blockIdx.x - M.cta0[i];
     const int nsubs = M.P[i].nsubs;
@@ -427,6 +431,7 @@ __global__ void __launch_bounds__(FftPlan<N>::T, CorrOcc<N>::value)
     float2 *tws = sm2 + fft_buf_len<N>();
     float2 *dsm = sm2 + CorrSmem<N>::kBase;  // staged data row (kStage)
     const int tid = threadIdx.x;
+    wait_before();
     const int row = blockIdx.x;
     int gi = 0;
     while (gi + 1 < G.n && row >= G.rowstart[gi + 1])
@@ -786,6 +791,7 @@ template <int S, int ZU, bool PF>
 __global__ void __launch_bounds__(kHarmThreads, HarmOcc<S, ZU>::value)
     harmsum_kernel(const __grid_constant__ SearchDev P, const __grid_constant__ HarmTma T)
 {
+    wait_before();
     harmsum_body<S, ZU, PF>(P, &T, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -794,6 +800,7 @@ template <int S>
 __global__ void __launch_bounds__(kHarmThreads, HarmOcc<S, 4>::value)
     harmsum_group_kernel(const __grid_constant__ GroupLaunch M)
 {
+    wait_before();
     const int i = group_plan(M, blockIdx.x);
     const int local = blockIdx.x - M.cta0[i];
     const int nx = M.nx[i], nw = M.P[i].numw0;
@@ -1081,10 +1088,8 @@ cudaError_t launch_prep(const SearchDev &P, int maxfft, size_t smem, cudaStream_
 {
     const dim3 grid(P.nb, P.nsubs);
     if (maxfft > kPrepLong)
-        prep_kernel<true><<<grid, prep_threads(maxfft), smem, st>>>(P);
-    else
-        prep_kernel<false><<<grid, 256, smem, st>>>(P);
-    return cudaGetLastError();
+        return launch_follow(prep_kernel<true>, grid, prep_threads(maxfft), smem, st, P);
+    return launch_follow(prep_kernel<false>, grid, 256, smem, st, P);
 }
 
 template <int N>
@@ -1094,8 +1099,7 @@ static cudaError_t launch_corr_n(const SearchDev &P, const RowGroup &G, int rows
     // a group with fewer rows than two waves of CTAs also splits its rsteps
     const int wave = sm_count() * CorrOcc<N>::value;
     const int split = rows >= 2 * wave ? 1 : std::max(1, std::min(P.nb, (2 * wave + rows - 1) / rows));
-    corr_kernel<N><<<dim3(rows, split), FftPlan<N>::T, smem, st>>>(P, G);
-    return cudaGetLastError();
+    return launch_follow(corr_kernel<N>, dim3(rows, split), FftPlan<N>::T, smem, st, P, G);
 }
 
 cudaError_t corr_attrs(int fftlen)
@@ -1147,8 +1151,7 @@ static cudaError_t launch_harmsum_s(const SearchDev &P, const HarmTma &T, cudaSt
 {
     const size_t smem = harmsum_smem_bytes(P.nsubs, P.numz0);
     const dim3 grid((P.corr_uselen + kHarmThreads - 1) / kHarmThreads, P.numw0, P.nb);
-    harmsum_kernel<S, 4, PF><<<grid, kHarmThreads, smem, st>>>(P, T);
-    return cudaGetLastError();
+    return launch_follow(harmsum_kernel<S, 4, PF>, grid, kHarmThreads, smem, st, P, T);
 }
 
 template <bool PF>
@@ -1188,10 +1191,9 @@ cudaError_t launch_prep_group(GroupLaunch M, int maxfft, size_t smem, cudaStream
     }
     M.cta0[M.n] = x;
     if (maxfft > kPrepLong)
-        prep_group_kernel<true><<<x, prep_threads(maxfft), smem, st>>>(M);
-    else
-        prep_group_kernel<false><<<x, 256, smem, st>>>(M);
-    return cudaGetLastError();
+        return launch_follow(prep_group_kernel<true>, (unsigned)x, prep_threads(maxfft), smem, st,
+                             M);
+    return launch_follow(prep_group_kernel<false>, (unsigned)x, 256, smem, st, M);
 }
 
 int harmsum_wave_ctas(int nstages)
@@ -1214,8 +1216,7 @@ static cudaError_t launch_harmsum_group_s(GroupLaunch &M, cudaStream_t st)
     if (x >= (1ll << 31))
         return cudaErrorInvalidValue;
     M.cta0[M.n] = (int)x;
-    harmsum_group_kernel<S><<<(unsigned)x, kHarmThreads, smem, st>>>(M);
-    return cudaGetLastError();
+    return launch_follow(harmsum_group_kernel<S>, (unsigned)x, kHarmThreads, smem, st, M);
 }
 
 // Every plan of M must have nstages stages.

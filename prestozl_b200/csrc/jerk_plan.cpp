@@ -56,12 +56,12 @@ cudaError_t launch_fold_rows(const float2 *bank, const FoldSrc *src, int nrows, 
 int fold_twiddle_size(int L);
 void fold_twiddle_table(int L, float2 *out);
 cudaError_t fold_attrs(int L);
-cudaError_t launch_corr_fold(int L, const SearchDev &P, const FoldRows &R, bool follow,
+cudaError_t launch_corr_fold(int L, const SearchDev &P, const FoldRows &R, bool first,
                              cudaStream_t st);
 bool multi_takes(const FoldRows &R);
 cudaError_t multi_attrs();
 cudaError_t launch_corr_multi(const SearchDev *P, int np, const int (*sets)[2],
-                              const FoldRows *const *rows, int nsets, bool follow,
+                              const FoldRows *const *rows, int nsets, bool first,
                               cudaStream_t st);
 int fold_cta_rows(int L);
 int fold_wave_ctas(int L);
@@ -1774,7 +1774,7 @@ static int run_volumes(jerk_plan *p, SearchDev &a)
     int sets[kMaxRowSets][2], nsets = 0;
     const FoldRows *rows[kMaxRowSets];
     double mbytes = 0, mflops = 0;
-    bool follow = false;  // a correlation launch of this batch runs before
+    bool first = p->groups.empty();  // the next launch follows the prepared rows' own
     for (size_t i = 0; i < p->rowsets.size(); i++) {
         const FoldRows &R = p->rowsets[i];
         if (!p->own_launch[i]) {
@@ -1790,15 +1790,15 @@ static int run_volumes(jerk_plan *p, SearchDev &a)
             rowset_work(p, a, R, &bytes, &flops);
         const int tok = launch_begin(p, kclass(p, "corr_fold_" + std::to_string(R.len)), bytes,
                                      flops);
-        e = launch_corr_fold(R.len, a, R, follow, p->stream);
-        follow = true;
+        e = launch_corr_fold(R.len, a, R, first, p->stream);
+        first = false;
         launch_end(p, tok);
         if (e != cudaSuccess)
             return cuda_fail(e, "corr_fold_kernel");
     }
     if (nsets) {
         const int tok = launch_begin(p, kclass(p, "corr_multi"), mbytes, mflops);
-        e = launch_corr_multi(&a, 1, sets, rows, nsets, follow, p->stream);
+        e = launch_corr_multi(&a, 1, sets, rows, nsets, first, p->stream);
         launch_end(p, tok);
         if (e != cudaSuccess)
             return cuda_fail(e, "corr_multi_kernel");
@@ -2166,7 +2166,7 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
     int sets[kMaxGroupPlans * kMaxRowSets][2], nsets = 0;
     const FoldRows *rows[kMaxGroupPlans * kMaxRowSets];
     double mbytes = 0, mflops = 0;
-    bool follow = false;  // a correlation launch of this wave runs before
+    bool first = true;  // the next launch follows the prepared rows' own
     for (int i = 0; i < n; i++) {
         jerk_plan *p = W[i];
         const SearchDev &a = p->pass.a;
@@ -2175,6 +2175,7 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
             tok = launch_begin(p0, kclass(p0, "wave_corr_" + std::to_string(kv.first)), 0.0, 0.0);
             e = launch_corr(a, kv.first, G, G.rowstart[G.n], st);
             launch_end(p0, tok);
+            first = false;
             if (e != cudaSuccess)
                 return fail_all(e, "corr_kernel");
         }
@@ -2193,8 +2194,8 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
             }
             tok = launch_begin(p0, kclass(p0, "wave_corr_fold_" + std::to_string(R.len)), bytes,
                                flops);
-            e = launch_corr_fold(R.len, a, R, follow, st);
-            follow = true;
+            e = launch_corr_fold(R.len, a, R, first, st);
+            first = false;
             launch_end(p0, tok);
             if (e != cudaSuccess)
                 return fail_all(e, "corr_fold_kernel");
@@ -2202,7 +2203,7 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
     }
     if (nsets) {
         tok = launch_begin(p0, kclass(p0, "wave_corr_multi"), mbytes, mflops);
-        e = launch_corr_multi(M.P, n, sets, rows, nsets, follow, st);
+        e = launch_corr_multi(M.P, n, sets, rows, nsets, first, st);
         launch_end(p0, tok);
         if (e != cudaSuccess)
             return fail_all(e, "corr_multi_kernel");
