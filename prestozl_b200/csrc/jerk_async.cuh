@@ -76,14 +76,16 @@ inline cudaError_t smem_attrs(K kernel, bool carveout)
 }
 
 // Launches a kernel that may start while the one before it in the stream runs:
-// its CTAs take the SMs that the other's last CTAs leave idle, and
-// the launch itself costs no gap.  The kernel before calls let_follow, so that
-// this one starts once all of the other's CTAs have; without the call, when
-// they have ended.  wait_before returns when the kernel before has ended and
-// its writes can be read.  A kernel that needs those calls wait_before first thing;
-// one that does not calls it last, so that whatever comes after it finds both
+// its CTAs take the SMs that the other's last CTAs leave idle, and the launch
+// itself costs no gap.  The kernel before calls let_follow, so that this one
+// starts once all of the other's CTAs have; without the call, when they have
+// ended.  wait_before returns when the kernel before has ended and its writes
+// can be read.  A kernel that needs those calls wait_before first thing; one
+// that does not calls it last, so that whatever comes after it finds both
 // complete.  A kernel that waits first calls let_follow only after: the one
-// that follows may count on all that came before.
+// that follows may count on all that came before.  What the kernel before wrote
+// is not read through __ldg or a const __restrict__ parameter: the compiler may
+// move such a read to before the wait.
 template <class... Par, class... Arg>
 inline cudaError_t launch_follow(void (*kernel)(Par...), dim3 grid, unsigned block, size_t smem,
                                  cudaStream_t st, Arg &&...args)
@@ -98,7 +100,9 @@ inline cudaError_t launch_follow(void (*kernel)(Par...), dim3 grid, unsigned blo
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Arg>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Arg>(args)...);
+    const cudaError_t last = cudaGetLastError();  // as after <<<>>>: read and cleared
+    return e != cudaSuccess ? e : last;
 }
 
 __device__ __forceinline__ void let_follow()

@@ -40,3 +40,29 @@ def test_overlapped_launches_equal_serial(zmax, wmax, numharm, batch, rsteps):
             assert np.array_equal(got[1].view(np.uint32), want[1].view(np.uint32))
         plan.close()
     bank.close()
+
+
+def test_series_back_to_back_equal_alone():
+    """Series of several lengths whitened and zapped one right after the other:
+    each as with the device idle before every call."""
+    torch = pytest.importorskip("torch")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    series = [torch.randn(n, generator=g, device="cuda") for n in (32768, 98304, 786432, 32768)]
+    lo = np.array([0.2, 0.5, 0.5001]) * 16384
+
+    def one(ts, idle):
+        if idle:
+            torch.cuda.synchronize()
+        out = jerk.spectrum_from_timeseries(ts)
+        if idle:
+            torch.cuda.synchronize()
+        return jerk.zap_birdies(out, ts.numel(), lo, lo + 3.0)
+
+    alone = [one(ts, True).clone() for ts in series]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        got = [one(ts, False) for ts in series]
+        for a, b in zip(alone, got):
+            assert torch.equal(torch.view_as_real(a).view(torch.int32),
+                               torch.view_as_real(b).view(torch.int32))
