@@ -818,9 +818,11 @@ struct jerk_plan {
     StepDev *d_steps = nullptr;
     uint16_t *d_zinds = nullptr;
     int *d_wind = nullptr;
-    float2 *d_prepped = nullptr;
+    // prepared rows and row indices of a batch, and of the next, which is
+    // prepared while this one is correlated (null: not allocated, in turn)
+    float2 *d_prepped[2] = {};
     float *d_planes = nullptr;
-    uint16_t *d_rinds = nullptr;
+    uint16_t *d_rinds[2] = {};
     float2 *d_spec = nullptr;
     long long spec_cap = 0;
     unsigned long long *d_hit_keys = nullptr;
@@ -835,6 +837,8 @@ struct jerk_plan {
         SearchDev a{};
         long long first = 0, count = 0, next = 0, nbatch = 0, ndone = 0;
         bool all_enqueued = false;
+        int buf = 0;            // the buffers of the batch at next
+        bool prepared = false;  // its rows are prepared there
         bool capturing = false;  // being recorded into a graph: no host-side event queries
         int error = 0;  // first enqueue failure (the pass is then abandoned)
     } pass;
@@ -980,9 +984,11 @@ static void plan_free_device(jerk_plan *p)
     cudaFree(p->d_steps);
     cudaFree(p->d_zinds);
     cudaFree(p->d_wind);
-    cudaFree(p->d_prepped);
+    for (int i = 0; i < 2; i++) {
+        cudaFree(p->d_prepped[i]);
+        cudaFree(p->d_rinds[i]);
+    }
     cudaFree(p->d_planes);
-    cudaFree(p->d_rinds);
     cudaFree(p->d_spec);
     cudaFree(p->d_hit_keys);
     cudaFree(p->d_hit_pows);
@@ -1584,14 +1590,22 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
     JERK_CUDA_B(cudaMalloc(&p->d_wind, sizeof(int) * wind.size()));
     JERK_CUDA_B(cudaMemcpyAsync(p->d_wind, wind.data(), sizeof(int) * wind.size(),
                                 cudaMemcpyHostToDevice, p->stream));
-    JERK_CUDA_B(cudaMalloc(&p->d_prepped, sizeof(float2) * p->prepped_f2));
-    // one volume / rinds buffer: every launch of a pass runs on the plan's
+    const size_t rinds_bytes = sizeof(uint16_t) * (size_t)p->batch * nsubs * obs->corr_uselen;
+    JERK_CUDA_B(cudaMalloc(&p->d_prepped[0], sizeof(float2) * p->prepped_f2));
+    JERK_CUDA_B(cudaMalloc(&p->d_rinds[0], rinds_bytes));
+    // one volume buffer: every launch of a pass runs on the plan's
     // stream, so batch k + 1's correlation starts after batch k's harmonic
     // sum has read the volumes (running the two side by side on two streams
     // measured slower than back to back: their CTAs then share SMs)
     JERK_CUDA_B(cudaMalloc(&p->d_planes, sizeof(float) * p->plane_floats));
-    JERK_CUDA_B(cudaMalloc(&p->d_rinds, sizeof(uint16_t) * (size_t)p->batch * nsubs *
-                                            obs->corr_uselen));
+    // the next batch's buffers are the last to be allocated and may be missing
+    if (cudaMalloc(&p->d_prepped[1], sizeof(float2) * p->prepped_f2) != cudaSuccess ||
+        cudaMalloc(&p->d_rinds[1], rinds_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(p->d_prepped[1]);
+        p->d_prepped[1] = nullptr;
+        p->d_rinds[1] = nullptr;
+    }
     if (p->harm_mode >= 2 && p->harm_mode <= 4) {
         const int rc = build_harm_tma(p, p->harm_mode >= 3);
         if (rc != JERK_OK)
@@ -1671,9 +1685,9 @@ static SearchDev make_args(const jerk_plan *p, const float2 *spec)
     a.rowsets = p->d_rowsets;
     a.zinds = p->d_zinds;
     a.wind = p->d_wind;
-    a.prepped = p->d_prepped;
+    a.prepped = p->d_prepped[0];
     a.planes = p->d_planes;
-    a.rinds = p->d_rinds;
+    a.rinds = p->d_rinds[0];
     a.hit_keys = p->d_hit_keys;
     a.hit_pows = p->d_hit_pows;
     a.hit_count = p->d_hit_count;
@@ -1734,20 +1748,79 @@ static RowGroup row_group(const jerk_plan *p, const std::vector<int> &subs)
     return G;
 }
 
-static int run_volumes(jerk_plan *p, SearchDev &a)
+// Batch arguments: rsteps from k on (to the pass's end at most), in buffers buf.
+static void batch_args(const jerk_plan *p, long long k, int buf, SearchDev &a)
 {
-    {
-        double bytes = 0, flops = 0;
-        for (int s = 0; s < p->nsubs; s++) {
-            const int N = p->subs[s].fftlen;
-            bytes += (double)a.nb * (N / 2 * 8.0 + N / 2 * 8.0);
-            flops += (double)a.nb * fft_flops(N);
-        }
-        const int tok = launch_begin(p, kclass(p, "prep"), bytes, flops);
-        cudaError_t e = launch_prep(a, p->maxfft, p->prep_smem, p->stream);
-        launch_end(p, tok);
-        if (e != cudaSuccess)
-            return cuda_fail(e, "prep_kernel");
+    const jerk_plan::Pass &ps = p->pass;
+    a.first_rstep = k;
+    a.nb = (int)std::min<long long>(p->batch, ps.first + ps.count - k);
+    a.planes = p->d_planes;
+    a.prepped = p->d_prepped[buf];
+    a.rinds = p->d_rinds[buf];
+}
+
+// The batch at the pass's next rstep, and whether the one after it is to be
+// prepared beside it (into *ahead).
+static bool next_batch(jerk_plan *p, SearchDev *ahead)
+{
+    jerk_plan::Pass &ps = p->pass;
+    batch_args(p, ps.next, ps.buf, ps.a);
+    const long long after = ps.next + ps.a.nb;
+    if (!p->d_rinds[1] || after >= ps.first + ps.count)
+        return false;
+    *ahead = ps.a;
+    batch_args(p, after, ps.buf ^ 1, *ahead);
+    return true;
+}
+
+static void batch_enqueued(jerk_plan *p, bool ahead)
+{
+    jerk_plan::Pass &ps = p->pass;
+    ps.next += ps.a.nb;
+    ps.nbatch++;
+    ps.prepared = ahead;
+    if (ahead)
+        ps.buf ^= 1;
+}
+
+static void prep_work(const jerk_plan *p, const SearchDev &a, double *bytes, double *flops)
+{
+    for (int s = 0; s < p->nsubs; s++) {
+        const int N = p->subs[s].fftlen;
+        *bytes += (double)a.nb * (N / 2 * 8.0 + N / 2 * 8.0);
+        *flops += (double)a.nb * fft_flops(N);
+    }
+}
+
+static int run_prep(jerk_plan *p, const SearchDev &a)
+{
+    double bytes = 0, flops = 0;
+    prep_work(p, a, &bytes, &flops);
+    const int tok = launch_begin(p, kclass(p, "prep"), bytes, flops);
+    cudaError_t e = launch_prep(a, p->maxfft, p->prep_smem, p->stream);
+    launch_end(p, tok);
+    return e == cudaSuccess ? JERK_OK : cuda_fail(e, "prep_kernel");
+}
+
+// A batch's volumes (prepared: its rows are there already).  ahead, if not
+// null: the next batch's arguments, whose preparation runs beside this one's
+// correlation.  Preparation is a chain of latencies on a few CTAs: 16 us of a
+// 62-us batch at zmax 20, wmax 60, 8 harmonics; a pass takes 4.71 ms with it
+// in turn, 4.30 beside (zmax 100, 16 harmonics, 2^22 samples 14.07 and 13.68,
+// zmax 50, wmax 150 36.2 and 35.5).  Order: it waits for the last harmonic
+// sum, which reads the buffers it writes; the correlation starts once its CTAs
+// have, needing only what came before it.
+static int run_volumes(jerk_plan *p, const SearchDev &a, bool prepared, const SearchDev *ahead)
+{
+    if (!prepared) {
+        const int rc = run_prep(p, a);
+        if (rc != JERK_OK)
+            return rc;
+    }
+    if (ahead) {
+        const int rc = run_prep(p, *ahead);
+        if (rc != JERK_OK)
+            return rc;
     }
     cudaError_t e = cudaSuccess;
     for (auto &kv : p->groups) {
@@ -1774,7 +1847,7 @@ static int run_volumes(jerk_plan *p, SearchDev &a)
     int sets[kMaxRowSets][2], nsets = 0;
     const FoldRows *rows[kMaxRowSets];
     double mbytes = 0, mflops = 0;
-    bool first = p->groups.empty();  // the next launch follows the prepared rows' own
+    bool first = p->groups.empty() && !ahead;  // the next launch needs the one before
     for (size_t i = 0; i < p->rowsets.size(); i++) {
         const FoldRows &R = p->rowsets[i];
         if (!p->own_launch[i]) {
@@ -1874,12 +1947,9 @@ static int pass_enqueue_one(jerk_plan *p)
 {
     jerk_plan::Pass &ps = p->pass;
     SearchDev &a = ps.a;
-    const long long k = ps.next;
-    a.first_rstep = k;
-    a.nb = (int)std::min<long long>(p->batch, ps.first + ps.count - k);
-    a.planes = p->d_planes;
-    a.rinds = p->d_rinds;
-    int rc = run_volumes(p, a);
+    SearchDev after;
+    const bool ahead = next_batch(p, &after);
+    int rc = run_volumes(p, a, ps.prepared, ahead ? &after : nullptr);
     if (rc != JERK_OK)
         return rc;
     double bytes = 0, flops = 0;
@@ -1891,8 +1961,7 @@ static int pass_enqueue_one(jerk_plan *p)
         return cuda_fail(e, "harmsum_kernel");
     if (!ps.capturing)
         JERK_CUDA(cudaEventRecord(p->ev_batch[ps.nbatch % jerk_plan::kRing], p->stream));
-    ps.next += a.nb;
-    ps.nbatch++;
+    batch_enqueued(p, ahead);
     return JERK_OK;
 }
 
@@ -2128,21 +2197,24 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
     const int n = (int)W.size();
     int maxfft = 0;
     size_t prep_smem = 0;
-    double pbytes = 0, pflops = 0;
-    for (jerk_plan *p : W) {
-        jerk_plan::Pass &ps = p->pass;
-        SearchDev &a = ps.a;
-        a.first_rstep = ps.next;
-        a.nb = (int)std::min<long long>(p->batch, ps.first + ps.count - ps.next);
-        a.planes = p->d_planes;
-        a.rinds = p->d_rinds;
+    // rows to prepare before this wave's correlation, and beside it
+    GroupLaunch M{}, now{}, next{};
+    bool ahead[kMaxGroupPlans];
+    double work[2][2] = {};  // bytes, operations of either
+    for (int i = 0; i < n; i++) {
+        jerk_plan *p = W[i];
+        ahead[i] = next_batch(p, &next.P[next.n]);
+        M.P[M.n++] = p->pass.a;
+        if (!p->pass.prepared) {
+            prep_work(p, p->pass.a, &work[0][0], &work[0][1]);
+            now.P[now.n++] = p->pass.a;
+        }
+        if (ahead[i]) {
+            prep_work(p, next.P[next.n], &work[1][0], &work[1][1]);
+            next.n++;
+        }
         maxfft = std::max(maxfft, p->maxfft);
         prep_smem = std::max(prep_smem, p->prep_smem);
-        for (int s = 0; s < p->nsubs; s++) {
-            const int N = p->subs[s].fftlen;
-            pbytes += (double)a.nb * (N / 2 * 8.0 + N / 2 * 8.0);
-            pflops += (double)a.nb * fft_flops(N);
-        }
     }
     auto fail_all = [&](cudaError_t e, const char *what) {
         const int rc = cuda_fail(e, what);
@@ -2150,15 +2222,18 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
             p->pass.error = rc;
         return rc;
     };
-    GroupLaunch M{};
-    M.n = n;
-    for (int i = 0; i < n; i++)
-        M.P[i] = W[i]->pass.a;
-    int tok = launch_begin(p0, kclass(p0, "wave_prep"), pbytes, pflops);
-    cudaError_t e = launch_prep_group(M, maxfft, prep_smem, st);
-    launch_end(p0, tok);
-    if (e != cudaSuccess)
-        return fail_all(e, "prep_group_kernel");
+    cudaError_t e = cudaSuccess;
+    int tok = 0;
+    for (const GroupLaunch *G : {&now, &next}) {
+        if (!G->n)
+            continue;
+        tok = launch_begin(p0, kclass(p0, "wave_prep"), work[G == &next][0],
+                           work[G == &next][1]);
+        e = launch_prep_group(*G, maxfft, prep_smem, st);
+        launch_end(p0, tok);
+        if (e != cudaSuccess)
+            return fail_all(e, "prep_group_kernel");
+    }
 
     // correlation: the row sets that fill the GPU twice over by themselves
     // (and the long unfolded lengths) in their plan's own launches, all the
@@ -2166,7 +2241,7 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
     int sets[kMaxGroupPlans * kMaxRowSets][2], nsets = 0;
     const FoldRows *rows[kMaxGroupPlans * kMaxRowSets];
     double mbytes = 0, mflops = 0;
-    bool first = true;  // the next launch follows the prepared rows' own
+    bool first = !next.n;  // the next launch needs the one before
     for (int i = 0; i < n; i++) {
         jerk_plan *p = W[i];
         const SearchDev &a = p->pass.a;
@@ -2250,11 +2325,11 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
             return fail_all(e, "harmsum_group_kernel");
     }
 
-    for (jerk_plan *p : W) {
+    for (int i = 0; i < n; i++) {
+        jerk_plan *p = W[i];
         jerk_plan::Pass &ps = p->pass;
         JERK_CUDA(cudaEventRecord(p->ev_batch[ps.nbatch % jerk_plan::kRing], st));
-        ps.next += ps.a.nb;
-        ps.nbatch++;
+        batch_enqueued(p, ahead[i]);
         if (ps.next >= ps.first + ps.count) {
             const int rc = pass_finish_enqueue(p);
             if (rc != JERK_OK)
@@ -2557,8 +2632,9 @@ extern "C" long long jerk_plan_device_bytes(const jerk_plan *p)
     if (!p)
         return 0;
     return (long long)(sizeof(float) * p->plane_floats +
-                       sizeof(uint16_t) * (size_t)p->batch * p->nsubs * p->obs.corr_uselen +
-                       sizeof(float2) * p->prepped_f2 +
+                       (p->d_rinds[1] ? 2 : 1) *
+                           (sizeof(uint16_t) * (size_t)p->batch * p->nsubs * p->obs.corr_uselen +
+                            sizeof(float2) * p->prepped_f2) +
                        (sizeof(unsigned long long) + sizeof(float)) * p->max_hits +
                        sizeof(StepDev) * p->hsteps.size() + sizeof(float2) * p->spec_cap +
                        sizeof(float2) * p->fold_f2 +
@@ -2590,7 +2666,7 @@ extern "C" int jerk_debug_volume(jerk_plan *p, const void *spectrum, int spectru
     SearchDev a = make_args(p, spec);
     a.first_rstep = rstep;
     a.nb = 1;
-    rc = run_volumes(p, a);
+    rc = run_volumes(p, a, false, nullptr);
     if (rc != JERK_OK)
         return rc;
     JERK_CUDA(cudaStreamSynchronize(p->stream));

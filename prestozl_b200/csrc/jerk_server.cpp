@@ -154,8 +154,9 @@ static long long plan_footprint(const Geometry &g, int batch)
         folded += jerk::fold_bytes(s, (int)stride);
     }
     const long long rsteps = (long long)((g.obs.highestbin - g.obs.rlo) / (g.obs.corr_uselen / 2)) + 1;
-    return vol * batch + chunks * batch +
-           2LL * batch * (long long)g.subs.size() * g.obs.corr_uselen +
+    // (the chunks and row indices of two batches)
+    return vol * batch + 2 * chunks * batch +
+           4LL * batch * (long long)g.subs.size() * g.obs.corr_uselen +
            (long long)(1 << 22) * 12 + rsteps * (long long)g.subs.size() * 24 +
            g.obs.numbins * 8 + folded + (64LL << 20);
 }
