@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(FftPlan<M>::T)
     pw_response_kernel(const PolishRow *__restrict__ rows, const int *__restrict__ list,
                        const float2 *__restrict__ tw, float2 *__restrict__ bank)
 {
+    let_follow();
     constexpr int T = FftPlan<M>::T;
     extern __shared__ float2 pw_smem[];
     float2 *buf = pw_smem;
@@ -222,6 +223,7 @@ __global__ void __launch_bounds__(FftPlan<M>::T)
         row[placed(k, numkern, R.fftlen)] =
             make_float2((float)(hx + 0.5 * gy), (float)(hy - 0.5 * gx));
     }
+    wait_before();
 }
 
 // ---------------------------------------------------------------------------
@@ -239,8 +241,7 @@ struct PolishTw {
 // spread_no_pad (src/corr_prep.c:37-74) by 8, then the forward FFT
 template <int N>
 __device__ __forceinline__ void pd_data(const PolishHarm &H, const float2 *tw,
-                                        const float2 *__restrict__ windows,
-                                        float2 *__restrict__ dfft, float2 *buf)
+                                        const float2 *windows, float2 *dfft, float2 *buf)
 {
     constexpr int T = FftPlan<N>::T;
     const float2 *src = windows + H.win;
@@ -256,8 +257,10 @@ __device__ __forceinline__ void pd_data(const PolishHarm &H, const float2 *tw,
 
 __global__ void __launch_bounds__(512)
     pd_data_kernel(const PolishHarm *__restrict__ harms, const PolishTw W,
-                   const float2 *__restrict__ windows, float2 *__restrict__ dfft)
+                   const float2 *windows, float2 *dfft)
 {
+    wait_before();
+    let_follow();
     extern __shared__ float2 p_smem[];
     const PolishHarm &H = harms[blockIdx.x];
     switch (H.fftlen) {
@@ -273,10 +276,9 @@ __global__ void __launch_bounds__(512)
 // (src/correlations.c:3-55, CORR) and the chop of corr_complex: amplitude i of
 // the volume is y[khw * 8 + i]
 template <int N>
-__device__ __forceinline__ void pc_corr(const PolishHarm &H, const float2 *__restrict__ kresp,
-                                        long long rowi, const float2 *tw,
-                                        const float2 *__restrict__ dfft, float *__restrict__ terms,
-                                        float *__restrict__ tails, float2 *buf, float *pw)
+__device__ __forceinline__ void pc_corr(const PolishHarm &H, const float2 *kresp,
+                                        long long rowi, const float2 *tw, const float2 *dfft,
+                                        float *terms, float *tails, float2 *buf, float *pw)
 {
     constexpr int T = FftPlan<N>::T;
     float2 *krow = buf + fft_buf_len<N>();
@@ -314,10 +316,11 @@ __device__ __forceinline__ void pc_corr(const PolishHarm &H, const float2 *__res
 
 __global__ void __launch_bounds__(512)
     pc_corr_kernel(const PolishRow *__restrict__ rows, const PolishHarm *__restrict__ harms,
-                   const PolishTw W, const float2 *__restrict__ bank,
-                   const float2 *__restrict__ dfft, float *__restrict__ terms,
-                   float *__restrict__ tails)
+                   const PolishTw W, const float2 *bank, const float2 *dfft, float *terms,
+                   float *tails)
 {
+    wait_before();
+    let_follow();
     extern __shared__ float2 p_smem[];
     __shared__ float pw[kWin];
     const long long rowi = blockIdx.x;
@@ -340,10 +343,10 @@ __global__ void __launch_bounds__(512)
 // *best, which starts at 0.  (One CTA for all 6936 sums took 66 us.)
 constexpr int kArgThreads = 128;
 __global__ void __launch_bounds__(kArgThreads)
-    ps_argmax_kernel(const float *__restrict__ terms, const float *__restrict__ tails,
-                     const PolishHarm *__restrict__ harms, int numharm,
-                     unsigned long long *__restrict__ best)
+    ps_argmax_kernel(const float *terms, const float *tails, const PolishHarm *__restrict__ harms,
+                     int numharm, unsigned long long *best)
 {
+    wait_before();
     const int c = blockIdx.x * kArgThreads + threadIdx.x;
     unsigned long long key = 0;
     if (c < kCells * kNumR) {
@@ -457,8 +460,8 @@ template <int M> struct PW {
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess)
             return e;
-        pw_response_kernel<M><<<count, FftPlan<M>::T, smem, st>>>(rows, list, tw, bank);
-        return cudaGetLastError();
+        return launch_follow(pw_response_kernel<M>, count, FftPlan<M>::T, smem, st, rows, list, tw,
+                             bank);
     }
 };
 long long next2(long long x)
@@ -477,8 +480,7 @@ struct InterpPoint {
 };
 
 __global__ void interp_w_kernel(const InterpPoint *__restrict__ pts, const int *__restrict__ list,
-                                const PolishTw W, const float2 *__restrict__ windows,
-                                float2 *__restrict__ ans);
+                                const PolishTw W, const float2 *windows, float2 *ans);
 
 // One run of spectrum values read from a spectrum held on the device:
 // count values from index src (zero outside [0, numdata)) to dst[off] with
@@ -495,6 +497,7 @@ gather_windows_kernel(const float2 *__restrict__ spec, long long numdata,
                       const WinSeg *__restrict__ segs, float2 *__restrict__ win,
                       float2 *__restrict__ ans)
 {
+    let_follow();
     const WinSeg s = segs[blockIdx.x];
     float2 *dst = (s.to_ans ? ans : win) + s.off;
     for (int i = threadIdx.x; i < s.count; i += kGatherThreads) {
@@ -858,6 +861,8 @@ extern "C" int jerk_polish_rzw(jerk_polisher *p, const void *spectrum, long long
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(dev ? (void *)p->d_segs : (void *)p->windows, hw, b_win,
                             cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(p->d_best, 0, sizeof(unsigned long long), st);
     if (e == cudaSuccess && dev) {
         gather_windows_kernel<<<numharm, kGatherThreads, 0, st>>>(data, numdata, p->d_segs,
                                                                   p->windows, nullptr);
@@ -866,39 +871,37 @@ extern "C" int jerk_polish_rzw(jerk_polisher *p, const void *spectrum, long long
     if (e != cudaSuccess)
         return p_cuda(e, "jerk_polish_rzw: upload");
 
-    // ---- device: responses, kernel FFTs, data FFTs, correlations, sum and argmax
-    if (nzr > 0) {
-        pzr_response_kernel<<<nzr, kRespThreads, 0, st>>>(p->d_rows, p->d_lists, p->bank);
-        e = cudaGetLastError();
-    }
-    for (int s = 0; s < kNumSizes && e == cudaSuccess; s++)
-        if (mcount[s])
-            e = p_dispatch<PW>(kSizes[s], (const PolishRow *)p->d_rows,
-                               (const int *)p->d_lists + mfirst[s], mcount[s],
-                               (const float2 *)(p->tw + p->twoff[s]), p->bank, maxkern[s], st);
-    if (e == cudaSuccess) {
+    // ---- device: data FFTs, responses, kernel FFTs and correlations, sum and
+    // argmax.  The responses need only the uploads: the launches of either
+    // length run beside one another and the data's (in turn, each with its
+    // last wave, a 16-harmonic candidate took 465 us, 437 now).
+    {
         int N = 0;
         for (const PolishHarm &h : H)
             N = std::max(N, h.fftlen);
         const PolishTw W = p->tables();
         const int threads = N / 16 < 64 ? 64 : N / 16;  // the widest plan's (512 and less: 64)
         const size_t b_buf = sizeof(float2) * (size_t)fft_buf_len_rt(N);
-        e = cudaMemsetAsync(p->d_best, 0, sizeof(unsigned long long), st);
-        if (e == cudaSuccess) {
-            pd_data_kernel<<<numharm, threads, b_buf, st>>>(p->d_harms, W, p->windows, p->dfft);
+        if (e == cudaSuccess)
+            e = launch_follow(pd_data_kernel, numharm, threads, b_buf, st, p->d_harms, W, p->windows,
+                              p->dfft);
+        if (e == cudaSuccess && nzr > 0) {
+            pzr_response_kernel<<<nzr, kRespThreads, 0, st>>>(p->d_rows, p->d_lists, p->bank);
             e = cudaGetLastError();
         }
-        if (e == cudaSuccess) {
-            pc_corr_kernel<<<(unsigned)nrows, threads, b_buf + sizeof(float2) * N, st>>>(
-                p->d_rows, p->d_harms, W, p->bank, p->dfft, p->terms, p->tails);
-            e = cudaGetLastError();
-        }
+        for (int s = 0; s < kNumSizes && e == cudaSuccess; s++)
+            if (mcount[s])
+                e = p_dispatch<PW>(kSizes[s], (const PolishRow *)p->d_rows,
+                                   (const int *)p->d_lists + mfirst[s], mcount[s],
+                                   (const float2 *)(p->tw + p->twoff[s]), p->bank, maxkern[s], st);
+        if (e == cudaSuccess)
+            e = launch_follow(pc_corr_kernel, (unsigned)nrows, threads,
+                              b_buf + sizeof(float2) * N, st, p->d_rows, p->d_harms, W, p->bank,
+                              p->dfft, p->terms, p->tails);
     }
-    if (e == cudaSuccess) {
-        ps_argmax_kernel<<<(kCells * kNumR + kArgThreads - 1) / kArgThreads, kArgThreads, 0, st>>>(
-            p->terms, p->tails, p->d_harms, numharm, p->d_best);
-        e = cudaGetLastError();
-    }
+    if (e == cudaSuccess)
+        e = launch_follow(ps_argmax_kernel, (kCells * kNumR + kArgThreads - 1) / kArgThreads,
+                          kArgThreads, 0, st, p->terms, p->tails, p->d_harms, numharm, p->d_best);
     unsigned long long key = 0;
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(&key, p->d_best, sizeof(key), cudaMemcpyDeviceToHost, st);
@@ -972,8 +975,10 @@ __device__ __forceinline__ void corr_acc(float2 d, float re, float im, double &a
 
 __global__ void __launch_bounds__(kInterpThreads)
     interp_zr_kernel(const InterpPoint *__restrict__ pts, const int *__restrict__ list,
-                     const float2 *__restrict__ windows, float2 *__restrict__ ans)
+                     const float2 *windows, float2 *ans)
 {
+    wait_before();
+    let_follow();
     const int pi = list[blockIdx.x];
     const InterpPoint P = pts[pi];
     const float2 *d = windows + P.win;
@@ -1050,8 +1055,7 @@ __global__ void __launch_bounds__(kInterpThreads)
 // drops into shared memory; then the correlation with the data window.
 template <int M>
 __device__ __forceinline__ void interp_w(const InterpPoint &P, int pi, const float2 *tw,
-                                         const float2 *__restrict__ windows,
-                                         float2 *__restrict__ ans, float2 *buf)
+                                         const float2 *windows, float2 *ans, float2 *buf)
 {
     constexpr int T = FftPlan<M>::T;
     float2 *win = buf + fft_buf_len<M>();
@@ -1107,8 +1111,9 @@ __device__ __forceinline__ void interp_w(const InterpPoint &P, int pi, const flo
 // length took 32 us a call, three calls a candidate.
 __global__ void __launch_bounds__(512)
     interp_w_kernel(const InterpPoint *__restrict__ pts, const int *__restrict__ list,
-                    const PolishTw W, const float2 *__restrict__ windows, float2 *__restrict__ ans)
+                    const PolishTw W, const float2 *windows, float2 *ans)
 {
+    wait_before();
     extern __shared__ float2 p_smem[];
     const int pi = list[blockIdx.x];
     const InterpPoint &P = pts[pi];
@@ -1250,9 +1255,8 @@ int interp_points(jerk_polisher *p, const float2 *data, long long numdata, int n
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && !zr.empty()) {
-        interp_zr_kernel<<<(int)zr.size(), kInterpThreads, 0, st>>>(d_pts, p->d_lists, p->windows,
-                                                                     p->dfft);
-        e = cudaGetLastError();
+        e = launch_follow(interp_zr_kernel, (int)zr.size(), kInterpThreads, 0, st, d_pts, p->d_lists,
+                          p->windows, p->dfft);
     }
     const int nw = (int)(lists.size() - zr.size());
     if (e == cudaSuccess && nw) {
@@ -1262,9 +1266,8 @@ int interp_points(jerk_polisher *p, const float2 *data, long long numdata, int n
                 M = kSizes[s];
                 smem = std::max(smem, fft_buf_len_rt(M) + maxkern[s] + 1);
             }
-        interp_w_kernel<<<nw, M / 16 < 64 ? 64 : M / 16, sizeof(float2) * smem, st>>>(
-            d_pts, p->d_lists + zr.size(), p->tables(), p->windows, p->dfft);
-        e = cudaGetLastError();
+        e = launch_follow(interp_w_kernel, nw, M / 16 < 64 ? 64 : M / 16, sizeof(float2) * smem, st,
+                          d_pts, p->d_lists + zr.size(), p->tables(), p->windows, p->dfft);
     }
     float2 *hans = (float2 *)(hs + o_ans);
     if (e == cudaSuccess)

@@ -66,3 +66,27 @@ def test_series_back_to_back_equal_alone():
         for a, b in zip(alone, got):
             assert torch.equal(torch.view_as_real(a).view(torch.int32),
                                torch.view_as_real(b).view(torch.int32))
+
+
+def test_polishing_in_sequence_equals_fresh():
+    """Candidates of one, few and many harmonics, with and without w, polished
+    one after another by one polisher: each as by a polisher of its own, from a
+    spectrum on the device and on the host."""
+    torch = pytest.importorskip("torch")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(9)
+    spec = torch.view_as_complex(torch.randn((1 << 20, 2), generator=g, device="cuda"))
+    host = spec.cpu().numpy()
+    cands = [(1, 40000.25, 3.0, 0.0), (16, 30123.5, 9.5, -14.0), (4, 90000.0, -40.0, 60.0),
+             (8, 20011.75, 0.0, 0.0), (16, 30123.5, 9.5, -14.0)]
+    shared = jerk.Polisher()
+    for numharm, r, z, w in cands:
+        fresh = jerk.Polisher()
+        want = fresh.optimize(host, numharm, r, z, w)
+        fresh.close()
+        for src in (spec, host):
+            got = shared.optimize(src, numharm, r, z, w)
+            assert tuple(got[0]) == tuple(want[0])
+            assert np.array_equal(np.asarray(got[1]["pow"]), np.asarray(want[1]["pow"]))
+            assert np.array_equal(np.asarray(got[2]), np.asarray(want[2]))
+    shared.close()
