@@ -546,20 +546,30 @@ struct RingOps {
         using R = Ring<S, QMax>;
         RingGroup G;
         G.M = M;
-        // CTAs in proportion to the plans' rows
+        // CTAs in proportion to the plans' tile rows, what is left over to
+        // whichever has the most rows per CTA
         const int wave = sm_count() * R::Occ;
-        double rows = 0;
-        auto rows_of = [](const SearchDev &P) {
-            return (double)P.nb * P.numw0 * P.numz0 * P.corr_uselen;
-        };
+        double work[kMaxGroupPlans], all = 0.0;
+        int share[kMaxGroupPlans], dealt = 0;
+        for (int i = 0; i < M.n; i++) {
+            const SearchDev &P = M.P[i];
+            work[i] = (double)P.nb * P.numw0 * P.numz0 * ((P.corr_uselen + R::C - 1) / R::C);
+            all += work[i];
+        }
         for (int i = 0; i < M.n; i++)
-            rows += rows_of(M.P[i]);
+            dealt += share[i] = std::max(1, (int)(work[i] / all * wave));
+        for (; dealt < wave; dealt++) {
+            int most = 0;
+            for (int i = 1; i < M.n; i++)
+                if (work[i] * share[most] > work[most] * share[i])
+                    most = i;
+            share[most]++;
+        }
         int x = 0;
         for (int i = 0; i < M.n; i++) {
-            const int share = std::max(1, (int)(rows_of(M.P[i]) / rows * wave));
-            G.W[i] = ring_plan(M.P[i], R::C, share);
+            G.W[i] = ring_plan(M.P[i], R::C, share[i]);
             G.M.cta0[i] = x;
-            x += std::min(G.W[i].items, share);
+            x += std::min(G.W[i].items, share[i]);
         }
         G.M.cta0[M.n] = x;
         if (R::Early)

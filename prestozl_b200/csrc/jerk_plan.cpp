@@ -2291,12 +2291,17 @@ static int enqueue_wave(const std::vector<jerk_plan *> &W)
     for (int i = 0; i < n; i++) {
         jerk_plan *p = W[i];
         const SearchDev &a = p->pass.a;
-        // (the ring splits its rows evenly over the resident CTAs, alone or
-        // merged; the gather form merges what does not fill two waves)
+        // The gather form merges what does not fill two waves.  The ring splits
+        // its rows over the resident CTAs, alone or merged: merged, small plans
+        // share one start and end (three of 0.5 GB volumes, 66.6 -> 64.7 ms a
+        // search); beside a large plan they get one CTA or two, whose rounding is
+        // then the whole launch's time (two plans of 2.6 GB and two of 0.1 GB:
+        // 399 ms of sums, 202 so), so a large one is launched by itself.
         const bool ring = use_ring(p, a);
         const long long ctas = (long long)((a.corr_uselen + 127) / 128) * a.numw0 * a.nb;
-        if (ring || ((p->harm_mode <= 1 || p->harm_mode == kHarmRing) &&
-                     ctas < 2 * harmsum_wave_ctas(a.nstages))) {
+        if (ring ? 4.0 * (double)p->plane_floats / p->batch * a.nb < 1e9
+                 : (p->harm_mode <= 1 || p->harm_mode == kHarmRing) &&
+                       ctas < 2 * harmsum_wave_ctas(a.nstages)) {
             byS[{p->obs.numharmstages, ring}].push_back(i);
             continue;
         }
