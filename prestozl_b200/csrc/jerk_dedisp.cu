@@ -400,13 +400,16 @@ void launch_tiling(const int *off, int worklen, int numdms, int nsub, int sms, i
                    int *tile)
 {
     double best = 0.0;
-    for (int t : {512, 256, 128})
-        for (int gsz : {64, 32, 16, 8, 4, 2, 1}) {
-            const long long ngroups = (numdms + gsz - 1) / gsz;
-            double staged = 0.0;
-            if (ngroups > 65535 || dd_tables(off, numdms, nsub, gsz, t, nullptr, nullptr, false,
-                                             &staged) > kSmemTwo)
+    for (int gsz : {64, 32, 16, 8, 4, 2, 1}) {
+        const long long ngroups = (numdms + gsz - 1) / gsz;
+        if (ngroups > 65535)
+            continue;
+        double spans = 0.0;  // the windows' words beyond their tile
+        const size_t bytes = dd_tables(off, numdms, nsub, gsz, 0, nullptr, nullptr, false, &spans);
+        for (int t : {512, 256, 128}) {
+            if (bytes + sizeof(float) * (size_t)((nsub * (long long)t + 3) & ~3LL) > kSmemTwo)
                 continue;
+            const double staged = spans + (double)ngroups * nsub * t;
             const double adds = (double)numdms * t * nsub * (t >= 256 ? 1.0 : 1.5);
             const double ctas = (double)ngroups * ((worklen + t - 1) / t);
             const double cost = (14.0 * staged + adds) / (double)ngroups *
@@ -417,6 +420,7 @@ void launch_tiling(const int *off, int worklen, int numdms, int nsub, int sms, i
                 *tile = t;
             }
         }
+    }
 }
 
 // The offsets table on the host: copied from device memory (as getDedisp
