@@ -49,19 +49,19 @@ WORKLOAD = "jerk search, 2^25-sample spectra, -zmax 200 -wmax 300 -numharm 16 -s
 # lanes x 2 flops per FMA x 1965 MHz); the correlation kernels are bound by it.
 FP32_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12
 
-# DRAM traffic of one fftlen-2048 correlation launch (corr_fold_kernel) at 16
-# rsteps per batch, from an ncu capture (dram__bytes_read.sum /
-# dram__bytes_write.sum) of
-#   python bench.py --rsteps 128 --steps 1 --warmup 1 --no-cpu-baseline --no-ref-gpu
-#                   --e2e-steps 1 --batch 16 --no-extras
-# The read side (folded kernel rows + data rows) is paid once per launch; the
-# write side (the volumes) grows with the rsteps per batch.
-CORR2048_TRAFFIC = {"read": 491.168256e6, "write": 2241.328e6, "batch": 16}
+# DRAM traffic of one correlation launch over the rows of half length 1024
+# (corr_fold_kernel<1024>, the dominant launch) at 16 rsteps per batch, from an
+# ncu capture (dram__bytes.sum.per_second over gpu__time_duration.sum) of a
+# 2^24-sample spectrum at the paper geometry.  The read side, the folded kernel
+# rows (14,572 rows of 2 x 1024 complex), is paid once per launch; the rest, the
+# volumes, grows with the rsteps per batch.
+CORR_TRAFFIC = {"kernel": "corr_fold_1024", "total": 1451e6, "rows": 14572 * 2 * 1024 * 8.0,
+                "batch": 16}
 
 
-def corr2048_traffic(batch: int) -> float:
-    t = CORR2048_TRAFFIC
-    return t["read"] + t["write"] * batch / t["batch"]
+def corr_traffic(batch: int) -> float:
+    t = CORR_TRAFFIC
+    return t["rows"] + (t["total"] - t["rows"]) * batch / t["batch"]
 
 
 def peaks():
@@ -323,8 +323,8 @@ def input_prep_leg(device, reps: int = 5):
     ms = e0.elapsed_time(e1) / reps
     alg = 8.0 * N_SAMPLES  # the series read once, the spectrum written once
     return {"samples": N_SAMPLES, "ms_per_series": ms, "algorithmic_bytes": alg,
-            "achieved_gbs": alg / ms / 1e6, "kernels": "rf_twiddle x2, rf_column, rf_row, "
-            "rf_post, dr_level, dr_scale", "launches": 7,
+            "achieved_gbs": alg / ms / 1e6, "kernels": "rf_twiddle, rf_column, rf_row, "
+            "rf_post, dr_level, dr_scale", "launches": 6,
             "note": "three FFT passes and two red-noise passes move about 5x the algorithmic "
                     "bytes; one-off per series (about 0.02 % of its search)"}
 
@@ -381,7 +381,7 @@ def dedisp_leg(device, reps: int = 5, worklen: int = 65536, nsub: int = 64,
            "dedisp_ms": ms_dd, "dedisp_gadds_per_s": adds / ms_dd / 1e6,
            "dedisp_algorithmic_bytes": dd_bytes, "dedisp_achieved_gbs": dd_bytes / ms_dd / 1e6,
            "downsample_ms": ms_ds, "downsample_achieved_gbs": ds_bytes / ms_ds / 1e6,
-           "bound": "dedisp: shared-memory load wavefronts (about 1.03 per 32 adds in the "
+           "bound": "dedisp: shared-memory load wavefronts (one per 32 adds in the "
                     "sums, plus the window staging); downsample: HBM"}
     try:
         from oracle import bindings as ob
@@ -429,10 +429,9 @@ def polish_leg(spec_np, cands, max_cands: int = 64):
         counts[str(nh)] = counts.get(str(nh), 0) + 1
     return {"candidates": len(args), "ms_per_candidate": dt * 1000.0 / len(args),
             "numharm_counts": counts,
-            "timing": "host wall clock around each synchronous call (upload, 6 kernel kinds, "
+            "timing": "host wall clock around each synchronous call (upload, kernels, "
                       "result copy)",
-            "launches_per_candidate": "2 + 3 per distinct kernel FFT length + 1 per w-response "
-                                      "FFT length + 1"}
+            "launches_per_candidate": "4 + 1 per w-response FFT length"}
 
 
 def run_extras(args):
@@ -1057,7 +1056,7 @@ def main():
     per_launch_s = d["ms"] / 1000.0 / launches
     achieved = d["bytes"] / launches / per_launch_s / 1e9
     fp32_achieved = d["flops"] / launches / per_launch_s / 1e12
-    traffic = corr2048_traffic(args.batch) if dname == "corr_2048" else None
+    traffic = corr_traffic(args.batch) if dname == CORR_TRAFFIC["kernel"] else None
     peak, peak_kind = peaks()
     hs = kstats.get("harmsum")
     harmsum_roofline = None

@@ -112,14 +112,16 @@ typedef struct jerk_config {
     void *stream;             /* cudaStream_t to run on; NULL = a private stream */
     const void *device_bank;  /* optional resident bank (jerk_bank_generate); it
                                  must be complete when the plan is created (the
-                                 plan folds its fftlen-2048 and -1280 rows from it
+                                 plan folds its rows of fftlen 512 to 4096 from it
                                  then) */
     int harm_mode;            /* harmonic-sum kernel (a tuning knob; results do
                                  not depend on it): 1 = gather (global loads),
                                  2 = gather + TMA prefetch of the next tile into
                                  L2, 3 / 4 = TMA copies of 8 / 16-row tiles into
                                  shared memory (modes 2-4 fall back to 1 where
-                                 tensor maps cannot be built); 0 = 1 */
+                                 tensor maps cannot be built); 0 = rows copied
+                                 through a ring in shared memory on volumes of 48
+                                 MB and more per batch, to 16 harmonics, else 1 */
     int use_graph;            /* nonzero: each jerk_search / jerk_search_async
                                  pass is captured once per (first_rstep,
                                  num_rsteps) into a CUDA graph and replayed for

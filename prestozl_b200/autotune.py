@@ -11,8 +11,8 @@ and cached in a JSON file (``$JERK_TUNE_CACHE``, default
 
 The FFT radix plans are fixed per fftlen (``csrc/jerk_fft.cuh``) and the
 kernels' tile shapes are compile-time; the run-time knobs are B and the
-harmonic-sum kernel (jerk_config.harm_mode: plain gathers, gathers with TMA
-prefetch into L2, or TMA tiles in shared memory).
+harmonic-sum kernel (jerk_config.harm_mode: the default, plain gathers, gathers
+with TMA prefetch into L2, or TMA tiles in shared memory).
 """
 
 from __future__ import annotations
@@ -24,7 +24,7 @@ from typing import Dict, Optional, Sequence
 from . import jerk
 
 DEFAULT_CANDIDATES = (16, 32, 64)
-DEFAULT_HARM_MODES = (1, 2, 4)
+DEFAULT_HARM_MODES = (0, 1, 2, 4)
 
 
 def cache_path() -> str:

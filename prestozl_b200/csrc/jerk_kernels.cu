@@ -2,7 +2,9 @@
 // dense contraction, so there is no tensor-core path).
 //
 // Per batch of rsteps (one rstep = corr_uselen interbinned fundamental
-// bins), three kernels run on one stream:
+// bins), three steps run on one stream; rows of fftlen 512 to 4096 are correlated
+// by jerk_fold.cu (half-length transforms of folded rows), and large volumes
+// summed by jerk_harm.cu (rows copied through shared memory):
 //
 //  1. prep_kernel      one CTA per (rstep, subharmonic): gathers fftlen/2
 //                      spectral bins, block-median normalises them exactly as
@@ -20,7 +22,7 @@
 //  3. harmsum_kernel   one thread per fundamental (w, z, r): the stage-0
 //                      threshold, then the subharmonic adds in the reference's
 //                      order with a threshold after each stage; hits go to a
-//                      compact list through warp-aggregated atomics.
+//                      compact list through atomics.
 //                      (reference: src/accel_utils.c:1356-1377, 1507-1555;
 //                      src/accel_kernels.cu:781-862)
 #include <cuda_runtime.h>
