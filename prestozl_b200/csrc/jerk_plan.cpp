@@ -2671,6 +2671,12 @@ extern "C" int jerk_debug_volume(jerk_plan *p, const void *spectrum, int spectru
     SearchDev a = make_args(p, spec);
     a.first_rstep = rstep;
     a.nb = 1;
+    // a pass in flight may hold its next batch's prepared rows: the volume's go
+    // into the other buffers, which the batches enqueued so far have read when
+    // this preparation starts
+    const int buf = p->pass.prepared ? p->pass.buf ^ 1 : 0;
+    a.prepped = p->d_prepped[buf];
+    a.rinds = p->d_rinds[buf];
     rc = run_volumes(p, a, false, nullptr);
     if (rc != JERK_OK)
         return rc;
