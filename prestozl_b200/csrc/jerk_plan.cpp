@@ -1641,6 +1641,16 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
     return JERK_OK;
 }
 
+static int copy_spectrum(jerk_plan *p, float2 *dst, const void *spectrum, int on_device)
+{
+    JERK_CUDA(cudaMemcpyAsync(dst, spectrum, sizeof(float2) * p->obs.numbins,
+                              on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                              p->stream));
+    if (!on_device)
+        p->h2d_bytes += (long long)sizeof(float2) * p->obs.numbins;
+    return JERK_OK;
+}
+
 static int stage_spectrum(jerk_plan *p, const void *spectrum, int on_device, const float2 **spec)
 {
     if (on_device && !p->use_graph) {
@@ -1653,13 +1663,8 @@ static int stage_spectrum(jerk_plan *p, const void *spectrum, int on_device, con
         JERK_CUDA(cudaMalloc(&p->d_spec, sizeof(float2) * p->obs.numbins));
         p->spec_cap = p->obs.numbins;
     }
-    JERK_CUDA(cudaMemcpyAsync(p->d_spec, spectrum, sizeof(float2) * p->obs.numbins,
-                              on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                              p->stream));
-    if (!on_device)
-        p->h2d_bytes += (long long)sizeof(float2) * p->obs.numbins;
     *spec = p->d_spec;
-    return JERK_OK;
+    return copy_spectrum(p, p->d_spec, spectrum, on_device);
 }
 
 static SearchDev make_args(const jerk_plan *p, const float2 *spec)
@@ -2665,7 +2670,22 @@ extern "C" int jerk_debug_volume(jerk_plan *p, const void *spectrum, int spectru
         rstep >= p->nrsteps)
         return fail(JERK_EINVAL, "jerk_debug_volume: bad argument");
     const float2 *spec = nullptr;
-    int rc = stage_spectrum(p, spectrum, spectrum_on_device, &spec);
+    int rc = JERK_OK;
+    // a pass in flight may read the staged spectrum: the volume's own is then
+    // read in place, or copied to an array that lives until it is done
+    struct Staged {
+        float2 *d = nullptr;
+        ~Staged() { cudaFree(d); }
+    } own;
+    if (p->in_flight && spectrum_on_device) {
+        spec = (const float2 *)spectrum;
+    } else if (p->in_flight && p->inflight_spec == p->d_spec) {
+        JERK_CUDA(cudaMalloc(&own.d, sizeof(float2) * p->obs.numbins));
+        rc = copy_spectrum(p, own.d, spectrum, spectrum_on_device);
+        spec = own.d;
+    } else {
+        rc = stage_spectrum(p, spectrum, spectrum_on_device, &spec);
+    }
     if (rc != JERK_OK)
         return rc;
     SearchDev a = make_args(p, spec);

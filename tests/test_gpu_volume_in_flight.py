@@ -9,7 +9,7 @@ from prestozl_b200 import jerk
 pytestmark = pytest.mark.gpu
 
 
-def _problem(torch, batch):
+def _problem(torch, batch, max_hits=0, graph=False):
     N = 1 << 20
     g = torch.Generator(device="cuda")
     g.manual_seed(21)
@@ -20,7 +20,8 @@ def _problem(torch, batch):
         obs.powcut[i] = 11.0 + 3.0 * (1 << i) ** 0.75
     subs = jerk.subharm_sizes(obs, fftlen)
     bank = jerk.DeviceBank(subs)
-    return spec, jerk.JerkPlan(obs, subs, batch=batch, device_bank=bank.ptr.value), bank
+    return spec, jerk.JerkPlan(obs, subs, batch=batch, max_hits=max_hits, use_graph=graph,
+                               device_bank=bank.ptr.value), bank
 
 
 def _same_hits(got, want):
@@ -47,3 +48,26 @@ def test_volume_between_waves_leaves_the_pass_alone(waves):
         assert r == r0 and np.array_equal(v.view(np.uint32), v0.view(np.uint32))
     plan.close()
     bank.close()
+
+
+@pytest.mark.parametrize("graph,host", [(False, True), (True, False), (True, True)])
+def test_volume_of_another_spectrum_leaves_a_staged_pass_alone(graph, host):
+    """The pass reads its spectrum from the plan's own copy (host memory, or a plan
+    that replays graphs); the volume is of another spectrum, and the pass is also
+    run again from that copy (more hits than the buffer holds)."""
+    torch = pytest.importorskip("torch")
+    spec, plan, bank = _problem(torch, batch=4, max_hits=64, graph=graph)
+    other = torch.flip(spec, (0,))
+    if host:
+        spec, other = spec.cpu().numpy(), other.cpu().numpy()
+    ref_spec, ref, ref_bank = _problem(torch, batch=4)
+    want = ref.search(ref_spec, 2, 39, want_hits=True)[1:]
+    v0 = ref.volume(torch.flip(ref_spec, (0,)), 20, 1)
+    plan.begin(spec, 2, 39)
+    assert jerk.group_advance([plan], ahead=2) == 1
+    v = plan.volume(other, 20, 1)
+    assert v[1] == v0[1] and np.array_equal(v[0].view(np.uint32), v0[0].view(np.uint32))
+    _same_hits(plan.collect(want_hits=True)[1:], want)
+    assert len(want[0]) > 64
+    for p in (plan, bank, ref, ref_bank):
+        p.close()
