@@ -613,21 +613,26 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiOcc)
     const FoldRows R = P.rowsets[S.set];
     int b0, b1;
     rstep_chunk(P.nb, S.ny, local % S.ny, &b0, &b1);
+    // Warps past the row's own leave at once: the barriers of the row's body
+    // count the threads that have not left, and one that waited for the kernel
+    // before would hold its CTA's first barrier until that kernel had ended.
     switch (R.len) {
 #define JERK_MF(LL)                                                       \
     case LL:                                                              \
-        if (threadIdx.x < Multi<LL>::F::Threads)                          \
-            fold_cta<LL, Multi<LL>::Rows>(P, R, g * Multi<LL>::Rows, b0, b1); \
+        if (threadIdx.x >= Multi<LL>::F::Threads)                         \
+            return;                                                       \
+        fold_cta<LL, Multi<LL>::Rows>(P, R, g * Multi<LL>::Rows, b0, b1); \
         break;
     JERK_MF(256) JERK_MF(384) JERK_MF(512) JERK_MF(640) JERK_MF(768) JERK_MF(1024)
 #undef JERK_MF
 #define JERK_MC(NN)                                        \
-    case -NN:                                              \
-        if (threadIdx.x < (FftPlan<NN>::T + 31) / 32 * 32) { \
-            const int2 rm = R.map[g];                      \
-            corr_body<NN>(P, rm.x, rm.y, b0, b1);          \
-        }                                                  \
-        break;
+    case -NN: {                                            \
+        if (threadIdx.x >= (FftPlan<NN>::T + 31) / 32 * 32) \
+            return;                                        \
+        const int2 rm = R.map[g];                          \
+        corr_body<NN>(P, rm.x, rm.y, b0, b1);              \
+        break;                                             \
+    }
     JERK_MC(128) JERK_MC(192) JERK_MC(256) JERK_MC(384)
 #undef JERK_MC
     default: break;

@@ -1134,10 +1134,11 @@ static int build_harm_tma(jerk_plan *p, bool in_smem)
 // Whether a row set is launched by itself rather than merged with others: its
 // CTAs make two waves; or, for the half lengths whose rows leave a warp of the
 // merged launch's four idle (768, 640, 384), four waves over the rsteps --
-// the launches overlap, so that a last partial wave is no loss.  Measured (us
+// the launches overlap, so that a last partial wave is no loss.  Measured (ms
 // per pass; merged against own): 6 trials of 2^21 samples, zmax 50, wmax 150,
-// 8 harmonics 105900 / 101300; 2^22 samples, zmax 100, 16 harmonics 14660 /
-// 14500, and 15300 with its 359 rows of 1024 by themselves as well.
+// 8 harmonics 103.4 / 100.3; 2^22 samples, zmax 100, 16 harmonics 13.75 /
+// 13.70, and 14.32 with its 359 rows of 1024 by themselves as well; against it
+// 2^21 samples, zmax 100, wmax 100, 4 harmonics, batches of 8, 18.2 / 19.0.
 static bool own_launch_wins(int L, long long n, int batch)
 {
     const long long groups = n / fold_cta_rows(L), wave = fold_wave_ctas(L);
