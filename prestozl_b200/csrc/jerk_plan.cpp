@@ -1026,6 +1026,31 @@ extern "C" void jerk_plan_destroy(jerk_plan *p)
     delete p;
 }
 
+// Device memory for a plan that holds its own already (a larger hit buffer, a
+// staged spectrum).  Where there is none left, the buffers that let a batch be
+// prepared ahead make room: the plan works without them, and a batch prepared
+// there is prepared again in its turn.
+template <class T>
+static cudaError_t plan_malloc(jerk_plan *p, T **ptr, size_t bytes)
+{
+    *ptr = nullptr;
+    cudaError_t e = cudaMalloc(ptr, bytes);
+    if (e != cudaErrorMemoryAllocation || !p->d_rinds[1])
+        return e;
+    cudaGetLastError();
+    e = cudaStreamSynchronize(p->stream);
+    if (e != cudaSuccess)
+        return e;
+    drop_graph(p);  // a captured pass holds them
+    for (void *b : {(void *)p->d_prepped[1], (void *)p->d_rinds[1]})
+        cudaFree(b);
+    p->d_prepped[1] = nullptr;
+    p->d_rinds[1] = nullptr;
+    p->pass.prepared = false;
+    p->pass.buf = 0;
+    return cudaMalloc(ptr, bytes);
+}
+
 static int alloc_hits(jerk_plan *p, long long cap)
 {
     drop_graph(p);  // the captured pass holds the old hit buffers
@@ -1033,8 +1058,9 @@ static int alloc_hits(jerk_plan *p, long long cap)
     cudaFree(p->d_hit_pows);
     p->d_hit_keys = nullptr;
     p->d_hit_pows = nullptr;
-    JERK_CUDA(cudaMalloc(&p->d_hit_keys, sizeof(unsigned long long) * cap));
-    JERK_CUDA(cudaMalloc(&p->d_hit_pows, sizeof(float) * cap));
+    p->max_hits = 0;  // a pass without them stores nothing
+    JERK_CUDA(plan_malloc(p, &p->d_hit_keys, sizeof(unsigned long long) * cap));
+    JERK_CUDA(plan_malloc(p, &p->d_hit_pows, sizeof(float) * cap));
     p->max_hits = cap;
     return JERK_OK;
 }
@@ -1599,14 +1625,6 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
     // sum has read the volumes (running the two side by side on two streams
     // measured slower than back to back: their CTAs then share SMs)
     JERK_CUDA_B(cudaMalloc(&p->d_planes, sizeof(float) * p->plane_floats));
-    // the next batch's buffers are the last to be allocated and may be missing
-    if (cudaMalloc(&p->d_prepped[1], sizeof(float2) * p->prepped_f2) != cudaSuccess ||
-        cudaMalloc(&p->d_rinds[1], rinds_bytes) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(p->d_prepped[1]);
-        p->d_prepped[1] = nullptr;
-        p->d_rinds[1] = nullptr;
-    }
     if (p->harm_mode >= 2 && p->harm_mode <= 4) {
         const int rc = build_harm_tma(p, p->harm_mode >= 3);
         if (rc != JERK_OK)
@@ -1636,6 +1654,15 @@ extern "C" int jerk_plan_create(jerk_plan **out, const jerk_obs *obs, const jerk
         if (rc != JERK_OK)
             return bail(rc);
     }
+    // the next batch's buffers come last and may be missing; what is allocated
+    // later (plan_malloc) may take their place
+    if (cudaMalloc(&p->d_prepped[1], sizeof(float2) * p->prepped_f2) != cudaSuccess ||
+        cudaMalloc(&p->d_rinds[1], rinds_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(p->d_prepped[1]);
+        p->d_prepped[1] = nullptr;
+        p->d_rinds[1] = nullptr;
+    }
     JERK_CUDA_B(cudaStreamSynchronize(p->stream));
 #undef JERK_CUDA_B
     *out = p;
@@ -1661,7 +1688,7 @@ static int stage_spectrum(jerk_plan *p, const void *spectrum, int on_device, con
     if (p->spec_cap < p->obs.numbins) {
         cudaFree(p->d_spec);
         p->d_spec = nullptr;
-        JERK_CUDA(cudaMalloc(&p->d_spec, sizeof(float2) * p->obs.numbins));
+        JERK_CUDA(plan_malloc(p, &p->d_spec, sizeof(float2) * p->obs.numbins));
         p->spec_cap = p->obs.numbins;
     }
     *spec = p->d_spec;
@@ -2681,7 +2708,7 @@ extern "C" int jerk_debug_volume(jerk_plan *p, const void *spectrum, int spectru
     if (p->in_flight && spectrum_on_device) {
         spec = (const float2 *)spectrum;
     } else if (p->in_flight && p->inflight_spec == p->d_spec) {
-        JERK_CUDA(cudaMalloc(&own.d, sizeof(float2) * p->obs.numbins));
+        JERK_CUDA(plan_malloc(p, &own.d, sizeof(float2) * p->obs.numbins));
         rc = copy_spectrum(p, own.d, spectrum, spectrum_on_device);
         spec = own.d;
     } else {
