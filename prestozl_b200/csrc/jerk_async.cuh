@@ -42,7 +42,8 @@ __device__ __forceinline__ bool bar_wait(uint64_t *bar, unsigned parity)
 
 // Status bits written by the kernels (read back after each pass).
 constexpr unsigned kStatusRind = 1u;     // harmsum: a subharmonic r index left its row
-constexpr unsigned kStatusCopy = 2u;     // a copy into shared memory did not complete
+constexpr unsigned kStatusCopy = 2u;     // correlation: a copy into shared memory did not complete
+constexpr unsigned kStatusSumCopy = 4u;  // harmsum: the same
 
 // SMs of the current device (queried once; every B200 has 148)
 inline int sm_count()

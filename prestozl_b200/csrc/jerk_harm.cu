@@ -356,7 +356,7 @@ __device__ __forceinline__ void ring_body(const SearchDev &P, const RingPlan &W,
             const unsigned total = __reduce_add_sync(0xffffffffu, fresh ? bytes : 0u);
             if (!__all_sync(0xffffffffu, bar_wait(&empty[slot], phase) && !*(volatile int *)&s_dead)) {
                 if (s == 0)
-                    atomicOr(P.status, kStatusCopy);
+                    atomicOr(P.status, kStatusSumCopy);
                 *(volatile int *)&s_dead = 1;
                 // the copies in flight land before the CTA ends (bounded)
                 for (int d = 0; d < R::D; d++)
@@ -412,7 +412,7 @@ __device__ __forceinline__ void ring_body(const SearchDev &P, const RingPlan &W,
         for (; I.z < I.zend; I.z++) {
             if (!bar_wait(&full[slot], phase)) {
                 *(volatile int *)&s_dead = 1;
-                atomicOr(P.status, kStatusCopy);
+                atomicOr(P.status, kStatusSumCopy);
                 ok = false;
                 break;
             }

@@ -398,21 +398,22 @@ __global__ void __launch_bounds__(LONG ? 1024 : 256, LONG ? 1 : 2)
 
 // A wait that must run out: the correlation's bounded wait (bar_wait) on an
 // mbarrier whose phase 0 nothing completes (no copy is involved, so nothing
-// is left in flight).  It gives up after its poll limit and reports as a
-// data-row copy that never completed would.  Launched by plans whose wait
-// probe is on (jerk_debug_wait_probe), one thread.
-__global__ void wait_probe_kernel(unsigned int *status)
+// is left in flight).  It gives up after its poll limit and reports as a copy
+// that never completed would: the correlation's or the harmonic sum's, by
+// `bits`.  Launched by plans whose wait probe is on (jerk_debug_wait_probe),
+// one thread.
+__global__ void wait_probe_kernel(unsigned int *status, unsigned bits)
 {
     __shared__ uint64_t s_probe;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_probe)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     if (!bar_wait(&s_probe, 0) && status)
-        atomicOr(status, kStatusCopy);
+        atomicOr(status, bits);
 }
 
-cudaError_t launch_wait_probe(unsigned int *status, cudaStream_t st)
+cudaError_t launch_wait_probe(unsigned int *status, bool sum, cudaStream_t st)
 {
-    wait_probe_kernel<<<1, 1, 0, st>>>(status);
+    wait_probe_kernel<<<1, 1, 0, st>>>(status, sum ? kStatusSumCopy : kStatusCopy);
     return cudaGetLastError();
 }
 
@@ -886,7 +887,7 @@ __global__ void __launch_bounds__(kHarmThreads, HarmTmaOcc<S, ZT>::value)
     __syncthreads();
     if (smem_u32(box) & 127u) {  // unreachable by construction; never issue a misaligned copy
         if (tid == 0)
-            atomicOr(P.status, kStatusCopy);
+            atomicOr(P.status, kStatusSumCopy);
         return;
     }
 
@@ -933,7 +934,7 @@ __global__ void __launch_bounds__(kHarmThreads, HarmTmaOcc<S, ZT>::value)
         const bool ok = bar_wait(&s_bar, t & 1);
         if (__syncthreads_or(!ok)) {
             if (tid == 0) {
-                atomicOr(P.status, kStatusCopy);
+                atomicOr(P.status, kStatusSumCopy);
                 bar_wait(&s_bar, t & 1);  // once more, bounded, for the copies in flight
             }
             return;

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "jerk.h"
+#include "jerk_async.cuh"
 #include "jerk_kernels.cuh"
 
 namespace jerk {
@@ -45,7 +46,7 @@ size_t harmsum_tma_smem_bytes(const HarmTma &T, int nsubs, int numz0);
 bool fftlen_supported(int n);
 cudaError_t launch_prep_group(GroupLaunch M, int maxfft, size_t smem, cudaStream_t st);
 cudaError_t launch_harmsum_group(GroupLaunch M, int nstages, cudaStream_t st);
-cudaError_t launch_wait_probe(unsigned int *status, cudaStream_t st);
+cudaError_t launch_wait_probe(unsigned int *status, bool sum, cudaStream_t st);
 cudaError_t fold_plan_attrs();
 cudaError_t launch_fold_roots(double2 *roots, int n, cudaStream_t st);
 cudaError_t launch_fold_support(const float2 *bank, const long long *src, int nrows, int N,
@@ -1928,7 +1929,7 @@ static int pass_begin(jerk_plan *p, const float2 *spec, long long first, long lo
     // a pass that reported a failed wait or index leaves no trace in the next
     JERK_CUDA(cudaMemsetAsync(p->d_status, 0, sizeof(unsigned int), p->stream));
     if (p->wait_probe)
-        JERK_CUDA(launch_wait_probe(p->d_status, p->stream));
+        JERK_CUDA(launch_wait_probe(p->d_status, p->wait_probe == 2, p->stream));
     return JERK_OK;
 }
 
@@ -2054,9 +2055,12 @@ static int finish_search_pass(jerk_plan *p, unsigned int *nhits_out)
     JERK_CUDA(cudaEventSynchronize(p->ev_done));
     collect_timings(p);
     p->d2h_bytes += 2 * sizeof(unsigned int);
-    if (p->h_counts[1] & 2u)
+    const unsigned status = p->h_counts[1];  // kStatus* (jerk_async.cuh)
+    if (status & kStatusCopy)
         return fail(JERK_ECUDA, "correlation: a data-row copy into shared memory timed out");
-    if (p->h_counts[1])
+    if (status & kStatusSumCopy)
+        return fail(JERK_ECUDA, "harmonic sum: a row copy into shared memory timed out");
+    if (status)
         return fail(JERK_EINVAL, "harmonic sum: a subharmonic r index left its row");
     *nhits_out = p->h_counts[0];
     return JERK_OK;
@@ -2686,7 +2690,7 @@ extern "C" int jerk_debug_wait_probe(jerk_plan *p, int on)
         return fail(JERK_EINVAL, "jerk_debug_wait_probe: null plan");
     if (p->in_flight)
         return fail(JERK_EINVAL, "jerk_debug_wait_probe: a search is in flight");
-    p->wait_probe = on != 0;
+    p->wait_probe = on == 2 ? 2 : on != 0;
     drop_graph(p);  // a captured pass holds the old launch arguments
     return JERK_OK;
 }

@@ -725,10 +725,11 @@ class JerkPlan:
         lib().jerk_plan_transfer_stats(self._p, C.byref(h), C.byref(d))
         return h.value, d.value
 
-    def set_wait_probe(self, on: bool) -> None:
+    def set_wait_probe(self, on) -> None:
         """Test hook: later passes also run one bounded wait that must give
-        up, and fail with JERK_ECUDA (jerk_debug_wait_probe)."""
-        _check(lib().jerk_debug_wait_probe(self._p, int(bool(on))))
+        up, and fail with JERK_ECUDA (jerk_debug_wait_probe; 2: as the
+        harmonic sum's copies would)."""
+        _check(lib().jerk_debug_wait_probe(self._p, int(on)))
 
     def volume(self, spectrum, rstep: int, sub: int):
         """ffdot volume [numw][numz][numrs] of one (rstep, subharmonic)."""
