@@ -582,9 +582,13 @@ int dr_layout(int numamps, DrRuns *out)
     return nb;
 }
 
+// Three words a block: level, mid, len.  There are far fewer blocks than
+// numamps / kDrInit (their length grows from 6 bins to 17 by bin 18 and 35 by
+// bin 400), and the first 21 fit in the rounding to 256 bytes: a size for one
+// word per kDrInit bins, which a caller may have allocated once, holds them.
 size_t dr_scratch(int numamps)
 {
-    return 3 * align256(sizeof(float) * (size_t)(numamps / kDrInit + 2));  // level, mid, len
+    return align256(sizeof(float) * (size_t)(numamps / kDrInit + 2));
 }
 
 // ---------------------------------------------------------------------------
@@ -725,13 +729,11 @@ int deredden_impl(void *spectrum, long long numamps, void *scratch, long long sc
                          "jerk_deredden: scratch smaller than jerk_deredden_scratch_bytes");
     DrRuns runs;
     const int nb = dr_layout((int)numamps, &runs);
-    if (nb < 1)
+    if (nb < 1 || 3 * sizeof(float) * (size_t)nb > dr_scratch((int)numamps))
         return set_error(JERK_EUNSUPPORTED, "jerk_deredden: block layout too long");
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t part = align256(sizeof(float) * (size_t)(numamps / kDrInit + 2));
     float *level = (float *)scratch;
-    int *mid = (int *)((unsigned char *)scratch + part);
-    int *len = (int *)((unsigned char *)scratch + 2 * part);
+    int *mid = (int *)scratch + nb, *len = mid + nb;
     float2 *x = (float2 *)spectrum;
     const int threads = 32 * kDrWarps;
     cudaError_t e = launch_follow(dr_level_kernel, (nb + kDrWarps - 1) / kDrWarps, threads, 0, st, x,
