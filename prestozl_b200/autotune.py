@@ -1,13 +1,12 @@
 """Autotuning of rsteps per launch (the batch size B) per search geometry.
 
 B trades kernel-bank reuse (each kernel row is read from HBM once per batch
-and kept in registers for B rsteps) against the size of the double-buffered
-ffdot volumes (2 x B x ~160 MB at -zmax 200 -wmax 300 -numharm 16) and the
-granularity of the overlap between a batch's harmonic sums and the next
-batch's correlations.  The best B depends on the geometry (fftlen, numz,
-numw, stages, corr_uselen), so it is measured once on a short partial search
-and cached in a JSON file (``$JERK_TUNE_CACHE``, default
-``~/.cache/prestozl_b200/autotune.json``).
+and kept in registers for B rsteps) against the size of the ffdot volumes
+(B x ~160 MB at -zmax 200 -wmax 300 -numharm 16).  The best B depends on the
+geometry (fftlen, numz, numw, stages, corr_uselen), so it is measured once on a
+short partial search and cached in a JSON file (``$JERK_TUNE_CACHE``, default
+``~/.cache/prestozl_b200/autotune.json``); a choice timed with other kernels than
+the present ones is measured again.
 
 The FFT radix plans are fixed per fftlen (``csrc/jerk_fft.cuh``) and the
 kernels' tile shapes are compile-time; the run-time knobs are B and the
@@ -17,11 +16,13 @@ with TMA prefetch into L2, or TMA tiles in shared memory).
 
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import os
 from typing import Dict, Optional, Sequence
 
-from . import jerk
+from . import build, jerk
 
 DEFAULT_CANDIDATES = (16, 32, 64)
 DEFAULT_HARM_MODES = (0, 1, 2, 4)
@@ -37,6 +38,24 @@ def geometry_key(obs: jerk.Obs, subs: Sequence[dict]) -> str:
     f = subs[0]
     return (f"fftlen={f['fftlen']}:numz={f['numz']}:numw={f['numw']}:"
             f"stages={obs.numharmstages}:uselen={obs.corr_uselen}")
+
+
+@functools.lru_cache(maxsize=None)
+def kernels() -> str:
+    """Names the kernels a choice was timed with: a digest of their sources."""
+    h = hashlib.sha256()
+    for f in build.SOURCES + build.HEADERS:
+        with open(os.path.join(build.CSRC, f), "rb") as fh:
+            h.update(fh.read())
+    return h.hexdigest()[:16]
+
+
+def _usable(entry: Optional[dict]) -> bool:
+    """Whether an entry still says what is fastest: one that tune() timed with
+    other kernels does not (its harm_mode may be a form that is no longer the
+    fastest, or may lack one that was not there).  One that was put there
+    without timings is the user's own choice."""
+    return bool(entry) and ("ms_per_rstep" not in entry or entry.get("kernels") == kernels())
 
 
 def _load() -> Dict[str, dict]:
@@ -59,8 +78,10 @@ def _store(db: Dict[str, dict]) -> None:
 
 
 def cached(obs: jerk.Obs, subs: Sequence[dict]) -> Optional[dict]:
-    """The cached choice for this geometry ({"batch_rsteps", "harm_mode", ...})."""
-    return _load().get(geometry_key(obs, subs))
+    """The cached choice for this geometry ({"batch_rsteps", "harm_mode", ...});
+    one timed with other kernels than these is a miss."""
+    entry = _load().get(geometry_key(obs, subs))
+    return entry if _usable(entry) else None
 
 
 def tune(obs: jerk.Obs, subs: Sequence[dict], bank_ptr: int, spectrum,
@@ -74,8 +95,11 @@ def tune(obs: jerk.Obs, subs: Sequence[dict], bank_ptr: int, spectrum,
 
     key = geometry_key(obs, subs)
     db = _load() if use_cache else {}
-    if use_cache and key in db:
-        return db[key]
+    entry = db.get(key)
+    if _usable(entry) and ("ms_per_rstep" not in entry or
+                           (entry["batch_rsteps"] in candidates and
+                            entry["harm_mode"] in harm_modes)):
+        return entry
     times = {}
     for B in candidates:
         for hr in harm_modes:
@@ -99,7 +123,7 @@ def tune(obs: jerk.Obs, subs: Sequence[dict], bank_ptr: int, spectrum,
     best = min(times, key=times.get)
     entry = {"batch_rsteps": best[0], "harm_mode": best[1],
              "ms_per_rstep": {f"B{k[0]}/mode{k[1]}": v for k, v in times.items()},
-             "rsteps_timed": rsteps}
+             "rsteps_timed": rsteps, "kernels": kernels()}
     if use_cache:
         db[key] = entry
         _store(db)
