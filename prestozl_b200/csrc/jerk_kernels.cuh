@@ -116,10 +116,11 @@ struct SearchDev {
 };
 
 // A bank row to fold (jerk_fold.cu): offset (float2) in the bank, -1 for a
-// padding row; its fftlen; its support, -1 to fold the row's own values.
+// padding row; its fftlen; its support, -1 to fold the row's own values; the
+// support it is expected to have, where that is to be checked (else 0).
 struct FoldSrc {
     long long off;
-    int N, h;
+    int N, h, expect;
 };
 
 // Tensor maps of the harmonic sum's TMA path: subharmonic s's batch volumes

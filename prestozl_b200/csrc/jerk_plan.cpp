@@ -52,7 +52,7 @@ cudaError_t launch_fold_roots(double2 *roots, int n, cudaStream_t st);
 cudaError_t launch_fold_support(const float2 *bank, const long long *src, int nrows, int N,
                                 const double2 *rootsN, int *half, cudaStream_t st);
 cudaError_t launch_fold_rows(const float2 *bank, const FoldSrc *src, int nrows, int L, int maxN,
-                             const double2 *roots, const int *roots_at, float2 *out,
+                             const double2 *roots, const int *roots_at, float2 *out, int *differs,
                              cudaStream_t st);
 int fold_twiddle_size(int L);
 void fold_twiddle_table(int L, float2 *out);
@@ -1153,11 +1153,6 @@ static int build_harm_tma(jerk_plan *p, bool in_smem)
     return JERK_OK;
 }
 
-// The plan's row sets.  Fold the bank's rows of every folded length: measure
-// each row's support, choose its half length, lay out the classes (their
-// prepared windows from *data_off on) and write the folded rows, class after
-// class, longest half length first; then the maps of the short lengths that
-// do not fold (fftlen 128 to 384).
 // Whether a row set is launched by itself rather than merged with others: its
 // CTAs make two waves; or, for the half lengths whose rows leave a warp of the
 // merged launch's four idle (768, 640, 384), four waves over the rsteps --
@@ -1173,84 +1168,30 @@ static bool own_launch_wins(int L, long long n, int batch)
     return groups >= 2 * wave || (idle && groups * batch >= 4 * wave);
 }
 
-static int fold_bank(jerk_plan *p, const std::vector<int> &maxnumrs, long long *data_off)
+// Scratch of folding a bank on the device, freed on every path (cudaFree waits
+// for the kernels reading it), and the tables in it.
+struct FoldScratch {
+    char *mem = nullptr;
+    double2 *roots = nullptr;     // exp(-2 pi i m / n) of every length n taken
+    int *roots_at = nullptr;      // [n / 128]: where they start
+    long long *src = nullptr;     // the rows' places in the bank
+    FoldSrc *fsrc = nullptr;
+    int *half = nullptr;          // their supports
+    int *differs = nullptr;       // set where a support is not the expected one
+    ~FoldScratch() { cudaFree(mem); }
+};
+
+// The plan's row sets for supports `half` (of subharmonic s from first_row[s]
+// on): the rows of every folded length in the shortest half length that holds
+// them, laid out by class (their prepared windows from *data_off on) and written
+// class after class, longest half length first; then the maps of the short
+// lengths that do not fold (fftlen 128 to 384).  check: the supports are what
+// generated rows have; *same says whether the bank's do.
+static int fold_rows(jerk_plan *p, const std::vector<int> &maxnumrs, const std::vector<int> &half,
+                     const std::vector<long long> &first_row, const FoldScratch &sc, bool check,
+                     long long *data_off, bool *same)
 {
-    std::map<int, std::vector<int>> subs_of;  // fftlen -> subharmonics
-    for (int s = 0; s < p->nsubs; s++)
-        if (folded_fftlen(p->subs[s].fftlen))
-            subs_of[p->subs[s].fftlen].push_back(s);
     cudaStream_t st = p->stream;
-    JERK_CUDA(fold_plan_attrs());
-
-    // root tables of every length the folding may take
-    int roots_at[4096 / 128 + 1];
-    int nroots = 0, maxN = 0;
-    std::fill(std::begin(roots_at), std::end(roots_at), -1);
-    std::vector<int> lens(std::begin(kFoldLens), std::end(kFoldLens));
-    for (auto &kv : subs_of) {
-        lens.push_back(kv.first);
-        maxN = std::max(maxN, kv.first);
-    }
-    for (int n : lens)
-        if (n <= maxN && roots_at[n / 128] < 0) {
-            roots_at[n / 128] = nroots;
-            nroots += n;
-        }
-
-    // supports
-    long long nrows = 0;
-    for (auto &kv : subs_of)
-        for (int s : kv.second)
-            nrows += (long long)p->subs[s].numw * p->subs[s].numz;
-    if (nrows > INT_MAX)
-        return fail(JERK_EUNSUPPORTED, "too many kernel rows");
-    std::vector<long long> src;
-    src.reserve(nrows);
-    std::vector<long long> first_row(p->nsubs, 0);
-    for (auto &kv : subs_of)
-        for (int s : kv.second) {
-            first_row[s] = (long long)src.size();
-            const long long n = (long long)p->subs[s].numw * p->subs[s].numz;
-            for (long long r = 0; r < n; r++)
-                src.push_back(p->hsubs[s].kern_off + r * kv.first);
-        }
-    // scratch of this function: roots, supports, then the row sources (the
-    // padding adds at most three rows a class); freed on every path (cudaFree
-    // waits for the kernels reading it)
-    struct Scratch {
-        char *p = nullptr;
-        ~Scratch() { cudaFree(p); }
-    } sc;
-    const size_t pad_rows = 4 * (size_t)kNumFoldLens * p->nsubs;
-    const size_t b_roots = sizeof(double2) * nroots, b_at = 256,
-                 b_src = sizeof(long long) * (size_t)nrows,
-                 b_fsrc = sizeof(FoldSrc) * ((size_t)nrows + pad_rows),
-                 b_half = sizeof(int) * (size_t)nrows;
-    static_assert(sizeof(roots_at) <= 256, "roots_at");
-    JERK_CUDA(cudaMalloc(&sc.p, b_roots + b_at + b_src + b_fsrc + b_half + 16));
-    double2 *d_roots = (double2 *)sc.p;
-    int *d_roots_at = (int *)(sc.p + b_roots);
-    long long *d_src = (long long *)(sc.p + b_roots + b_at);
-    FoldSrc *d_fsrc = (FoldSrc *)(sc.p + b_roots + b_at + b_src);
-    int *d_half = (int *)(sc.p + b_roots + b_at + b_src + b_fsrc);
-    for (int n : lens)
-        if (n <= maxN && roots_at[n / 128] >= 0)
-            JERK_CUDA(launch_fold_roots(d_roots + roots_at[n / 128], n, st));
-    JERK_CUDA(cudaMemcpyAsync(d_roots_at, roots_at, sizeof(roots_at), cudaMemcpyHostToDevice, st));
-    JERK_CUDA(cudaMemcpyAsync(d_src, src.data(), sizeof(long long) * nrows, cudaMemcpyHostToDevice,
-                              st));
-    for (auto &kv : subs_of) {
-        const long long at = first_row[kv.second.front()];
-        long long n = 0;
-        for (int s : kv.second)
-            n += (long long)p->subs[s].numw * p->subs[s].numz;
-        JERK_CUDA(launch_fold_support(p->d_bank, d_src + at, (int)n, kv.first,
-                                      d_roots + roots_at[kv.first / 128], d_half + at, st));
-    }
-    std::vector<int> half(nrows);
-    JERK_CUDA(cudaMemcpyAsync(half.data(), d_half, sizeof(int) * nrows, cudaMemcpyDeviceToHost, st));
-    JERK_CUDA(cudaStreamSynchronize(st));
-
     // classes: a subharmonic's rows of one half length
     struct Built {
         std::vector<FoldSrc> src;
@@ -1288,12 +1229,15 @@ static int fold_bank(jerk_plan *p, const std::vector<int> &maxnumrs, long long *
             Built &B = built[i];
             B.maxN = std::max(B.maxN, sh.fftlen);
             for (int r : of[i]) {
+                // (rows of the whole length fold whatever their support: a
+                // sixteenth of them is checked)
+                const bool whole = c.len == M;
                 B.src.push_back({d.kern_off + (long long)r * sh.fftlen, sh.fftlen,
-                                 c.len == M ? -1 : h[r]});
+                                 whole ? -1 : h[r], check && !(whole && r % 16) ? h[r] : 0});
                 B.map.push_back(make_int2(ci, r));
             }
             while (B.src.size() % fold_cta_rows(c.len)) {
-                B.src.push_back({-1, sh.fftlen, -1});
+                B.src.push_back({-1, sh.fftlen, -1, 0});
                 B.map.push_back(make_int2(-1, 0));
             }
             p->fold_classes.push_back(c);
@@ -1322,6 +1266,8 @@ static int fold_bank(jerk_plan *p, const std::vector<int> &maxnumrs, long long *
         JERK_CUDA(cudaMalloc(&p->d_fold, sizeof(float2) * f2));
     if (total)
         JERK_CUDA(cudaMalloc(&p->d_foldmap, sizeof(int2) * total));
+    if (check)
+        JERK_CUDA(cudaMemsetAsync(sc.differs, 0, sizeof(int), st));
     long long row = 0, at = 0;
     for (int i = kNumFoldLens - 1; i >= 0; i--) {
         const Built &B = built[i];
@@ -1329,12 +1275,12 @@ static int fold_bank(jerk_plan *p, const std::vector<int> &maxnumrs, long long *
         if (!n)
             continue;
         const int L = kFoldLens[i];
-        JERK_CUDA(cudaMemcpyAsync(d_fsrc + row, B.src.data(), sizeof(FoldSrc) * n,
+        JERK_CUDA(cudaMemcpyAsync(sc.fsrc + row, B.src.data(), sizeof(FoldSrc) * n,
                                   cudaMemcpyHostToDevice, st));
         JERK_CUDA(cudaMemcpyAsync(p->d_foldmap + row, B.map.data(), sizeof(int2) * n,
                                   cudaMemcpyHostToDevice, st));
-        JERK_CUDA(launch_fold_rows(p->d_bank, d_fsrc + row, (int)n, L, B.maxN, d_roots, d_roots_at,
-                                   p->d_fold + at, st));
+        JERK_CUDA(launch_fold_rows(p->d_bank, sc.fsrc + row, (int)n, L, B.maxN, sc.roots,
+                                   sc.roots_at, p->d_fold + at, check ? sc.differs : nullptr, st));
         FoldRows R{};
         R.len = L;
         R.n = (int)n;
@@ -1359,8 +1305,120 @@ static int fold_bank(jerk_plan *p, const std::vector<int> &maxnumrs, long long *
     }
     if (p->rowsets.size() > (size_t)kMaxRowSets)
         return fail(JERK_EUNSUPPORTED, "too many row sets");
+    int differs = 0;
+    if (check) {
+        JERK_CUDA(cudaMemcpyAsync(&differs, sc.differs, sizeof(int), cudaMemcpyDeviceToHost, st));
+        JERK_CUDA(cudaStreamSynchronize(st));
+    }
+    *same = !differs;
     // the host tables above are pageable: copied before these calls returned
     return JERK_OK;
+}
+
+// Folds the bank's rows into the plan's row sets.  Generated rows are as wide as
+// their responses, which the folding checks; measuring every row first
+// transforms each back twice (a plan on a shared bank, zmax 300, wmax 600, 2
+// harmonics: 10.8 ms with that, 7.7 without; 200, 300, 16: 12.9 and 12.5).
+static int fold_bank(jerk_plan *p, const std::vector<int> &maxnumrs, long long *data_off)
+{
+    std::map<int, std::vector<int>> subs_of;  // fftlen -> subharmonics
+    for (int s = 0; s < p->nsubs; s++)
+        if (folded_fftlen(p->subs[s].fftlen))
+            subs_of[p->subs[s].fftlen].push_back(s);
+    cudaStream_t st = p->stream;
+    JERK_CUDA(fold_plan_attrs());
+
+    // root tables of every length the folding may take
+    int roots_at[4096 / 128 + 1];
+    int nroots = 0, maxN = 0;
+    std::fill(std::begin(roots_at), std::end(roots_at), -1);
+    std::vector<int> lens(std::begin(kFoldLens), std::end(kFoldLens));
+    for (auto &kv : subs_of) {
+        lens.push_back(kv.first);
+        maxN = std::max(maxN, kv.first);
+    }
+    for (int n : lens)
+        if (n <= maxN && roots_at[n / 128] < 0) {
+            roots_at[n / 128] = nroots;
+            nroots += n;
+        }
+
+    long long nrows = 0;
+    bool generated = !p->own_bank;  // as the rows' (z, w) would be by the sizes
+    std::vector<long long> first_row(p->nsubs, 0);
+    for (auto &kv : subs_of)
+        for (int s : kv.second) {
+            const jerk_subharm &sh = p->subs[s];
+            first_row[s] = nrows;
+            nrows += (long long)sh.numw * sh.numz;
+            generated = generated && sh.numz == sh.zmax / kDZ * 2 + 1 &&
+                        sh.numw == sh.wmax / kDW * 2 + 1;
+        }
+    if (nrows > INT_MAX)
+        return fail(JERK_EUNSUPPORTED, "too many kernel rows");
+    // (the padding adds at most three rows a class)
+    FoldScratch sc;
+    const size_t pad_rows = 4 * (size_t)kNumFoldLens * p->nsubs;
+    const size_t b_roots = sizeof(double2) * nroots, b_at = 256,
+                 b_src = sizeof(long long) * (size_t)nrows,
+                 b_fsrc = sizeof(FoldSrc) * ((size_t)nrows + pad_rows),
+                 b_half = sizeof(int) * (size_t)nrows;
+    static_assert(sizeof(roots_at) <= 256, "roots_at");
+    JERK_CUDA(cudaMalloc(&sc.mem, b_roots + b_at + b_src + b_fsrc + b_half + 16));
+    sc.roots = (double2 *)sc.mem;
+    sc.roots_at = (int *)(sc.mem + b_roots);
+    sc.src = (long long *)(sc.mem + b_roots + b_at);
+    sc.fsrc = (FoldSrc *)(sc.mem + b_roots + b_at + b_src);
+    sc.half = (int *)(sc.mem + b_roots + b_at + b_src + b_fsrc);
+    sc.differs = sc.half + nrows;
+    for (int n : lens)
+        if (n <= maxN && roots_at[n / 128] >= 0)
+            JERK_CUDA(launch_fold_roots(sc.roots + roots_at[n / 128], n, st));
+    JERK_CUDA(cudaMemcpyAsync(sc.roots_at, roots_at, sizeof(roots_at), cudaMemcpyHostToDevice, st));
+
+    std::vector<int> half(nrows);
+    bool same = false;
+    if (generated) {
+        for (auto &kv : subs_of)
+            for (int s : kv.second) {
+                const jerk_subharm &sh = p->subs[s];
+                for (int ii = 0; ii < sh.numw; ii++)
+                    for (int jj = 0; jj < sh.numz; jj++)
+                        half[first_row[s] + (long long)ii * sh.numz + jj] =
+                            w_resp_halfwidth(-sh.zmax + jj * kDZ, -sh.wmax + ii * kDW);
+            }
+        const long long at = *data_off;
+        const int rc = fold_rows(p, maxnumrs, half, first_row, sc, true, data_off, &same);
+        if (rc != JERK_OK || same)
+            return rc;
+        *data_off = at;
+        cudaFree(p->d_fold);
+        cudaFree(p->d_foldmap);
+        p->d_fold = nullptr;
+        p->d_foldmap = nullptr;
+        p->fold_classes.clear();
+        p->rowsets.clear();
+        p->own_launch.clear();
+        for (SubDev &d : p->hsubs)
+            d.cls0 = d.ncls = 0;
+    }
+    std::vector<long long> src(nrows);
+    for (auto &kv : subs_of)
+        for (int s : kv.second)
+            for (long long r = 0; r < (long long)p->subs[s].numw * p->subs[s].numz; r++)
+                src[first_row[s] + r] = p->hsubs[s].kern_off + r * kv.first;
+    JERK_CUDA(cudaMemcpyAsync(sc.src, src.data(), b_src, cudaMemcpyHostToDevice, st));
+    for (auto &kv : subs_of) {
+        const long long at = first_row[kv.second.front()];
+        long long n = 0;
+        for (int s : kv.second)
+            n += (long long)p->subs[s].numw * p->subs[s].numz;
+        JERK_CUDA(launch_fold_support(p->d_bank, sc.src + at, (int)n, kv.first,
+                                      sc.roots + roots_at[kv.first / 128], sc.half + at, st));
+    }
+    JERK_CUDA(cudaMemcpyAsync(half.data(), sc.half, b_half, cudaMemcpyDeviceToHost, st));
+    JERK_CUDA(cudaStreamSynchronize(st));
+    return fold_rows(p, maxnumrs, half, first_row, sc, false, data_off, &same);
 }
 
 static int plane_stride(int numrs) { return (numrs + kPlaneAlign - 1) / kPlaneAlign * kPlaneAlign; }
