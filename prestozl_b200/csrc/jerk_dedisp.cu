@@ -29,7 +29,6 @@
 #include <climits>
 #include <cstdint>
 #include <cstdio>
-#include <utility>
 #include <vector>
 
 #include "jerk.h"
@@ -280,7 +279,8 @@ struct jerk_dedisperser {
     size_t smem = 0;
     int ps = 0;         // words per row of positions
     bool quads = true;  // staged by 16-byte loads where the blocks allow it
-    int *d_offsets = nullptr, *d_glo = nullptr, *d_gbase = nullptr, *d_grel = nullptr, *d_glen = nullptr;
+    int *d_offsets = nullptr;  // [numdms][nsub], then the other tables
+    const int *d_glo = nullptr, *d_gbase = nullptr, *d_grel = nullptr, *d_glen = nullptr;
     std::vector<int> h_offsets;
 };
 
@@ -303,14 +303,22 @@ size_t dd_tables(const int *off, int numdms, int nsub, int G, int T, std::vector
         base->assign((size_t)ngroups * (nsub + 1), 0);
     }
     size_t worst = 0;
+    std::vector<int> low(nsub), high(nsub);
     for (int g = 0; g < ngroups; g++) {
+        // (along the rows of the offsets, which the compiler vectorises)
+        const int *o = off + (size_t)g * G * nsub;
+        std::copy(o, o + nsub, low.begin());
+        std::copy(o, o + nsub, high.begin());
+        for (int d = g * G + 1; d < std::min(numdms, (g + 1) * G); d++) {
+            o += nsub;
+            for (int s = 0; s < nsub; s++) {
+                low[s] = std::min(low[s], o[s]);
+                high[s] = std::max(high[s], o[s]);
+            }
+        }
         long long total = 0;
         for (int s = 0; s < nsub; s++) {
-            int mn = INT_MAX, mx = INT_MIN;
-            for (int d = g * G; d < std::min(numdms, (g + 1) * G); d++) {
-                mn = std::min(mn, off[(size_t)d * nsub + s]);
-                mx = std::max(mx, off[(size_t)d * nsub + s]);
-            }
+            const int mn = low[s], mx = high[s];
             if (apart) {
                 const long long want = (nsub % 4 ? 4 * (s % 8) : 16 * (s / 4 & 1)) + mn;
                 total += (((want - total) % 32) + 32) % 32;
@@ -531,25 +539,21 @@ extern "C" int jerk_dedisperser_create(jerk_dedisperser **out, int worklen, int 
         d->smem += pad;
     }
     d->h_offsets.assign(offsets, offsets + (size_t)numdms * nsub);
-    const size_t b_off = sizeof(int) * (size_t)numdms * nsub;
-    cudaError_t e = cudaMalloc(&d->d_offsets, b_off);
-    if (e == cudaSuccess)
-        e = cudaMalloc(&d->d_glo, sizeof(int) * lo.size());
-    if (e == cudaSuccess)
-        e = cudaMalloc(&d->d_gbase, sizeof(int) * base.size());
-    if (e == cudaSuccess)
-        e = cudaMemcpy(d->d_offsets, offsets, b_off, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(d->d_glo, lo.data(), sizeof(int) * lo.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(d->d_gbase, base.data(), sizeof(int) * base.size(), cudaMemcpyHostToDevice);
-    for (auto t : {std::make_pair(&d->d_grel, &rel), std::make_pair(&d->d_glen, &len)}) {
-        if (e == cudaSuccess)
-            e = cudaMalloc(t.first, sizeof(int) * t.second->size());
-        if (e == cudaSuccess)
-            e = cudaMemcpy(*t.first, t.second->data(), sizeof(int) * t.second->size(),
-                           cudaMemcpyHostToDevice);
+    // every table in one array: one allocation and one copy
+    std::vector<int> all(d->h_offsets);
+    size_t at[4];
+    int i = 0;
+    for (const std::vector<int> *t : {&lo, &base, &rel, &len}) {
+        at[i++] = all.size();
+        all.insert(all.end(), t->begin(), t->end());
     }
+    cudaError_t e = cudaMalloc(&d->d_offsets, sizeof(int) * all.size());
+    if (e == cudaSuccess)
+        e = cudaMemcpy(d->d_offsets, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice);
+    d->d_glo = d->d_offsets + at[0];
+    d->d_gbase = d->d_offsets + at[1];
+    d->d_grel = d->d_offsets + at[2];
+    d->d_glen = d->d_offsets + at[3];
     for (auto k : {dedisp_kernel<4, 8>, dedisp_kernel<4, 4>, dedisp_kernel<1, 8>,
                    dedisp_kernel<1, 4>})
         if (e == cudaSuccess)
@@ -568,10 +572,6 @@ extern "C" void jerk_dedisperser_destroy(jerk_dedisperser *d)
     if (!d)
         return;
     cudaFree(d->d_offsets);
-    cudaFree(d->d_glo);
-    cudaFree(d->d_gbase);
-    cudaFree(d->d_grel);
-    cudaFree(d->d_glen);
     delete d;
 }
 
