@@ -48,15 +48,13 @@ constexpr unsigned kStatusSumCopy = 4u;  // harmsum: the same
 // SMs of the current device (queried once; every B200 has 148)
 inline int sm_count()
 {
-    static int n = 0;
-    if (n <= 0) {
+    static const int n = [] {
         int dev = 0, v = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0)
-            n = v;
-        else
-            return 148;
-    }
+        return cudaGetDevice(&dev) == cudaSuccess &&
+                       cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) ==
+                           cudaSuccess && v > 0
+                   ? v : 148;
+    }();
     return n;
 }
 

@@ -38,10 +38,10 @@ struct CorrSmem {
     static constexpr int value = kBase + (kStage ? N / 2 : 0);
 };
 
-// Kernel row lrow of subharmonic s (fftlen N), rsteps [b0, b1) of the batch,
-// by the CTA's first warps that hold its T threads.  The merged launch
-// runs it for the short lengths; corr_kernel, one length per launch, keeps a
-// copy of the loop that reads its arguments straight from the parameters.
+// Kernel row lrow of subharmonic s (fftlen N, one of the short lengths of the
+// merged launch), rsteps [b0, b1) of the batch, by the CTA's first warps that
+// hold its T threads.  (corr_kernel runs the long lengths, whose rows need not
+// fit in registers nor their data beside the tables, with its own loop.)
 template <int N>
 __device__ __forceinline__ void corr_body(const SearchDev &P, const int s, const int lrow,
                                           const int b0, const int b1)
@@ -49,13 +49,12 @@ __device__ __forceinline__ void corr_body(const SearchDev &P, const int s, const
     constexpr int R0 = FftPlan<N>::R0;
     constexpr int T = FftPlan<N>::T;
     constexpr int TWN = FftPlan<N>::twsize();
-    constexpr bool kStage = CorrSmem<N>::kStage;
-    constexpr bool kBig = CorrBig<N>::value;
+    static_assert(CorrSmem<N>::kStage && !CorrBig<N>::value, "a short length");
     extern __shared__ __align__(16) float2 sm2[];
     __shared__ uint64_t s_bar;
     float2 *buf = sm2;
     float2 *tws = sm2 + fft_buf_len<N>();
-    float2 *dsm = sm2 + CorrSmem<N>::kBase;  // staged data row (kStage)
+    float2 *dsm = sm2 + CorrSmem<N>::kBase;  // staged data row
     const int tid = threadIdx.x;
     const SubDev sd = P.subs[s];
     const float2 *D0 = P.prepped + sd.data_off;
@@ -67,32 +66,23 @@ __device__ __forceinline__ void corr_body(const SearchDev &P, const int s, const
     // tid + r N/R0, so inputs r and r + R0/2 read the same value.
     static_assert(R0 % 2 == 0 && (N / R0) * (R0 / 2) == N / 2, "half-row reads");
     constexpr unsigned kRowBytes = N / 2 * sizeof(float2);
-    if constexpr (kStage) {
-        if (tid == 0) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_bar)) : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-        __syncthreads();
-        if (tid == 0 && b0 < b1)
-            bulk_row_load(dsm, D0 + (long long)b0 * N, kRowBytes, &s_bar);
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&s_bar)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    __syncthreads();
+    if (tid == 0 && b0 < b1)
+        bulk_row_load(dsm, D0 + (long long)b0 * N, kRowBytes, &s_bar);
 
-    const float2 *tw = kBig ? P.twiddles + sd.twoff : tws;
-    if constexpr (!kBig) {
-        for (int i = tid; i < TWN; i += T)
-            tws[i] = P.twiddles[sd.twoff + i];
-    }
-
+    for (int i = tid; i < TWN; i += T)
+        tws[i] = P.twiddles[sd.twoff + i];
 
     // the kernel row, in the order this thread's first-stage butterfly reads it
-    // (kBig: read from global memory at every rstep instead)
     float2 kreg[R0];
     const float2 *K = P.bank + sd.kern_off + (long long)lrow * N;
-    if constexpr (!kBig) {
 #pragma unroll
-        for (int r = 0; r < R0; r++)
-            kreg[r] = tid < T ? K[tid + r * (N / R0)] : make_float2(0.f, 0.f);
-    }
+    for (int r = 0; r < R0; r++)
+        kreg[r] = tid < T ? K[tid + r * (N / R0)] : make_float2(0.f, 0.f);
     __syncthreads();
 
     const int offset = sd.halfwidth * 2;  // binoffset * ACCEL_NUMBETWEEN
@@ -112,31 +102,20 @@ __device__ __forceinline__ void corr_body(const SearchDev &P, const int s, const
             if ((unsigned)kk < (unsigned)numrs)
                 outp[kk] = o;
         };
-        if constexpr (kStage) {
-            // rstep b's row is (or will shortly be) in dsm; once every thread
-            // has read it, thread 0 starts the copy of rstep b + 1's row
-            if (!bar_wait(&s_bar, (b - b0) & 1) && P.status)
-                atomicOr(P.status, kStatusCopy);
-            auto in = [&](int r) -> float2 {
-                // kBig: the kernel row is read from global memory here too
-                return cmulconj(dsm[tid + (r % (R0 / 2)) * (N / R0)],
-                                kBig ? K[tid + r * (N / R0)] : kreg[r]);
-            };
-            auto mid = [&] {
-                if (tid == 0 && b + 1 < b1) {
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    bulk_row_load(dsm, D0 + (long long)(b + 1) * N, kRowBytes, &s_bar);
-                }
-            };
-            fft_block<N, +1>(buf, tw, tid, in, out, mid);
-        } else {
-            const float2 *D = D0 + (long long)b * N;
-            auto in = [&](int r) -> float2 {
-                const int m = tid + r * (N / R0);
-                return cmulconj(D[tid + (r % (R0 / 2)) * (N / R0)], kBig ? K[m] : kreg[r]);
-            };
-            fft_block<N, +1>(buf, tw, tid, in, out);
-        }
+        // rstep b's row is (or will shortly be) in dsm; once every thread
+        // has read it, thread 0 starts the copy of rstep b + 1's row
+        if (!bar_wait(&s_bar, (b - b0) & 1) && P.status)
+            atomicOr(P.status, kStatusCopy);
+        auto in = [&](int r) -> float2 {
+            return cmulconj(dsm[tid + (r % (R0 / 2)) * (N / R0)], kreg[r]);
+        };
+        auto mid = [&] {
+            if (tid == 0 && b + 1 < b1) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                bulk_row_load(dsm, D0 + (long long)(b + 1) * N, kRowBytes, &s_bar);
+            }
+        };
+        fft_block<N, +1>(buf, tws, tid, in, out, mid);
         __syncthreads();
     }
 }

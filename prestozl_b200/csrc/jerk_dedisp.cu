@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "jerk.h"
+#include "jerk_async.cuh"
 #include "jerk_kernels.cuh"
 
 using jerk::set_error;
@@ -250,19 +251,6 @@ downsample_kernel(F *__restrict__ out, const F *__restrict__ in, long long n, in
             t++;
         }
     }
-}
-
-int num_sms()
-{
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            sms < 1)
-            sms = 148;
-    }
-    return sms;
 }
 
 int dd_cuda(cudaError_t e, const char *what)
@@ -517,7 +505,7 @@ extern "C" int jerk_dedisperser_create(jerk_dedisperser **out, int worklen, int 
     int G = 0, T = 0;
     if ((rc = jerk_dedisp_plan(worklen, nsub, numdms, offsets, &G, &T, nullptr)) != JERK_OK)
         return rc;
-    launch_tiling(offsets, worklen, numdms, nsub, num_sms(), &G, &T);
+    launch_tiling(offsets, worklen, numdms, nsub, jerk::sm_count(), &G, &T);
     jerk_dedisperser *d = new jerk_dedisperser;
     d->worklen = worklen;
     d->nsub = nsub;
@@ -626,7 +614,7 @@ extern "C" int jerk_downsample_subbands(float *out, const float *in, int worklen
     const bool quads = nsub % 4 == 0 && ((uintptr_t)in % 16) == 0 && ((uintptr_t)out % 16) == 0;
     const int nv = quads ? nsub / 4 : nsub;
     const long long n = (long long)worklen * nv;
-    const long long blocks = std::min<long long>((n + kDsThreads - 1) / kDsThreads, 8LL * num_sms());
+    const long long blocks = std::min<long long>((n + kDsThreads - 1) / kDsThreads, 8LL * jerk::sm_count());
     cudaStream_t st = (cudaStream_t)stream;
     if (quads)
         downsample_kernel<<<(int)blocks, kDsThreads, 0, st>>>((float4 *)out, (const float4 *)in, n,

@@ -1915,6 +1915,10 @@ static int run_volumes(jerk_plan *p, const SearchDev &a, bool prepared, const Se
             return rc;
     }
     cudaError_t e = cudaSuccess;
+    // The next launch needs the kernel before (as in enqueue_wave): after the
+    // next batch's preparation the rows are older than it, and whatever waited
+    // for it lets the others go.
+    bool first = !ahead;
     for (auto &kv : p->groups) {
         const RowGroup G = row_group(p, kv.second);
         // algorithmic traffic: each kernel row read once per batch, each
@@ -1931,15 +1935,15 @@ static int run_volumes(jerk_plan *p, const SearchDev &a, bool prepared, const Se
             flops += nrow * a.nb * (fft_flops(N) + 6.0 * N) + nrow * numrs * 3.0;
         }
         const int tok = launch_begin(p, kclass(p, "corr_" + std::to_string(N)), bytes, flops);
-        e = launch_corr(a, N, G, G.rowstart[G.n], p->stream);
+        e = launch_corr(a, N, G, G.rowstart[G.n], p->stream);  // (waits)
         launch_end(p, tok);
+        first = false;
         if (e != cudaSuccess)
             return cuda_fail(e, "corr_kernel");
     }
     int sets[kMaxRowSets][2], nsets = 0;
     const FoldRows *rows[kMaxRowSets];
     double mbytes = 0, mflops = 0;
-    bool first = p->groups.empty() && !ahead;  // the next launch needs the one before
     for (size_t i = 0; i < p->rowsets.size(); i++) {
         const FoldRows &R = p->rowsets[i];
         if (!p->own_launch[i]) {
