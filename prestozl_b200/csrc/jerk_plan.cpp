@@ -84,6 +84,10 @@ static thread_local std::string g_err;
 
 static int fail(int code, const std::string &msg)
 {
+    // an error that has been reported (an allocation that did not fit) is not
+    // the next launch's
+    if (code == JERK_ECUDA)
+        cudaGetLastError();
     g_err = msg;
     return code;
 }

@@ -2,12 +2,27 @@
 search still has to allocate takes the place of the plan's optional buffers, and
 the hits are those of a device with room."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from prestozl_b200 import jerk
 
 pytestmark = pytest.mark.gpu
+
+
+def _fill(torch, need, filled):
+    """Takes device memory until less than `need` bytes are left."""
+    size = torch.cuda.mem_get_info()[0]
+    while size >= 1 << 20 and torch.cuda.mem_get_info()[0] >= need:
+        p = C.c_void_p()
+        if (torch.cuda.mem_get_info()[0] - size >= need // 4 and
+                jerk.lib().jerk_device_alloc(size, C.byref(p)) == jerk.JERK_OK):
+            filled.append(p)
+        else:
+            size //= 2
+    assert torch.cuda.mem_get_info()[0] < need
 
 
 @pytest.mark.parametrize("graph", [False, True])
@@ -29,23 +44,15 @@ def test_host_spectrum_is_staged_on_a_full_device(graph):
     assert len(want[0]) > 0
     plan = jerk.JerkPlan(obs, subs, batch=batch, device_bank=bank.ptr.value, use_graph=graph)
     torch.cuda.synchronize()
+    torch.cuda.empty_cache()
     need = 8 * (N // 2)
-    # all but half a spectrum, a piece at a time
-    filled, piece = [], torch.cuda.mem_get_info()[0] // 2
-    while piece >= 1 << 20:
-        if torch.cuda.mem_get_info()[0] - piece < need // 2:
-            piece //= 2
-            continue
-        try:
-            filled.append(torch.empty(piece, dtype=torch.uint8, device="cuda"))
-        except torch.cuda.OutOfMemoryError:
-            piece //= 2
+    filled = []
     try:
-        assert torch.cuda.mem_get_info()[0] < need
+        _fill(torch, need, filled)
         got = plan.search(host, want_hits=True)[1:]
     finally:
-        del filled
-        torch.cuda.empty_cache()
+        for p in filled:
+            jerk.lib().jerk_device_free(p)
     again = plan.search(host, want_hits=True)[1:]
     for h in (got, again):
         assert np.array_equal(h[0], want[0])
