@@ -113,7 +113,11 @@ typedef struct jerk_config {
     const void *device_bank;  /* optional resident bank (jerk_bank_generate); it
                                  must be complete when the plan is created (the
                                  plan folds its rows of fftlen 512 to 4096 from it
-                                 then) */
+                                 then).  Of these rows, here and in
+                                 jerk_subharm.kernels, the taps count that carry a
+                                 row's energy but for 4e-14 of it -- the rounding
+                                 of its own 32-bit values; a response with a
+                                 fainter tail than 2e-7 loses that tail */
     int harm_mode;            /* harmonic-sum kernel (a tuning knob; results do
                                  not depend on it): 1 = gather (global loads),
                                  2 = gather + TMA prefetch of the next tile into
@@ -175,8 +179,8 @@ int jerk_search_collect(jerk_plan *plan, jerk_cand **cands, long long *ncands, j
 /* The batched form across plans: several searches (spectra of any length,
  * plans of any geometry) advanced in waves of merged launches.  One wave
  * takes the next batch of every listed plan with work left (up to 12 per
- * wave) and runs one prep launch, one correlation launch per FFT length and
- * one harmonic-sum launch per stage count over all of them, so small
+ * wave) and runs its preparation, correlations and harmonic sums in launches
+ * over all of them (a plan's own where its work fills the GPU), so small
  * searches share the GPU instead of each underfilling it.  Each plan's
  * results are bitwise those of jerk_search.  Replaces, for this purpose, the
  * reference's process pool (bin/accelsearch_pipeline_cu.py:296-407), whose

@@ -811,7 +811,8 @@ __global__ void __launch_bounds__(kHarmThreads, HarmOcc<S, 4>::value)
 }
 
 // ---------------------------------------------------------------------------
-// 3b. Harmonic summing fed by TMA (the default where its boxes fit).
+// 3b. Harmonic summing fed by TMA (harm_mode 3 and 4; the default forms are the
+// gathers above and the ring of row copies in jerk_harm.cu).
 //
 // Same thread mapping, same float adds in the same order and the same hit
 // keys as harmsum_kernel, so the results are bitwise the same; the
@@ -1180,8 +1181,7 @@ cudaError_t launch_harmsum(const SearchDev &P, const HarmTma &T, bool prefetch, 
 
 // ---------------------------------------------------------------------------
 // Waves: one launch per kernel kind over the current batches of several
-// plans.  The caller fills M.n, M.P and (corr) M.G; the launchers fill the
-// CTA ranges.
+// plans.  The caller fills M.n and M.P; the launchers fill the CTA ranges.
 
 cudaError_t launch_prep_group(GroupLaunch M, int maxfft, size_t smem, cudaStream_t st)
 {

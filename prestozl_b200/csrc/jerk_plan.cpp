@@ -2257,12 +2257,13 @@ extern "C" int jerk_search_ready(jerk_plan *p)
 }
 
 // ---------------------------------------------------------------------------
-// Waves: the current batches of several plans' passes in merged launches --
-// one prep launch, one correlation launch per FFT length and one harmonic
-// sum per stage count, each covering every plan of the wave (up to
-// kMaxGroupPlans) -- so spectra of uneven length and geometry share launches
-// and small ones fill the GPU together.  Every plan's CTAs run as in its own
-// launches, so its results are bitwise the same.
+// Waves: the current batches of several plans' passes in merged launches, each
+// covering every plan of the wave (up to kMaxGroupPlans): one preparation (and
+// one of the next batches), one correlation and one harmonic sum per stage count
+// and form, so spectra of uneven length and geometry share launches and small
+// ones fill the GPU together; what fills it by itself (a plan's row sets, long
+// unfolded lengths, large volumes) keeps launches of its own.  Every plan's sums
+// run as in its own launches, so its results are bitwise the same.
 
 extern "C" int jerk_search_begin(jerk_plan *p, const void *spectrum, int spectrum_on_device,
                                  long long first_rstep, long long num_rsteps)
@@ -2531,10 +2532,6 @@ struct HitGeom {
     std::function<long long(long long)> rlo_of;
 };
 
-// Hits in key order -- the reference's insertion order (rstep, stage, w, z,
-// r; src/accel_utils_cu.c:857-929) -- decoded into candidates with their
-// sigma and inserted with the reference's rule.  order receives the sorted
-// permutation of the input.
 // order[i]: the index of the i-th key in ascending order.  Keys are distinct;
 // many are sorted by 11-bit digits of the bits they use.
 static void sort_keys(const unsigned long long *keys, uint32_t n, std::vector<uint32_t> &order)
@@ -2564,6 +2561,10 @@ static void sort_keys(const unsigned long long *keys, uint32_t n, std::vector<ui
     }
 }
 
+// Hits in key order -- the reference's insertion order (rstep, stage, w, z,
+// r; src/accel_utils_cu.c:857-929) -- decoded into candidates with their
+// sigma and inserted with the reference's rule.  order receives the sorted
+// permutation of the input.
 static void hits_to_list(const HitGeom &g, const unsigned long long *keys, const float *pows,
                          uint32_t nh, std::vector<uint32_t> &order, CandList &L)
 {
